@@ -191,7 +191,8 @@ __device__ __forceinline__ BwdItem decode_item(const BwdParams& p, int w) {
 // abort flag: the producer's own waits are all bounded, so it always gets to publish the next item (after a failure:
 // the end marker), and all threads of a role must see the SAME item -- their loops, named barriers and
 // warp-collective instructions depend on it.  Its own limit is generous and is not expected to be reached.
-__device__ __forceinline__ int next_item(BwdShared& sh, int k, volatile uint32_t* abort_flag, unsigned int* status, BwdItem& out) {
+__device__ __forceinline__ int next_item(BwdShared& sh, int k, volatile uint32_t* abort_flag, unsigned int* status, BwdItem& out,
+                                         bool whole_warp = false) {
   uint64_t* bar = &sh.item_full[k & 1];
   const uint32_t parity = (k >> 1) & 1;
   uint32_t polls = 0;
@@ -204,7 +205,9 @@ __device__ __forceinline__ int next_item(BwdShared& sh, int k, volatile uint32_t
   }
   const int w = sh.item[k & 1];
   out = sh.decoded[k & 1];                // (stale behind the end marker: never looked at)
-  mbar_arrive(&sh.item_empty[k & 1]);     // the slot may be reused once every consumer has read it
+  // the slot may be reused once every consumer has read it (the MMA warp counts as one)
+  if (whole_warp) __syncwarp();
+  if (!whole_warp || (threadIdx.x & 31) == 0) mbar_arrive(&sh.item_empty[k & 1]);
   return w;
 }
 
@@ -232,7 +235,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
   BwdShared& sh = *reinterpret_cast<BwdShared*>(sStage + 32768);
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = static_cast<int>(warp_uniform(tid >> 5));
   const int lane = tid & 31;
   // The CTA is persistent: it takes work items (decode_item) one after the other from a global counter until none is
   // left.  Its tensor memory, barriers and warp roles live for the whole kernel; the K/V tiles of the next item are
@@ -271,7 +274,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem = sh.tmem_base;
+  const uint32_t tmem = warp_uniform(sh.tmem_base);
   volatile uint32_t* abort_flag = &sh.abort_flag;
 
   if (warp >= kProducerWarp) {
@@ -279,7 +282,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
     reg_dealloc<kRegsControl>();
     if (warp == kProducerWarp) {
       // ---------------------------------------------------------------- TMA producer (and keeper of the work list)
-      if (lane == 0) {
+      if (elect_one()) {
         prefetch_tmap(&p.map_q); prefetch_tmap(&p.map_k); prefetch_tmap(&p.map_v); prefetch_tmap(&p.map_do);
         prefetch_tmap(&p.map_dq);
         int g0 = 0, live = 0;
@@ -340,7 +343,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
     } else if (warp == kMmaWarp) {
       // ---------------------------------------------------------------- MMA issuer
       // Tensor-pipe order per Q tile n:  dP^T(n) | dV(n), S^T(n+1) | dK(n), dQ(n).
-      if (lane == 0) {
+      {
         const uint32_t idesc_s = make_idesc(BF16, 128, 128, false, false);     // S^T, dP^T
         const uint32_t idesc_kv = make_idesc(BF16, 128, DPAD, false, true);    // dV, dK
         const uint32_t idesc_dq = make_idesc(BF16, 128, DPAD, true, true);     // dQ
@@ -357,18 +360,20 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
 
         auto issue_st = [&](int st) {   // S^T = K Q^T
           const uint32_t kQ = kQ0 + st * kTileUnits;
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < DPAD / 16; ++kk) {
-            const uint32_t off = (kk >> 2) * 1024u + (kk & 3) * 2u;   // 16-byte units
-            umma_ss_lohi(tmem + kColST, kK + off, k_hi, kQ + off, k_hi, idesc_s, kk > 0);
+            for (int kk = 0; kk < DPAD / 16; ++kk) {
+              const uint32_t off = (kk >> 2) * 1024u + (kk & 3) * 2u;   // 16-byte units
+              umma_ss_lohi(tmem + kColST, kK + off, k_hi, kQ + off, k_hi, idesc_s, kk > 0);
+            }
+            umma_commit(&sh.st_full);
           }
-          umma_commit(&sh.st_full);
         };
 
         int g0 = 0, live = 0;
         for (int k = 0;; ++k) {
           BwdItem it;
-          const int w = next_item(sh, k, abort_flag, p.status, it);
+          const int w = next_item(sh, k, abort_flag, p.status, it, true);
           if (w >= total_items) break;
           if (it.n_iter == 0) continue;
           const int n_iter = it.n_iter;
@@ -384,23 +389,27 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
             // dP^T = V dO^T as early as possible: it only needs dO and the previous dQ out of its columns
             mbar_wait(&sh.do_full, gn & 1, abort_flag, p.status, DEV_TIMEOUT_TMA);
             tc_fence_after_sync();
+            if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < DPAD / 16; ++kk) {
-              const uint32_t off = (kk >> 2) * 1024u + (kk & 3) * 2u;
-              umma_ss_lohi(tmem + kColDP, kV + off, k_hi, kDO + off, k_hi, idesc_s, kk > 0);
+              for (int kk = 0; kk < DPAD / 16; ++kk) {
+                const uint32_t off = (kk >> 2) * 1024u + (kk & 3) * 2u;
+                umma_ss_lohi(tmem + kColDP, kV + off, k_hi, kDO + off, k_hi, idesc_s, kk > 0);
+              }
+              umma_commit(&sh.dp_full);
             }
-            umma_commit(&sh.dp_full);
             // dV += P^T dO as soon as P^T is in tensor memory (the compute warps go on to dS meanwhile);
             // P^T of query columns [64h, 64h+64) sits in S^T columns [64h, 64h+32)
             mbar_wait(&sh.p_ready, gn & 1, abort_flag, p.status, DEV_TIMEOUT_SYNC);
             // the first products of an item overwrite dK and dV: the previous item's must have been read out
             if (n == 0 && live > 0) mbar_wait(&sh.acc_free, (live - 1) & 1, abort_flag, p.status, DEV_TIMEOUT_SYNC);
             tc_fence_after_sync();
+            if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < kTile / 16; ++kk)
-              umma_ts_lohi(tmem + kColDV, tmem + kColST + (kk >> 2) * 64 + (kk & 3) * 8, mDO + kk * 128u, mn_hi,
-                           idesc_kv, n > 0 || kk > 0);
-            umma_commit(&sh.do_empty);
+              for (int kk = 0; kk < kTile / 16; ++kk)
+                umma_ts_lohi(tmem + kColDV, tmem + kColST + (kk >> 2) * 64 + (kk & 3) * 8, mDO + kk * 128u, mn_hi,
+                             idesc_kv, n > 0 || kk > 0);
+              umma_commit(&sh.do_empty);
+            }
             // S^T of the next Q tile right behind it (the tensor pipe runs in order, so P^T has been consumed)
             if (n + 1 < n_iter) {
               mbar_wait(&sh.q_full[stn], ((gn + 1) / kStages) & 1, abort_flag, p.status, DEV_TIMEOUT_TMA);
@@ -410,16 +419,18 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
             // dK += dS^T Q and dQ = dS K once dS^T is in shared memory
             mbar_wait(&sh.ds_ready, gn & 1, abort_flag, p.status, DEV_TIMEOUT_SYNC);
             tc_fence_after_sync();
+            if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < kTile / 16; ++kk)   // dK: A = dS^T packed over the dP^T columns, like P^T over S^T
-              umma_ts_lohi(tmem + kColDK, tmem + kColDP + (kk >> 2) * 64 + (kk & 3) * 8, mQ + kk * 128u, mn_hi,
-                           idesc_kv, n > 0 || kk > 0);
+              for (int kk = 0; kk < kTile / 16; ++kk)   // dK: A = dS^T packed over the dP^T columns, like P^T over S^T
+                umma_ts_lohi(tmem + kColDK, tmem + kColDP + (kk >> 2) * 64 + (kk & 3) * 8, mQ + kk * 128u, mn_hi,
+                             idesc_kv, n > 0 || kk > 0);
 #pragma unroll
-            for (int kk = 0; kk < kTile / 16; ++kk)
-              umma_ss_lohi(tmem + kColDP, mDS + kk * 128u, mn_hi, mK + kk * 128u, mn_hi, idesc_dq, kk > 0);
-            umma_commit(&sh.dq_full);     // (the drain passes it on to the producer as q_empty[st]: one commit less here)
+              for (int kk = 0; kk < kTile / 16; ++kk)
+                umma_ss_lohi(tmem + kColDP, mDS + kk * 128u, mn_hi, mK + kk * 128u, mn_hi, idesc_dq, kk > 0);
+              umma_commit(&sh.dq_full);     // (the drain passes it on to the producer as q_empty[st]: one commit less here)
+            }
           }
-          umma_commit(&sh.kv_empty);
+          if (elect_one()) umma_commit(&sh.kv_empty);
           g0 += n_iter;
           ++live;
         }

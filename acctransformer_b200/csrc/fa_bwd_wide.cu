@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(kWThreads, 1) fa_bwd_wide_kernel(const __grid_
   WideShared& sh = *reinterpret_cast<WideShared*>(sStage + 16384);
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = static_cast<int>(warp_uniform(tid >> 5));
   const int lane = tid & 31;
   const int n_kv = p.N / p.kv_group;
   const int bh_kv = blockIdx.y;
@@ -124,14 +124,14 @@ __global__ void __launch_bounds__(kWThreads, 1) fa_bwd_wide_kernel(const __grid_
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem = sh.tmem_base;
+  const uint32_t tmem = warp_uniform(sh.tmem_base);
   volatile uint32_t* abort_flag = &sh.abort_flag;
 
   if (warp >= kWProducerWarp) {
     reg_dealloc<kWRegsControl>();
     if (warp == kWProducerWarp) {
       // ---------------------------------------------------------------- TMA producer
-      if (lane == 0 && n_steps > 0) {
+      if (n_steps > 0 && elect_one()) {
         prefetch_tmap(&p.map_q); prefetch_tmap(&p.map_k); prefetch_tmap(&p.map_v); prefetch_tmap(&p.map_do);
         prefetch_tmap(&p.map_dq);
         mbar_expect_tx(&sh.kv_full, 2 * kKvTileBytes);
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(kWThreads, 1) fa_bwd_wide_kernel(const __grid_
       }
     } else if (warp == kWMmaWarp) {
       // ---------------------------------------------------------------- MMA issuer
-      if (lane == 0 && n_steps > 0) {
+      if (n_steps > 0) {
         const uint32_t idesc_s = make_idesc(BF16, 128, kSub, false, false);    // S^T, dP^T
         const uint32_t idesc_kv = make_idesc(BF16, 128, 128, false, true);     // dV, dK halves
         const uint32_t idesc_dq = make_idesc(BF16, 128, kSub, true, true);     // dQ^T half
@@ -171,41 +171,51 @@ __global__ void __launch_bounds__(kWThreads, 1) fa_bwd_wide_kernel(const __grid_
           const uint32_t par = m & 1;
           mbar_wait(&sh.q_full, par, abort_flag, p.status, DEV_TIMEOUT_TMA);
           tc_fence_after_sync();
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < 16; ++kk)   // S^T = K Q^T over the whole width
-            umma_ss_lohi(tmem + kColST, kK + (kk >> 2) * 1024u + (kk & 3) * 2u, k_hi, kQ + (kk >> 2) * 512u + (kk & 3) * 2u,
-                         k_hi, idesc_s, kk > 0);
-          umma_commit(&sh.st_full);
+            for (int kk = 0; kk < 16; ++kk)   // S^T = K Q^T over the whole width
+              umma_ss_lohi(tmem + kColST, kK + (kk >> 2) * 1024u + (kk & 3) * 2u, k_hi, kQ + (kk >> 2) * 512u + (kk & 3) * 2u,
+                           k_hi, idesc_s, kk > 0);
+            umma_commit(&sh.st_full);
+          }
           mbar_wait(&sh.do_full, par, abort_flag, p.status, DEV_TIMEOUT_TMA);
           tc_fence_after_sync();
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < 16; ++kk)   // dP^T = V dO^T
-            umma_ss_lohi(tmem + kColDP, kV + (kk >> 2) * 1024u + (kk & 3) * 2u, k_hi, kDO + (kk >> 2) * 512u + (kk & 3) * 2u,
-                         k_hi, idesc_s, kk > 0);
-          umma_commit(&sh.dp_full);
+            for (int kk = 0; kk < 16; ++kk)   // dP^T = V dO^T
+              umma_ss_lohi(tmem + kColDP, kV + (kk >> 2) * 1024u + (kk & 3) * 2u, k_hi, kDO + (kk >> 2) * 512u + (kk & 3) * 2u,
+                           k_hi, idesc_s, kk > 0);
+            umma_commit(&sh.dp_full);
+          }
           // dV half += P^T dO half: P^T of queries [32h, 32h+32) sits in S^T columns [32h, 32h+16)
           mbar_wait(&sh.p_ready, par, abort_flag, p.status, DEV_TIMEOUT_SYNC);
           tc_fence_after_sync();
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < kSub / 16; ++kk)
-            umma_ts_lohi(tmem + kColDV, tmem + kColST + (kk >> 1) * 32 + (kk & 1) * 8, mDOh + kk * 128u, msub_hi, idesc_kv,
-                         m > 0 || kk > 0);
-          umma_commit(&sh.do_empty);
+            for (int kk = 0; kk < kSub / 16; ++kk)
+              umma_ts_lohi(tmem + kColDV, tmem + kColST + (kk >> 1) * 32 + (kk & 1) * 8, mDOh + kk * 128u, msub_hi, idesc_kv,
+                           m > 0 || kk > 0);
+            umma_commit(&sh.do_empty);
+          }
           // dK half += dS^T Q half
           mbar_wait(&sh.ds_ready, par, abort_flag, p.status, DEV_TIMEOUT_SYNC);
           tc_fence_after_sync();
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < kSub / 16; ++kk)
-            umma_ts_lohi(tmem + kColDK, tmem + kColDP + (kk >> 1) * 32 + (kk & 1) * 8, mQh + kk * 128u, msub_hi, idesc_kv,
-                         m > 0 || kk > 0);
-          umma_commit(&sh.q_empty);
+            for (int kk = 0; kk < kSub / 16; ++kk)
+              umma_ts_lohi(tmem + kColDK, tmem + kColDP + (kk >> 1) * 32 + (kk & 1) * 8, mQh + kk * 128u, msub_hi, idesc_kv,
+                           m > 0 || kk > 0);
+            umma_commit(&sh.q_empty);
+          }
           // dQ^T half = K half^T dS^T, once the drain has pulled the previous one out of its columns
           if (m > 0) mbar_wait(&sh.dq_read, (m - 1) & 1, abort_flag, p.status, DEV_TIMEOUT_SYNC);
           tc_fence_after_sync();
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < kTile / 16; ++kk)
-            umma_ss_lohi(tmem + kColDQ, mKh + kk * 128u, mkv_hi, mDS + kk * 128u, msub_hi, idesc_dq, kk > 0);
-          umma_commit(&sh.dq_full);
+            for (int kk = 0; kk < kTile / 16; ++kk)
+              umma_ss_lohi(tmem + kColDQ, mKh + kk * 128u, mkv_hi, mDS + kk * 128u, msub_hi, idesc_dq, kk > 0);
+            umma_commit(&sh.dq_full);
+          }
         }
       }
     }

@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
   __shared__ FwdShared sh;
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = static_cast<int>(warp_uniform(tid >> 5));
   const int lane = tid & 31;
   const ScoreMods& mods = p.mods;
 
@@ -144,13 +144,13 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem = sh.tmem_base;
+  const uint32_t tmem = warp_uniform(sh.tmem_base);
   volatile uint32_t* abort_flag = &sh.abort_flag;
 
   if (warp == 8) {
     // ------------------------------------------------------------------ TMA producer
     reg_dealloc<kRegsControl>();
-    if (lane == 0 && cta_hi >= cta_lo) {
+    if (cta_hi >= cta_lo && elect_one()) {
       prefetch_tmap(&p.map_q); prefetch_tmap(&p.map_k); prefetch_tmap(&p.map_v); prefetch_tmap(&p.map_o);
       mbar_expect_tx(&sh.q_full, NQ * kTileBytes);
       for (int qt = 0; qt < NQ; ++qt)
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
     // behind a burst of MMAs that is still executing, and each hand-off from the softmax groups is waited
     // for once.
     reg_dealloc<kRegsControl>();
-    if (lane == 0 && cta_hi >= cta_lo) {
+    if (cta_hi >= cta_lo) {
       const uint32_t idesc_s = make_idesc(BF16, 128, 128, false, false);
       const uint32_t idesc_o = make_idesc(BF16, 128, DPAD, false, true);
       const uint64_t kmajor = make_sdesc_base(16, 1024);
@@ -197,19 +197,21 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
 
       auto issue_s = [&](int qt, int st) {
         const uint32_t a0 = q_lo + qt * kTileUnits, b0 = kt_lo + st * kTileUnits;
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < DPAD / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * 1024u + (kk & 3) * 2u;   // 16-byte units
-          umma_ss_lohi(tmem + kColS + qt * 128, a0 + off, k_hi, b0 + off, k_hi, idesc_s, kk > 0);
+          for (int kk = 0; kk < DPAD / 16; ++kk) {
+            const uint32_t off = (kk >> 2) * 1024u + (kk & 3) * 2u;   // 16-byte units
+            umma_ss_lohi(tmem + kColS + qt * 128, a0 + off, k_hi, b0 + off, k_hi, idesc_s, kk > 0);
+          }
+          umma_commit(&sh.s_full[qt]);
         }
-        umma_commit(&sh.s_full[qt]);
       };
 
       // prologue: scores of the first K/V tile
       mbar_wait(&sh.k_full[0], 0, abort_flag, p.status, DEV_TIMEOUT_TMA);
       for (int qt = 0; qt < 2; ++qt)
         if (cta_lo >= rng[qt].lo && cta_lo <= rng[qt].hi) issue_s(qt, 0);
-      umma_commit(&sh.k_empty[0]);
+      if (elect_one()) umma_commit(&sh.k_empty[0]);
       mbar_wait(&sh.v_full[0], 0, abort_flag, p.status, DEV_TIMEOUT_TMA);
       int it = 0;
       for (int j = cta_lo; j <= cta_hi; ++j, ++it) {
@@ -227,9 +229,11 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
             // P arrives in two halves (key rows 0-63, then 64-127 of the V tile, which was seen full before)
             mbar_wait(&sh.p_half[qt], n_done[qt] & 1, abort_flag, p.status, DEV_TIMEOUT_SYNC);
             tc_fence_after_sync();
+            if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < kTile / 32; ++kk)
-              umma_ts_lohi(t_o, t_s + kk * 8, v0 + kk * 128u, mn_hi, idesc_o, n_done[qt] > 0 || kk > 0);
+              for (int kk = 0; kk < kTile / 32; ++kk)
+                umma_ts_lohi(t_o, t_s + kk * 8, v0 + kk * 128u, mn_hi, idesc_o, n_done[qt] > 0 || kk > 0);
+            }
           }
           if (sn && !k_seen) {
             mbar_wait(&sh.k_full[stn], full_parity_n, abort_flag, p.status, DEV_TIMEOUT_TMA);
@@ -238,20 +242,24 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
           if (pv) {
             mbar_wait(&sh.p_ready[qt], n_done[qt] & 1, abort_flag, p.status, DEV_TIMEOUT_SYNC);
             tc_fence_after_sync();
+            if (elect_one()) {
 #pragma unroll
-            for (int kk = kTile / 32; kk < kTile / 16; ++kk)
-              umma_ts_lohi(t_o, t_s + kk * 8, v0 + kk * 128u, mn_hi, idesc_o, true);
+              for (int kk = kTile / 32; kk < kTile / 16; ++kk)
+                umma_ts_lohi(t_o, t_s + kk * 8, v0 + kk * 128u, mn_hi, idesc_o, true);
+              if (j == rng[qt].hi) umma_commit(&sh.o_done[qt]);
+            }
             // O is only looked at after the Q tile's last K/V tile (the rescaling of earlier tiles is ordered by
             // s_full: the S product it waits for was issued after their P V), so one commit per Q tile is enough --
             // every commit costs this thread 80-95 cycles in which it issues nothing
-            if (j == rng[qt].hi) umma_commit(&sh.o_done[qt]);
             ++n_done[qt];
           }
           if (sn) issue_s(qt, stn);
         }
-        umma_commit(&sh.v_empty[st]);
+        if (elect_one()) {
+          umma_commit(&sh.v_empty[st]);
+          if (more) umma_commit(&sh.k_empty[stn]);
+        }
         if (more) {
-          umma_commit(&sh.k_empty[stn]);
           // the next V tile, waited for while the MMAs just issued still execute
           mbar_wait(&sh.v_full[stn], full_parity_n, abort_flag, p.status, DEV_TIMEOUT_TMA);
         }

@@ -127,6 +127,26 @@ __device__ __forceinline__ void reg_dealloc() {
 }
 
 // ------------------------------------------------------------------------------------------
+// one elected lane of a converged warp
+// ------------------------------------------------------------------------------------------
+// The single-thread instructions (tcgen05.mma / commit, TMA) take their operands from uniform registers.  Under
+// `if (lane == 0)` the compiler cannot know that one lane is active and wraps each of them in a loop over the distinct
+// operand values of the active lanes; under this predicate, inside code that the whole warp reaches together, it can.
+// Always the same lane for a full mask.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t pred;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(pred)
+      :
+      : "memory");
+  return pred != 0u;
+}
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t x) { return __shfl_sync(0xffffffffu, x, 0); }
+
+// ------------------------------------------------------------------------------------------
 // fences
 // ------------------------------------------------------------------------------------------
 // generic-proxy writes to shared memory -> visible to the async proxy (TMA / tcgen05.mma reads)
