@@ -25,7 +25,7 @@ ERR_NAMES = {
 }
 
 EXPORTS = [
-    "acct_fa_fwd", "acct_fa_bwd_workspace_bytes", "acct_fa_bwd", "acct_infer_prefill",
+    "acct_fa_fwd", "acct_fa_bwd_workspace_bytes", "acct_fa_bwd", "acct_fa_bwd_strided", "acct_infer_prefill",
     "acct_infer_decode_workspace_bytes", "acct_infer_decode", "acct_infer_decode_static", "acct_device_status",
     "acct_last_error", "acct_abi_version",
     "acct_ms_set_fa_attrs", "acct_ms_fa_fwd", "acct_ms_fa_grad", "acct_ms_infer_fa", "acct_dropout_mask",
@@ -92,6 +92,22 @@ class DecodeArgs(C.Structure):
 
 
 _lib = None
+_host = None
+
+
+def host():
+    """The native host path of the Python layers (csrc/torch_host.cpp), bound to the library ``load()`` loads."""
+    global _host
+    if _host is None:
+        load()
+        try:
+            from . import _torch_host
+        except ImportError as e:
+            raise ImportError("the _torch_host module is missing or does not match this torch: build it with "
+                              "`python -m acctransformer_b200.build`; there is no fallback path") from e
+        _torch_host.init(LIB_PATH)
+        _host = _torch_host
+    return _host
 
 
 def load():

@@ -1,5 +1,8 @@
 """Builds ``libacct_b200.so`` (the C-ABI library) from ``csrc/*.cu`` with nvcc for sm_100a.
 
+Beside it, ``_torch_host.so`` (the native host path of the Python layers) is compiled from ``csrc/torch_host.cpp`` with
+the host compiler against the installed torch.
+
 The library is built in-tree, next to this file, so that it travels with the source tree.
 ``python -m acctransformer_b200.build`` rebuilds it; ``build()`` is also what
 ``__graft_entry__.build()`` calls.
@@ -22,6 +25,23 @@ NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden", "--expt-relaxed-constexpr",
 ]
+HOST_SOURCE = "torch_host.cpp"
+HOST_PATH = os.path.join(HERE, "_torch_host.so")
+
+
+def _host_command(src, out):
+    """Compiles the CPython module; torch's own libraries are in the process before it is imported."""
+    import sysconfig
+
+    import torch
+    inc = os.path.join(os.path.dirname(torch.__file__), "include")
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wno-attributes",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            "-I" + inc, "-I" + os.path.join(inc, "torch", "csrc", "api", "include"), "-I" + sysconfig.get_paths()["include"],
+            "-I" + os.path.join(cuda, "include"), src, "-o", out,
+            "-L" + lib, "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10", "-ldl"]
 
 
 def _nvcc():
@@ -39,7 +59,7 @@ def _stale(target, deps):
 
 
 def build(force=False, verbose=False):
-    """Compile every CUDA source and link the shared library.  Returns its path."""
+    """Compile every CUDA source and the host module, and link the shared library.  Returns the library's path."""
     os.makedirs(OBJ_DIR, exist_ok=True)
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
     headers.append(os.path.join(os.path.dirname(HERE), "include", "acct_b200.h"))
@@ -59,11 +79,16 @@ def build(force=False, verbose=False):
         if verbose or r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
         if r.returncode != 0:
-            raise RuntimeError("nvcc failed: " + " ".join(cmd))
+            raise RuntimeError("compiling failed: " + " ".join(cmd))
+
+    host_src = os.path.join(CSRC, HOST_SOURCE)
+    if force or _stale(HOST_PATH, [host_src, os.path.join(os.path.dirname(HERE), "include", "acct_b200.h")]):
+        jobs.append(_host_command(host_src, HOST_PATH))
+    device_jobs = any(cmd[0] == nvcc for cmd in jobs)
 
     with ThreadPoolExecutor(max_workers=4) as ex:
         list(ex.map(run, jobs))
-    if force or jobs or _stale(LIB_PATH, objs):
+    if force or device_jobs or _stale(LIB_PATH, objs):
         run([nvcc, "-shared", "-o", LIB_PATH] + objs + ["-lcudart"])
     return LIB_PATH
 

@@ -77,6 +77,14 @@ int init_device(PerDevice** out) {
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return fail(ACCT_ERR_NO_DEVICE, "no CUDA device: %s", cudaGetErrorString(e));
   if (dev < 0 || dev >= kMaxDevices) return fail(ACCT_ERR_NO_DEVICE, "device index %d out of range", dev);
+  // A thread that has made no runtime call yet (an autograd engine's worker) has no context bound, and the driver call
+  // that encodes tensor maps needs one: bind the device's primary context once per thread and device.
+  static thread_local int t_bound = -1;
+  if (t_bound != dev) {
+    e = cudaSetDevice(dev);
+    if (e != cudaSuccess) return fail(ACCT_ERR_NO_DEVICE, "cudaSetDevice(%d): %s", dev, cudaGetErrorString(e));
+    t_bound = dev;
+  }
   std::lock_guard<std::mutex> lock(g_mutex);
   PerDevice& d = g_dev[dev];
   if (!d.ready) {
@@ -421,9 +429,19 @@ size_t acct_fa_bwd_workspace_bytes(const acct_fa_args* a) {
 }
 
 int acct_fa_bwd(const acct_fa_args* a, const acct_fa_bwd_io* g, void* stream) {
+  return acct_fa_bwd_strided(a, g, nullptr, stream);
+}
+
+int acct_fa_bwd_strided(const acct_fa_args* a, const acct_fa_bwd_io* g, const int64_t* d_o_stride, void* stream) {
   Strides st;
   int rc = validate_fa(a, &st, true);
   if (rc) return rc;
+  int64_t st_do[3];
+  {
+    int64_t given[3];
+    for (int i = 0; i < 3; ++i) given[i] = d_o_stride != nullptr && d_o_stride[i] != 0 ? d_o_stride[i] : st.o[i];
+    if ((rc = check_strides("d_o", given, a->S_q, a->N, a->D, st_do))) return rc;
+  }
   if (g == nullptr) return fail(ACCT_ERR_NULL, "backward io is NULL");
   if (!g->d_o || !g->dq || !g->dk || !g->dv || !a->lse) return fail(ACCT_ERR_NULL, "d_o, dq, dk, dv and lse must be non-NULL");
   if (!aligned16(g->d_o) || !aligned16(g->dq) || !aligned16(g->dk) || !aligned16(g->dv))
@@ -453,7 +471,7 @@ int acct_fa_bwd(const acct_fa_args* a, const acct_fa_bwd_io* g, void* stream) {
   TensorDesc4 t;
   t.dtype = a->dtype; t.ptr = g->d_o;
   t.dims[0] = a->D; t.dims[1] = a->S_q; t.dims[2] = a->N; t.dims[3] = a->B;
-  t.strides[0] = st.o[2]; t.strides[1] = st.o[1]; t.strides[2] = st.o[0];
+  t.strides[0] = st_do[2]; t.strides[1] = st_do[1]; t.strides[2] = st_do[0];
   if ((rc = make_tmap_4d(&p.map_do, t, wide ? 64 : kTile))) return rc;
   // the fp32 dQ accumulator, packed [B,N,S_q,D]: target of the kernel's TMA reduce-add
   t.dtype = ACCT_F32; t.ptr = dq_acc;
@@ -474,8 +492,8 @@ int acct_fa_bwd(const acct_fa_args* a, const acct_fa_bwd_io* g, void* stream) {
   }
 
   // one helper pass before the main kernel: row sums, and the zero-fill of the accumulator and the turn counters
-  cudaError_t e = launch_bwd_delta(a->o, g->d_o, delta, static_cast<int64_t>(rows), a->D, st.o[0], st.o[1], st.o[2], a->N,
-                                   a->S_q, bf16, s, dq_acc, dq_order, static_cast<int64_t>(q_tiles));
+  cudaError_t e = launch_bwd_delta(a->o, g->d_o, delta, static_cast<int64_t>(rows), a->D, st.o, st_do, a->N, a->S_q, bf16,
+                                   s, dq_acc, dq_order, static_cast<int64_t>(q_tiles));
   if (e != cudaSuccess) return fail_cuda(e, "launching the row-sum kernel");
   p.lse = a->lse; p.delta = delta; p.dq_acc = dq_acc;
   p.dq_order = (a->flags & ACCT_FLAG_DETERMINISTIC) ? dq_order : nullptr;

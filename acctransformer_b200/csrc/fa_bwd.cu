@@ -919,15 +919,18 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
   }
 }
 
+struct RowStrides {
+  int64_t b, h, s;
+};
+
 // D[row] = sum_d dO[row,d] * O[row,d]  (fp32).  LPR lanes x 16 bytes cover one row, so a warp takes 32 / LPR rows per
 // step and every lane loads; a thread block walks rows with a grid stride.
 // The same pass zero-fills what the main kernel adds into: row `row` of the packed fp32 dQ accumulator [rows, D] and
 // the turn counters (the reference leaves that to its runtime, which zero-fills "atomic add" outputs before the
 // launch: flash_attention_bwd.py:55-57).
 template <bool BF16, int LPR>
-__global__ void bwd_delta_kernel(const void* o, const void* d_o, float* delta, int64_t rows, int D, int64_t sb,
-                                 int64_t sh_, int64_t ss, int N, int S_q, float* zero_acc, unsigned int* counters,
-                                 int64_t n_counters) {
+__global__ void bwd_delta_kernel(const void* o, const void* d_o, float* delta, int64_t rows, int D, RowStrides so,
+                                 RowStrides sdo, int N, int S_q, float* zero_acc, unsigned int* counters, int64_t n_counters) {
   constexpr int RPW = 32 / LPR;
   const int lane = threadIdx.x & 31;
   const int sub = lane % LPR, rsub = lane / LPR;
@@ -946,9 +949,9 @@ __global__ void bwd_delta_kernel(const void* o, const void* d_o, float* delta, i
         z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
       }
       const int64_t bh = row / S_q;
-      const int64_t off = (bh / N) * sb + (bh % N) * sh_ + (row % S_q) * ss;
-      const uint4 a = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(o) + off + sub * 8);
-      const uint4 g = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(d_o) + off + sub * 8);
+      const int64_t bb = bh / N, hh = bh % N, rr = row % S_q;
+      const uint4 a = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(o) + bb * so.b + hh * so.h + rr * so.s + sub * 8);
+      const uint4 g = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(d_o) + bb * sdo.b + hh * sdo.h + rr * sdo.s + sub * 8);
       const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, gw[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -1015,32 +1018,22 @@ cudaError_t launch_fa_bwd(const BwdParams& p, bool bf16, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
-template <int LPR>
-static cudaError_t launch_bwd_delta_lpr(const void* o, const void* d_o, float* delta, int64_t rows, int D, int64_t sb,
-                                        int64_t sh_, int64_t ss, int N, int S_q, bool bf16, cudaStream_t stream,
-                                        float* zero_acc, unsigned int* counters, int64_t n_counters) {
+cudaError_t launch_bwd_delta(const void* o, const void* d_o, float* delta, int64_t rows, int D, const int64_t (&o_stride)[3],
+                             const int64_t (&do_stride)[3], int N, int S_q, bool bf16, cudaStream_t stream,
+                             float* zero_acc, unsigned int* counters, int64_t n_counters) {
+  const int lpr = D <= 64 ? 8 : (D <= 128 ? 16 : 32);       // lanes per row
   const int warps = 8;
-  const int64_t rows_per_block = static_cast<int64_t>(warps) * (32 / LPR);
+  const int64_t rows_per_block = static_cast<int64_t>(warps) * (32 / lpr);
   int64_t blocks = (rows + rows_per_block - 1) / rows_per_block;
   const int64_t cap = 148 * 32;   // a few waves of blocks; the grid stride covers the rest
   if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
-  if (bf16) bwd_delta_kernel<true, LPR><<<static_cast<unsigned>(blocks), warps * 32, 0, stream>>>(o, d_o, delta, rows, D, sb, sh_, ss, N, S_q, zero_acc, counters, n_counters);
-  else bwd_delta_kernel<false, LPR><<<static_cast<unsigned>(blocks), warps * 32, 0, stream>>>(o, d_o, delta, rows, D, sb, sh_, ss, N, S_q, zero_acc, counters, n_counters);
+  const RowStrides so = {o_stride[0], o_stride[1], o_stride[2]}, sdo = {do_stride[0], do_stride[1], do_stride[2]};
+  auto kern = lpr == 8 ? (bf16 ? bwd_delta_kernel<true, 8> : bwd_delta_kernel<false, 8>)
+              : lpr == 16 ? (bf16 ? bwd_delta_kernel<true, 16> : bwd_delta_kernel<false, 16>)
+                          : (bf16 ? bwd_delta_kernel<true, 32> : bwd_delta_kernel<false, 32>);
+  kern<<<static_cast<unsigned>(blocks), warps * 32, 0, stream>>>(o, d_o, delta, rows, D, so, sdo, N, S_q, zero_acc, counters, n_counters);
   return cudaGetLastError();
-}
-
-cudaError_t launch_bwd_delta(const void* o, const void* d_o, float* delta, int64_t rows, int D, int64_t o_stride_b,
-                             int64_t o_stride_h, int64_t o_stride_s, int N, int S_q, bool bf16,
-                             cudaStream_t stream, float* zero_acc, unsigned int* counters, int64_t n_counters) {
-  if (D <= 64)
-    return launch_bwd_delta_lpr<8>(o, d_o, delta, rows, D, o_stride_b, o_stride_h, o_stride_s, N, S_q, bf16, stream, zero_acc,
-                                   counters, n_counters);
-  if (D <= 128)
-    return launch_bwd_delta_lpr<16>(o, d_o, delta, rows, D, o_stride_b, o_stride_h, o_stride_s, N, S_q, bf16, stream, zero_acc,
-                                    counters, n_counters);
-  return launch_bwd_delta_lpr<32>(o, d_o, delta, rows, D, o_stride_b, o_stride_h, o_stride_s, N, S_q, bf16, stream, zero_acc,
-                                  counters, n_counters);
 }
 
 cudaError_t launch_bwd_convert_dq(const float* dq_acc, void* dq, int64_t n_elems, bool bf16, bool f32_out,

@@ -22,26 +22,27 @@ sizes are fixed inside the CUDA kernels.
 """
 from __future__ import annotations
 
-import torch
-
 from .... import ops as _ops
+from ...._lib import host as _host
 
 __all__ = ["get_flash_attention", "get_flash_attention_grad"]
 
 
-def _mask_tiles(attn_mask, enabled=True):
+def _mask_tiles(attn_mask):
     """Per-tile summary of a full attn_mask (made once per mask tensor, see ops.mask_tile_classes), with which the
     kernels read only the 128x128 tiles of the mask that are neither all 0 nor all 1; None for no mask / the tile form."""
-    if not enabled or attn_mask is None or _is_tile_mask(attn_mask) or not attn_mask.is_cuda:
+    if attn_mask is None or _is_tile_mask(attn_mask) or not attn_mask.is_cuda:
         return None
     return _ops.mask_tile_classes(attn_mask)
+
+
+_TILE_SHAPES = ((128, 128), (1, 128, 128))
 
 
 def _is_tile_mask(attn_mask):
     if attn_mask is None:
         return False
-    shp = tuple(attn_mask.shape)
-    return shp == (128, 128) or shp == (1, 128, 128)
+    return attn_mask.shape in _TILE_SHAPES
 
 
 def get_flash_attention_grad(prev_block_num=65536, next_block_num=65536, tiling_stgy_name='sparse',
@@ -66,42 +67,16 @@ def get_flash_attention_grad(prev_block_num=65536, next_block_num=65536, tiling_
     return fa_grad
 
 
-class _FlashAttentionFunction(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, query, key, value, attn_mask, dropout_mask, alibi_mask, cfg):
-        ctx.mask_tiles = _mask_tiles(attn_mask, cfg.get("classify_mask_tiles", True))
-        output, rowsum = _ops.fa_forward(
-            query, key, value, attn_mask, mask_tile128=_is_tile_mask(attn_mask), causal=cfg["causal"],
-            dropout_mask=dropout_mask, keep_prob=cfg["keep_prob"], alibi=alibi_mask,
-            prev_block_num=cfg["prev_block_num"], next_block_num=cfg["next_block_num"], scale=cfg["scale"],
-            tri_block=cfg.get("tri_block", 0), dropout_seed=cfg.get("dropout_seed"),
-            dropout_offset=cfg.get("dropout_offset", 0), mask_tiles=ctx.mask_tiles)
-        ctx.save_for_backward(query, key, value, output, rowsum,
-                              *(t for t in (attn_mask, dropout_mask, alibi_mask) if t is not None))
-        ctx.present = (attn_mask is not None, dropout_mask is not None, alibi_mask is not None)
-        ctx.cfg = cfg
-        ctx.mark_non_differentiable(rowsum)
-        return output, rowsum
-
-    @staticmethod
-    def backward(ctx, d_output, _d_rowsum):
-        saved = list(ctx.saved_tensors)
-        query, key, value, output, rowsum = saved[:5]
-        rest = saved[5:]
-        opt = []
-        for present in ctx.present:
-            opt.append(rest.pop(0) if present else None)
-        attn_mask, dropout_mask, alibi_mask = opt
-        cfg = ctx.cfg
-        dq, dk, dv = _ops.fa_backward(
-            query, key, value, output, rowsum, d_output.contiguous(), attn_mask,
-            mask_tile128=_is_tile_mask(attn_mask), causal=cfg["causal"], dropout_mask=dropout_mask,
-            keep_prob=cfg["keep_prob"], alibi=alibi_mask, prev_block_num=cfg["prev_block_num"],
-            next_block_num=cfg["next_block_num"], scale=cfg["scale"], grads_fp32=False,
-            tri_block=cfg.get("tri_block", 0), deterministic=cfg.get("deterministic", False),
-            dropout_seed=cfg.get("dropout_seed"), dropout_offset=cfg.get("dropout_offset", 0),
-            mask_tiles=ctx.mask_tiles)
-        return dq, dk, dv, None, None, None, None
+def _apply(query, key, value, attn_mask, dropout_mask, alibi_mask, causal, keep_prob, prev_block_num, next_block_num,
+           scale, tri_block=0, deterministic=False, dropout_seed=None, dropout_offset=0):
+    """The differentiable operator: (output, rowsum), by the native host path (its autograd node calls the grad
+    kernels and hands back dq, dk, dv in the input type)."""
+    tiles, tile_form = None, False
+    if attn_mask is not None:
+        tile_form = _is_tile_mask(attn_mask)
+        tiles = _mask_tiles(attn_mask)
+    return _host().fa_apply(query, key, value, attn_mask, dropout_mask, alibi_mask, tiles, tile_form, causal, keep_prob,
+                            prev_block_num, next_block_num, scale, tri_block, deterministic, dropout_seed, dropout_offset)
 
 
 def get_flash_attention(prev_block_num=65536, next_block_num=65536, tiling_stgy_name='sparse',
@@ -117,10 +92,8 @@ def get_flash_attention(prev_block_num=65536, next_block_num=65536, tiling_stgy_
         # generate the triangle and the tensor is not read
         if implicit_causal:
             attn_mask = None
-        cfg = dict(prev_block_num=prev_block_num, next_block_num=next_block_num, scale=scale,
-                   causal=causal or implicit_causal, keep_prob=keep_prob, deterministic=deterministic,
-                   dropout_seed=dropout_seed, dropout_offset=dropout_offset)
-        return _FlashAttentionFunction.apply(query, key, value, attn_mask, dropout_mask, alibi_mask, cfg)
+        return _apply(query, key, value, attn_mask, dropout_mask, alibi_mask, causal or implicit_causal, keep_prob,
+                      prev_block_num, next_block_num, scale, 0, deterministic, dropout_seed, dropout_offset)
 
     fa_forward.prev_block_num = prev_block_num
     fa_forward.next_block_num = next_block_num

@@ -11,7 +11,7 @@ import torch
 
 from . import _lib
 from ._lib import (ACCT_BF16, ACCT_F16, ACCT_U8, BAND_UNBOUNDED, FLAG_DETERMINISTIC, FLAG_DROPOUT_PHILOX, FLAG_GRAD_F32, MASK_FULL, MASK_NONE,
-                   MASK_TILE128, DecodeArgs, FaArgs, FaBwdIO, InferArgs, check, load)
+                   MASK_TILE128, DecodeArgs, FaArgs, FaBwdIO, check, host, load)
 
 _DTYPES = {torch.float16: ACCT_F16, torch.bfloat16: ACCT_BF16, torch.uint8: ACCT_U8, torch.bool: ACCT_U8}
 
@@ -309,34 +309,7 @@ def dropout_mask(B, N, S_q, S_k, keep_prob, dropout_seed, dropout_offset=0, devi
 
 def infer_prefill(q, k, v, *, causal=False, scale=1.0, seq_lens=None):
     """The inference op y = softmax(scale * q k^T) v on rank-3 [B*N,S,D] or rank-4 [B,N,S,D] input."""
-    lib = load()
-    for name, t in (("q", q), ("k", k), ("v", v)):
-        _require_cuda(name, t)
-    rank = q.dim()
-    if rank not in (3, 4):
-        raise ValueError("q must have rank 3 or 4")
-    if k.dim() != rank or v.dim() != rank or k.shape != v.shape:
-        raise ValueError("k and v must have q's rank and one shape")
-    q4, k4, v4 = (t.contiguous() if rank == 4 else t.contiguous().unsqueeze(0) for t in (q, k, v))
-    if q4.shape[0] != k4.shape[0] or q4.shape[3] != k4.shape[3] or q4.shape[1] % k4.shape[1] != 0:
-        raise ValueError("q and k must agree on batch and head_dim, and k's head count must divide q's")
-    y = torch.empty_like(q4)
-    a = InferArgs()
-    a.dtype = _DTYPES[q.dtype] if q.dtype in (torch.float16, torch.bfloat16) else -1
-    a.rank = rank
-    a.B, a.N, a.S_q, a.D = q4.shape[0], q4.shape[1], q4.shape[2], q4.shape[3]
-    a.S_k = k4.shape[2]
-    a.N_kv = k4.shape[1]
-    a.q, a.k, a.v, a.y = q4.data_ptr(), k4.data_ptr(), v4.data_ptr(), y.data_ptr()
-    a.causal = 1 if causal else 0
-    a.scale = float(scale)
-    sl = None
-    if seq_lens is not None:
-        sl = seq_lens.to(torch.int32).contiguous()
-        a.seq_lens = sl.data_ptr()
-    with torch.cuda.device(q.device):
-        check(lib.acct_infer_prefill(C.byref(a), _stream()))
-    return y if rank == 4 else y.squeeze(0)
+    return host().infer_prefill(q, k, v, causal, scale, seq_lens)
 
 
 class DecodeWorkspace:
@@ -356,49 +329,9 @@ def infer_decode(q, k_cache, v_cache, seq_lens=None, *, scale=None, num_splits=0
 
     With ``block_table`` ([B, max_pages] int32) the caches are page pools [num_pages, N_kv, page_size, D] and key
     position s of sequence b is row s % page_size of page block_table[b, s // page_size]."""
-    lib = load()
-    for name, t in (("q", q), ("k_cache", k_cache), ("v_cache", v_cache)):
-        _require_cuda(name, t)
-    B, N, one, D = q.shape
-    if one != 1:
-        raise ValueError("decode takes one query token: q must be [B, N, 1, D]")
-    N_kv = k_cache.shape[1]
-    paged = block_table is not None
-    if (k_cache.shape != v_cache.shape or (not paged and k_cache.shape[0] != B) or k_cache.shape[3] != D or N_kv < 1
-            or N % N_kv != 0):
-        raise ValueError("k_cache and v_cache must be [B, N_kv, S_max, D] (or page pools [pages, N_kv, page_size, D]) "
-                         "with N_kv dividing q's head count")
-    if k_cache.stride() != v_cache.stride():
-        raise ValueError("k_cache and v_cache must share strides")
-    q = q.contiguous()
-    y = out if out is not None else torch.empty_like(q)
     if workspace is None:
-        workspace = DecodeWorkspace(B, N, D, q.device, num_splits)
-    a = DecodeArgs()
-    a.dtype = _DTYPES.get(q.dtype, -1)
-    a.B, a.N, a.D = B, N, D
-    a.N_kv = N_kv
-    bt = None
-    if paged:
-        _require_cuda("block_table", block_table)
-        bt = block_table.to(torch.int32).contiguous()
-        if bt.dim() != 2 or bt.shape[0] != B:
-            raise ValueError("block_table must be [B, max_pages]")
-        a.block_table = bt.data_ptr()
-        a.page_size, a.max_pages = k_cache.shape[2], bt.shape[1]
-        a.S_max = a.page_size * a.max_pages
-    else:
-        a.S_max = k_cache.shape[2]
-    a.q, a.k_cache, a.v_cache, a.y = q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), y.data_ptr()
-    a.kv_stride = _strides3(k_cache)
-    sl = None
-    if seq_lens is not None:
-        sl = seq_lens.to(torch.int32).contiguous()
-        a.seq_lens = sl.data_ptr()
-    a.scale = float(scale if scale is not None else 1.0 / math.sqrt(D))
-    a.num_splits = num_splits
-    a.workspace, a.workspace_bytes = workspace.buf.data_ptr(), workspace.nbytes
-    with torch.cuda.device(q.device):
-        check(lib.acct_infer_decode(C.byref(a), _stream()))
-    del bt, sl
-    return y
+        for name, t in (("q", q), ("k_cache", k_cache), ("v_cache", v_cache)):
+            _require_cuda(name, t)
+        workspace = DecodeWorkspace(q.shape[0], q.shape[1], q.shape[3], q.device, num_splits)
+    return host().infer_decode(q, k_cache, v_cache, seq_lens, scale if scale is not None else 1.0 / math.sqrt(q.shape[-1]),
+                               num_splits, workspace.buf, out, block_table)

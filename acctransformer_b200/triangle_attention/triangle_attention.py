@@ -20,7 +20,7 @@ import torch
 
 from .. import ops as _ops
 from ..flash_attention.nn.layer.flash_attention import _draw_dropout_key
-from ..flash_attention.ops.flash_attention.flash_attention_impl import _FlashAttentionFunction
+from ..flash_attention.ops.flash_attention.flash_attention_impl import _apply
 
 __all__ = ["TriangleAttention"]
 
@@ -75,11 +75,8 @@ class TriangleAttention(torch.nn.Module):
         causal = self.assume_causal or (self.detect_causal_mask and attention_mask is not None
                                         and attention_mask.is_cuda and not torch.cuda.is_current_stream_capturing()
                                         and _ops.mask_is_causal(attention_mask))
-        cfg = dict(prev_block_num=65536, next_block_num=65536, scale=1.0, causal=causal,
-                   keep_prob=self.keep_prob, tri_block=0 if causal else self.block_size,
-                   dropout_seed=seed, dropout_offset=offset)
-        mask = None if causal else attention_mask
-        out, _ = _FlashAttentionFunction.apply(query, key, value, mask, drop_mask, None, cfg)
+        out, _ = _apply(query, key, value, None if causal else attention_mask, drop_mask, None, causal, self.keep_prob,
+                        65536, 65536, 1.0, 0 if causal else self.block_size, False, seed, offset)
         return out
 
     forward = construct

@@ -217,6 +217,11 @@ ACCT_API size_t acct_fa_bwd_workspace_bytes(const acct_fa_args* a);
 /* Backward: reads q,k,v,o,lse,d_o (+ the same mask/dropout/alibi/band arguments as the forward). */
 ACCT_API int acct_fa_bwd(const acct_fa_args* a, const acct_fa_bwd_io* g, void* stream);
 
+/* The same with an output gradient in a layout of its own: d_o_stride = its element strides of B, N, S (positive
+ * multiples of 8; NULL or 0 = those of `o`).  Behind a transpose back to [B, S, N*D], which is what an output
+ * projection reads, the gradient arrives as such a view and need not be copied first. */
+ACCT_API int acct_fa_bwd_strided(const acct_fa_args* a, const acct_fa_bwd_io* g, const int64_t* d_o_stride, void* stream);
+
 /* Inference op  y = softmax(scale * q k^T) v.
  *
  * Replaces  FlashAttentionTik(q, k, v) -> y

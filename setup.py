@@ -50,7 +50,7 @@ setup(
     version="0.2.0",
     description="FlashAttention2 / TriangleAttention / inference attention of acctransformer as hand-written CUDA for NVIDIA B200",
     packages=find_packages(where=".", include=["acctransformer", "acctransformer.*", "acctransformer_b200", "acctransformer_b200.*"]),
-    package_data={"acctransformer_b200": ["libacct_b200.so", "csrc/*.cu", "csrc/*.cuh"]},
+    package_data={"acctransformer_b200": ["libacct_b200.so", "_torch_host.so", "csrc/*.cu", "csrc/*.cuh", "csrc/*.cpp"]},
     data_files=[("include", ["include/acct_b200.h"])],
     python_requires=">=3.9",
     install_requires=["torch"],
