@@ -13,6 +13,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include "decode_common.cuh"
 #include "fa_kernels.cuh"
 
 namespace acct {
@@ -74,7 +75,8 @@ __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
 
 // G = query heads per key/value head (grouped-query attention): the G heads of a group share one pass over their
 // cache rows, so the cache is read once per group instead of once per query head.
-template <int LPR, bool BF16, int G>
+// CL: the parts of a slice are one cluster (decode_common.cuh)
+template <int LPR, bool BF16, int G, bool CL>
 __global__ void __launch_bounds__(kDecodeThreads) decode_split_kernel(const DecodeParams p) {
   constexpr int RPW = 32 / LPR;                 // cache rows per warp per load instruction
   constexpr int kWarps = kDecodeThreads / 32;
@@ -84,6 +86,7 @@ __global__ void __launch_bounds__(kDecodeThreads) decode_split_kernel(const Deco
 
   __shared__ float s_m[G][kGroups], s_l[G][kGroups];
   __shared__ float s_acc[G][kGroups][DMAX];
+  __shared__ float s_part[CL ? G : 1][CL ? DMAX : 1], s_pm[G], s_pl[G];    // this part's result, read by the cluster's other blocks
 
   const int split = blockIdx.x;
   const int n_kv = p.N / G;
@@ -357,16 +360,23 @@ __global__ void __launch_bounds__(kDecodeThreads) decode_split_kernel(const Deco
         const float w = (s_m[g][i] == -INFINITY) ? 0.f : ex2(s_m[g][i] - big);
         a = fmaf(s_acc[g][i][t], w, a);
       }
-      p.part_acc[slot * p.D + t] = a;
+      if constexpr (CL) s_part[g][t] = a;
+      else p.part_acc[slot * p.D + t] = a;
     }
     if (threadIdx.x == 0) {
       float lsum = 0.f;
 #pragma unroll
       for (int i = 0; i < kGroups; ++i) lsum += (s_m[g][i] == -INFINITY) ? 0.f : s_l[g][i] * ex2(s_m[g][i] - big);
-      p.part_ml[slot * 2] = big;
-      p.part_ml[slot * 2 + 1] = lsum;
+      if constexpr (CL) {
+        s_pm[g] = big;
+        s_pl[g] = lsum;
+      } else {
+        p.part_ml[slot * 2] = big;
+        p.part_ml[slot * 2 + 1] = lsum;
+      }
     }
   }
+  if constexpr (CL) cluster_merge<BF16>(p, &s_part[0][0], s_pm, s_pl, DMAX, b, h_kv, kDecodeThreads);
 }
 
 template <bool BF16>
@@ -399,11 +409,10 @@ cudaError_t launch_merge(const DecodeParams& p, bool bf16, cudaStream_t stream) 
 
 template <int LPR, int G>
 cudaError_t launch_decode_g(const DecodeParams& p, bool bf16, cudaStream_t stream) {
-  dim3 grid(p.splits, p.B * (p.N / G));
-  if (bf16) decode_split_kernel<LPR, true, G><<<grid, kDecodeThreads, 0, stream>>>(p);
-  else decode_split_kernel<LPR, false, G><<<grid, kDecodeThreads, 0, stream>>>(p);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
+  auto kern = p.clustered ? (bf16 ? decode_split_kernel<LPR, true, G, true> : decode_split_kernel<LPR, false, G, true>)
+                          : (bf16 ? decode_split_kernel<LPR, true, G, false> : decode_split_kernel<LPR, false, G, false>);
+  const cudaError_t e = launch_parts(kern, p, p.B * (p.N / G), kDecodeThreads, 0, stream);
+  if (e != cudaSuccess || p.clustered) return e;
   return launch_merge(p, bf16, stream);
 }
 
@@ -424,7 +433,7 @@ cudaError_t launch_decode(const DecodeParams& p, bool bf16, cudaStream_t stream)
   // several query heads per cache head, head_dim <= 128: the group goes on the rows of a tensor-core MMA
   if (p.kv_group >= kDecodeGqaMinGroup && p.D <= 128) {
     cudaError_t e = launch_decode_gqa_split(p, bf16, stream);
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess || p.clustered) return e;
     return launch_merge(p, bf16, stream);
   }
   if (p.D <= 64) return launch_decode_lpr<8>(p, bf16, stream);

@@ -21,6 +21,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include "decode_common.cuh"
 #include "fa_kernels.cuh"
 
 namespace acct {
@@ -81,7 +82,8 @@ __device__ __forceinline__ uint32_t pack16(float a, float b) {
 
 // DPAD: head_dim rounded up to 64 or 128 (cache rows are zero-filled past head_dim in shared memory).
 // UPPER: the group has more than 8 query heads, i.e. rows 8..15 of the MMAs carry heads too.
-template <int DPAD, bool BF16, bool UPPER>
+// CL: the parts of a slice are one cluster (decode_common.cuh).
+template <int DPAD, bool BF16, bool UPPER, bool CL>
 __global__ void __launch_bounds__(kGqaThreads) decode_gqa_kernel(const DecodeParams p) {
   constexpr int kRowBytes = DPAD * 2 + 16;               // 16 bytes of padding: ldmatrix rows fall on distinct banks
   constexpr int kTileBytes = kTileRows * kRowBytes;
@@ -270,6 +272,9 @@ __global__ void __launch_bounds__(kGqaThreads) decode_gqa_kernel(const DecodePar
   float* s_acc = reinterpret_cast<float*>(gsm);                      // [warp][16 heads][DPAD]
   float* s_m = s_acc + kGqaWarps * 16 * DPAD;                        // [warp][16]
   float* s_l = s_m + kGqaWarps * 16;
+  float* s_part = s_l + kGqaWarps * 16;                              // [16][DPAD]: this part's result, for the cluster
+  float* s_pm = s_part + 16 * DPAD;
+  float* s_pl = s_pm + 16;
 #pragma unroll
   for (int hi = 0; hi < (UPPER ? 2 : 1); ++hi) {
     const int head = g + 8 * hi;
@@ -292,7 +297,8 @@ __global__ void __launch_bounds__(kGqaThreads) decode_gqa_kernel(const DecodePar
         const float mw = s_m[w * 16 + head];
         a = fmaf(s_acc[(w * 16 + head) * DPAD + d], mw == -INFINITY ? 0.f : ex2f(mw - big), a);
       }
-      p.part_acc[slot * p.D + d] = a;
+      if constexpr (CL) s_part[head * DPAD + d] = a;
+      else p.part_acc[slot * p.D + d] = a;
     }
     if (threadIdx.x == 0) {
       float lsum = 0.f;
@@ -301,26 +307,31 @@ __global__ void __launch_bounds__(kGqaThreads) decode_gqa_kernel(const DecodePar
         const float mw = s_m[w * 16 + head];
         lsum += mw == -INFINITY ? 0.f : s_l[w * 16 + head] * ex2f(mw - big);
       }
-      p.part_ml[slot * 2] = big;
-      p.part_ml[slot * 2 + 1] = lsum;
+      if constexpr (CL) {
+        s_pm[head] = big;
+        s_pl[head] = lsum;
+      } else {
+        p.part_ml[slot * 2] = big;
+        p.part_ml[slot * 2 + 1] = lsum;
+      }
     }
   }
+  if constexpr (CL) cluster_merge<BF16>(p, s_part, s_pm, s_pl, DPAD, b, h_kv, kGqaThreads);
 }
 
 template <int DPAD>
 cudaError_t launch_gqa(const DecodeParams& p, bool bf16, cudaStream_t stream) {
   const size_t ring = static_cast<size_t>(kGqaWarps) * kRing * 2 * kTileRows * (DPAD * 2 + 16);
-  const size_t merge = static_cast<size_t>(kGqaWarps) * 16 * (DPAD + 2) * sizeof(float);
+  const size_t merge = static_cast<size_t>(kGqaWarps + 1) * 16 * (DPAD + 2) * sizeof(float);
   const size_t smem = ring > merge ? ring : merge;
   const bool upper = p.kv_group > 8;
-  void (*kern)(const DecodeParams) =
-      bf16 ? (upper ? decode_gqa_kernel<DPAD, true, true> : decode_gqa_kernel<DPAD, true, false>)
-           : (upper ? decode_gqa_kernel<DPAD, false, true> : decode_gqa_kernel<DPAD, false, false>);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+#define ACCT_GQA(BF, UP) (p.clustered ? decode_gqa_kernel<DPAD, BF, UP, true> : decode_gqa_kernel<DPAD, BF, UP, false>)
+  void (*kern)(const DecodeParams) = bf16 ? (upper ? ACCT_GQA(true, true) : ACCT_GQA(true, false))
+                                          : (upper ? ACCT_GQA(false, true) : ACCT_GQA(false, false));
+#undef ACCT_GQA
+  cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), smem);
   if (e != cudaSuccess) return e;
-  dim3 grid(p.splits, p.B * (p.N / p.kv_group));
-  kern<<<grid, kGqaThreads, smem, stream>>>(p);
-  return cudaGetLastError();
+  return launch_parts(kern, p, p.B * (p.N / p.kv_group), kGqaThreads, smem, stream);
 }
 
 }  // namespace

@@ -988,16 +988,12 @@ __global__ void bwd_convert_kernel(const float* __restrict__ src, void* __restri
   }
 }
 
-cudaError_t launch_fa_bwd(const BwdParams& p, bool bf16, cudaStream_t stream) {
+cudaError_t launch_fa_bwd(const BwdParams& p, bool bf16, int sm_count, cudaStream_t stream) {
   const int dpad = p.D <= 64 ? 64 : 128;
   const size_t smem = static_cast<size_t>(3 + kStages) * (dpad / 64) * 16384 + 2 * 32768 + sizeof(BwdShared);
   // persistent CTAs, one per SM (tensor memory and shared memory admit no more), fewer if there is less work
   const long long items = static_cast<long long>((p.S_k + kTile - 1) / kTile) * p.B * (p.N / p.kv_group);
-  int dev = 0, sms = 0;
-  cudaError_t e0 = cudaGetDevice(&dev);
-  if (e0 == cudaSuccess) e0 = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e0 != cudaSuccess) return e0;
-  dim3 grid(static_cast<unsigned>(items < sms ? items : sms));
+  dim3 grid(static_cast<unsigned>(items < sm_count ? items : sm_count));
   // (row groups of a multiple of 128 rows never cut a tile: the tile ranges alone take care of them)
   const bool masked = p.mods.mask_kind != 0 || (p.mods.tri_block > 0 && p.mods.tri_block % kTile != 0);
   const bool drop_u8_bits = p.mods.drop != nullptr && p.mods.drop_dtype == 2 /*U8*/ && p.S_k % 4 == 0 &&
@@ -1012,7 +1008,7 @@ cudaError_t launch_fa_bwd(const BwdParams& p, bool bf16, cudaStream_t stream) {
   else kern = bf16 ? ACCT_BWD_PICK(128, true) : ACCT_BWD_PICK(128, false);
 #undef ACCT_BWD_PICK
 #undef ACCT_BWD_DROP
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), smem);
   if (e != cudaSuccess) return e;
   kern<<<grid, kBwdThreads, smem, stream>>>(p);
   return cudaGetLastError();

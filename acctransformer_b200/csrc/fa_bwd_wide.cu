@@ -477,7 +477,7 @@ cudaError_t launch_fa_bwd_wide(const BwdParams& p, bool bf16, cudaStream_t strea
   const size_t smem = 2 * kKvTileBytes + 2 * kSubTileBytes + 2 * 16384 + sizeof(WideShared);
   dim3 grid(2 * ((p.S_k + kTile - 1) / kTile), p.B * (p.N / p.kv_group));
   void (*kern)(const BwdParams) = bf16 ? fa_bwd_wide_kernel<true> : fa_bwd_wide_kernel<false>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), smem);
   if (e != cudaSuccess) return e;
   kern<<<grid, kWThreads, smem, stream>>>(p);
   return cudaGetLastError();

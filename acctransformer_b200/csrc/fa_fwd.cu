@@ -746,7 +746,7 @@ cudaError_t launch_mask_classify(const void* mask, int dtype, int batch, int S_q
   return cudaGetLastError();
 }
 
-cudaError_t launch_fa_fwd(const FwdParams& p, bool bf16, cudaStream_t stream) {
+cudaError_t launch_fa_fwd(const FwdParams& p, bool bf16, int sm_count, cudaStream_t stream) {
   const int dpad = p.D <= 64 ? 64 : (p.D <= 128 ? 128 : 256);
   const int nq = dpad > 128 ? 1 : 2, stages = dpad > 128 ? 1 : kStages;
   const size_t smem = static_cast<size_t>(nq + 2 * stages) * (dpad / 64) * 16384 + 1024;
@@ -758,8 +758,7 @@ cudaError_t launch_fa_fwd(const FwdParams& p, bool bf16, cudaStream_t stream) {
   // what its thread blocks share through L2, stay small at such lengths; bounded by 48 MB all the same).
   FwdParams pp = p;
   {
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = sm_count;
     long long group = 8;
     if (16ll * n_pairs <= sms) {
       const long long unit_bytes = 4ll * p.S_k * p.D;                    // K and V of one slice, 16-bit
@@ -791,7 +790,7 @@ cudaError_t launch_fa_fwd(const FwdParams& p, bool bf16, cudaStream_t stream) {
   }
 #undef ACCT_FWD_BF
 #undef ACCT_FWD_DROP
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), smem);
   if (e != cudaSuccess) return e;
   kern<<<grid, kFwdThreads, smem, stream>>>(pp);
   return cudaGetLastError();

@@ -77,6 +77,7 @@ struct DecodeParams {
   const int* block_table;           // [B, max_pages] page numbers, or nullptr: contiguous caches
   int page_shift, max_pages;        // rows per page = 1 << page_shift; kv_stride_b is then the page stride
   int splits;
+  int clustered;                    // 1: the parts of a slice are one thread-block cluster and merge through its shared memory
   float scale_log2;
 };
 
@@ -89,9 +90,13 @@ cudaError_t launch_mask_check(const void* mask, int dtype, int batch, int S_q, i
 cudaError_t launch_mask_classify(const void* mask, int dtype, int batch, int S_q, int S_k, uint8_t* tiles,
                                  cudaStream_t stream);
 
+// Raises a kernel's dynamic shared memory limit, once per thread, kernel and device (the call costs the host about as
+// much as a launch argument block, and every operator call would repeat it).
+cudaError_t allow_smem(const void* kernel, size_t bytes);
+
 // Launchers: return cudaGetLastError() of the launch.
-cudaError_t launch_fa_fwd(const FwdParams& p, bool bf16, cudaStream_t stream);
-cudaError_t launch_fa_bwd(const BwdParams& p, bool bf16, cudaStream_t stream);
+cudaError_t launch_fa_fwd(const FwdParams& p, bool bf16, int sm_count, cudaStream_t stream);
+cudaError_t launch_fa_bwd(const BwdParams& p, bool bf16, int sm_count, cudaStream_t stream);
 // head_dim in (128, 256]: Q / dO maps with 64-row boxes, the dQ map with a 32 x 64 box, two turn counters per Q tile
 cudaError_t launch_fa_bwd_wide(const BwdParams& p, bool bf16, cudaStream_t stream);
 // writes the {0,1} mask the kernels' in-kernel dropout uses, [units, S_q, S_k] uint8 (units = B*N)

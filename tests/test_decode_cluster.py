@@ -1,0 +1,39 @@
+"""Decoding over few and short contexts, where the parts of a slice form one thread-block cluster that merges them."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import attention_ref as ref
+
+pytestmark = pytest.mark.gpu
+
+
+# one part (<= 128 keys), two (129 keys: the second part is all but empty), eight, and more slices than leave room for
+# eight parts; head groups on CUDA cores, on MMA rows 0-7 and 0-15; sequences of one key, so that most parts are empty
+@pytest.mark.parametrize("B,n_kv,group,S,D,dtype", [
+    (1, 1, 1, 1, 64, "float16"), (2, 3, 1, 128, 128, "bfloat16"), (2, 2, 1, 129, 40, "float16"),
+    (1, 2, 1, 1100, 256, "float16"), (3, 2, 4, 4096, 128, "bfloat16"), (2, 1, 16, 700, 64, "float16"),
+    (4, 16, 4, 1000, 128, "float16"), (8, 32, 1, 515, 80, "bfloat16"), (2, 2, 8, 257, 160, "float16"),
+])
+def test_clustered_parts_against_the_oracle(B, n_kv, group, S, D, dtype):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from acctransformer_b200 import _lib, ops
+    dt = getattr(torch, dtype)
+    g = torch.Generator().manual_seed(S + D)
+    q = torch.randn(B, n_kv * group, 1, D, generator=g).to(dt)
+    k, v = (torch.randn(B, n_kv, S, D, generator=g).to(dt) for _ in range(2))
+    lens = torch.randint(1, S + 1, (B,), generator=g, dtype=torch.int32)
+    lens[0], lens[-1] = 1, S
+    scale = 1.0 / math.sqrt(D)
+    y = ops.infer_decode(q.cuda(), k.cuda(), v.cuda(), lens.cuda(), scale=scale)
+    torch.cuda.synchronize()
+    _lib.device_status()
+    want = ref.decode_ref(q.float().numpy(), k.float().numpy().repeat(group, axis=1), v.float().numpy().repeat(group, axis=1),
+                          lens.numpy(), scale)
+    # results up to about 4 in size, rounded to 16 bits (half a unit: 2^-10 fp16, 2^-7 bf16); with head groups the
+    # probabilities are rounded to 16 bits too (at most 2^-11 / 2^-8 of the largest |v|, about 4)
+    tol = 4e-3 if dtype == "float16" else 3e-2
+    assert float(np.max(np.abs(y.float().cpu().numpy() - want))) <= tol
