@@ -194,7 +194,7 @@ struct FaBackward : public torch::autograd::Node {
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
     TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
-    variable_list out(3);
+    variable_list out(6);
     Tensor d_o = grads[0];
     if (!d_o.defined()) return out;
     const Tensor q = q_.unpack(), k = k_.unpack(), v = v_.unpack(), o = o_.unpack(shared_from_this()), lse = lse_.unpack();
@@ -206,7 +206,7 @@ struct FaBackward : public torch::autograd::Node {
     for (int i = 0; i < 3; ++i) as_is = as_is && ds[i] > 0 && ds[i] % 8 == 0;
     if (!as_is) {
       d_o = d_o.contiguous();
-      for (int i = 0; i < 3; ++i) ds[i] = d_o.stride(i);
+      ds[0] = ds[1] = ds[2] = 0;      // packed (the stride of a dimension of size 1 may be anything: not read)
     }
     acct_fa_args a;
     fill_args(a, q, k, v, o, lse, mask, drop, alibi, tiles, cfg);
@@ -303,9 +303,15 @@ PyObject* py_fa_apply(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (args[15] != Py_None) {
     c.has_seed = true;
     c.seed = PyLong_AsUnsignedLongLongMask(args[15]);
-    c.offset = static_cast<uint64_t>(int_arg(args[16]));
+    c.offset = PyLong_AsUnsignedLongLongMask(args[16]);
+    if (PyErr_Occurred()) throw python_error();
   }
   Tensor o, lse;
+  // as a Python autograd Function without a `jvp` does; a tangent would be dropped silently otherwise
+  for (const Tensor* t : {&q, &k, &v, &std::as_const(mask), &std::as_const(drop), &std::as_const(alibi)})
+    TORCH_CHECK_NOT_IMPLEMENTED(!t->defined() || !t->_fw_grad(/*level=*/0).defined(),
+                                "the flash attention operator does not support forward mode AD");
+  const variable_list inputs = {q, k, v, mask, drop, alibi};
   {
     pybind11::gil_scoped_release no_gil;
     {
@@ -318,9 +324,10 @@ PyObject* py_fa_apply(PyObject*, PyObject* const* args, Py_ssize_t n) {
       fill_args(a, q, k, v, o, lse, mask, drop, alibi, tiles, c);
       check(g_lib.fa_fwd(&a, stream_of(q)));
     }
-    if (torch::autograd::compute_requires_grad(q, k, v)) {
+    // (an optional input may require a gradient too: it gets none, but the output is part of the graph)
+    if (torch::autograd::compute_requires_grad(inputs)) {
       auto node = std::shared_ptr<FaBackward>(new FaBackward(), torch::autograd::deleteNode);
-      node->set_next_edges(torch::autograd::collect_next_edges(q, k, v));
+      node->set_next_edges(torch::autograd::collect_next_edges(inputs));
       node->cfg = c;
       node->q_ = SavedVariable(q, false);
       node->k_ = SavedVariable(k, false);

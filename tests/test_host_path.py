@@ -1,0 +1,57 @@
+"""The native host path of the cells takes and refuses what a Python autograd Function around the operator does."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(B, N, S, D, seed=0):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return [torch.randn(B, N, S, D, device="cuda", dtype=torch.float16, generator=g) for _ in range(4)]
+
+
+def _layer(D, **kw):
+    from acctransformer_b200 import FlashAttention
+    return FlashAttention(D, **kw)
+
+
+# an output gradient whose head dimension has size 1 and a stride that means nothing (1), one whose rows are not
+# 16-byte aligned, one expanded from a scalar
+@pytest.mark.parametrize("form", ["size-one stride", "misaligned", "expanded"])
+def test_output_gradient_in_any_layout(form):
+    q, k, v, d_o = _inputs(2, 1, 130, 64)
+    if form == "size-one stride":
+        odd = d_o.view(2, 130, 64).clone().unsqueeze(3).permute(0, 3, 1, 2)
+        assert odd.stride(1) == 1
+    elif form == "misaligned":
+        odd = d_o.new_empty(2, 1, 130, 65)[..., 1:]
+        odd.copy_(d_o)
+    else:
+        d_o = torch.full_like(d_o, 0.5)
+        odd = torch.full((), 0.5, device="cuda", dtype=d_o.dtype).expand(2, 1, 130, 64)
+    q, k, v = (t.requires_grad_() for t in (q, k, v))
+    out = _layer(64)(q, k, v)
+    want = torch.autograd.grad(out, (q, k, v), d_o, retain_graph=True)
+    got = torch.autograd.grad(out, (q, k, v), odd)
+    # dk and dv are reproducible; dq is summed over two K/V tiles, and a sum of two does not depend on the order
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
+def test_optional_input_that_requires_a_gradient_is_part_of_the_graph():
+    q, k, v, d_o = _inputs(1, 2, 128, 64)
+    alibi = torch.zeros(1, 2, 1, 128, device="cuda", dtype=torch.float16, requires_grad=True)
+    out = _layer(64, alibi=True)(q, k, v, None, alibi)
+    assert out.requires_grad
+    out.backward(d_o)
+    assert alibi.grad is None
+
+
+def test_forward_mode_is_refused():
+    import torch.autograd.forward_ad as fwad
+    q, k, v, t = _inputs(1, 2, 128, 64)
+    with fwad.dual_level():
+        with pytest.raises(NotImplementedError):
+            _layer(64)(fwad.make_dual(q, t), k, v)
