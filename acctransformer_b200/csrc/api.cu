@@ -266,8 +266,25 @@ unsigned int dropout_threshold(float keep_prob) {
   return static_cast<unsigned int>(t < 1 ? 1 : (t > 256 ? 256 : t));
 }
 
-ScoreMods make_mods(const acct_fa_args* a) {
+// A mask plan pays where a mask tensor with a summary is the only thing that limits the scores and there is enough work:
+// its passes cost 8 us and one read of q, k and v, a tile pair of forward and backward about 6 us on its SM.  3 000 tokens of
+// four documents, 2 x 32 heads of 128 (36 864 tile pairs): forward and backward 1 476 -> 479 us.  A band, valid lengths, row groups and alibi set limits or add terms that the bounds do not
+// cover; a dropout tensor may hold any factor.
+constexpr int64_t kPlanMinTilePairs = 8192;
+constexpr int64_t kPlanMaxMaskTiles = 16384;      // 64 MB of bits (an eighth of the mask's own size in 16 bits, twice)
+bool plan_applies(const acct_fa_args* a) {
+  if (a->mask_kind != ACCT_MASK_FULL || a->mask_tiles == nullptr || a->causal || a->alibi || a->alibi_slopes || a->seq_lens ||
+      a->tri_block > 0 || a->dropout_mask || a->prev_block_num < ACCT_BAND_UNBOUNDED || a->next_block_num < ACCT_BAND_UNBOUNDED)
+    return false;
+  const int64_t tq = (static_cast<int64_t>(a->S_q) + kTile - 1) / kTile, tk = (static_cast<int64_t>(a->S_k) + kTile - 1) / kTile;
+  return tq <= kPlanTiles && tk <= kPlanTiles && a->mask_batch * tq * tk <= kPlanMaxMaskTiles &&
+         static_cast<int64_t>(a->B) * a->N * tq * tk >= kPlanMinTilePairs;
+}
+
+ScoreMods make_mods(const acct_fa_args* a, const void* plan = nullptr) {
   ScoreMods m;
+  memset(&m.plan, 0, sizeof(m.plan));
+  if (plan != nullptr && plan_applies(a)) plan_parts(const_cast<void*>(plan), a->mask_batch, a->S_q, a->S_k, &m.plan);
   m.causal = a->causal ? 1 : 0;
   m.prev_block_num = a->prev_block_num >= ACCT_BAND_UNBOUNDED ? ACCT_BAND_UNBOUNDED : a->prev_block_num;
   m.next_block_num = a->next_block_num >= ACCT_BAND_UNBOUNDED ? ACCT_BAND_UNBOUNDED : a->next_block_num;
@@ -411,7 +428,36 @@ int acct_mask_classify_tiles(const void* mask, int32_t mask_dtype, int32_t mask_
   return ACCT_OK;
 }
 
-int acct_fa_fwd(const acct_fa_args* a, void* stream) {
+size_t acct_mask_plan_bytes(const acct_fa_args* a) {
+  if (a == nullptr || a->B <= 0 || a->N <= 0 || a->S_q <= 0 || a->S_k <= 0 || !plan_applies(a)) return 0;
+  PlanParts parts;
+  return plan_parts(nullptr, a->mask_batch, a->S_q, a->S_k, &parts);
+}
+
+int acct_mask_plan(const acct_fa_args* a, void* plan, void* stream) {
+  Strides st;
+  int rc = validate_fa(a, &st);
+  if (rc) return rc;
+  if (plan == nullptr) return fail(ACCT_ERR_NULL, "plan is NULL");
+  if (!aligned16(plan)) return fail(ACCT_ERR_ALIGN, "plan must be 16-byte aligned");
+  if (!plan_applies(a)) return fail(ACCT_ERR_SHAPE, "no mask plan for this call (acct_mask_plan_bytes returns 0)");
+  PerDevice* dev = nullptr;
+  if ((rc = init_device(&dev))) return rc;
+  const int n_kv = kv_heads(a);
+  const PlanOperand qkv[3] = {{a->q, {st.q[0], st.q[1], st.q[2]}, a->N, a->S_q},
+                              {a->k, {st.k[0], st.k[1], st.k[2]}, n_kv, a->S_k},
+                              {a->v, {st.v[0], st.v[1], st.v[2]}, n_kv, a->S_k}};
+  PlanParts parts;
+  plan_parts(plan, a->mask_batch, a->S_q, a->S_k, &parts);
+  cudaError_t e = launch_mask_plan(a->attn_mask, a->mask_dtype, a->mask_batch, a->mask_tiles, a->S_q, a->S_k, qkv, a->B, a->D,
+                                   a->dtype == ACCT_BF16, parts, static_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) return fail_cuda(e, "launching the mask plan kernels");
+  return ACCT_OK;
+}
+
+int acct_fa_fwd(const acct_fa_args* a, void* stream) { return acct_fa_fwd_planned(a, nullptr, stream); }
+
+int acct_fa_fwd_planned(const acct_fa_args* a, const void* plan, void* stream) {
   Strides st;
   int rc = validate_fa(a, &st);
   if (rc) return rc;
@@ -432,8 +478,9 @@ int acct_fa_fwd(const acct_fa_args* a, void* stream) {
   p.o_stride_b = st.o[0]; p.o_stride_h = st.o[1]; p.o_stride_s = st.o[2];
   p.B = a->B; p.N = a->N; p.S_q = a->S_q; p.S_k = a->S_k; p.D = a->D;
   p.kv_group = a->N / kv_heads(a);
+  p.scale = a->scale;
   p.scale_log2 = a->scale * kLog2e;
-  p.mods = make_mods(a);
+  p.mods = make_mods(a, plan);
   p.status = dev->status;
   cudaError_t e = launch_fa_fwd(p, a->dtype == ACCT_BF16, dev->info.sm_count, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail_cuda(e, "launching the forward kernel");
@@ -453,10 +500,15 @@ size_t acct_fa_bwd_workspace_bytes(const acct_fa_args* a) {
 }
 
 int acct_fa_bwd(const acct_fa_args* a, const acct_fa_bwd_io* g, void* stream) {
-  return acct_fa_bwd_strided(a, g, nullptr, stream);
+  return acct_fa_bwd_planned(a, g, nullptr, nullptr, nullptr, stream);
 }
 
 int acct_fa_bwd_strided(const acct_fa_args* a, const acct_fa_bwd_io* g, const int64_t* d_o_stride, void* stream) {
+  return acct_fa_bwd_planned(a, g, d_o_stride, nullptr, nullptr, stream);
+}
+
+int acct_fa_bwd_planned(const acct_fa_args* a, const acct_fa_bwd_io* g, const int64_t* d_o_stride, const void* plan,
+                        void* plan_scratch, void* stream) {
   Strides st;
   int rc = validate_fa(a, &st, true);
   if (rc) return rc;
@@ -515,9 +567,16 @@ int acct_fa_bwd_strided(const acct_fa_args* a, const acct_fa_bwd_io* g, const in
     if ((rc = make_tmap_4d(&p.map_dv, t, kTile))) return rc;
   }
 
+  p.mods = make_mods(a, wide || (a->flags & ACCT_FLAG_DETERMINISTIC) ? nullptr : plan);   // (turns are counted per K/V tile)
+  if (p.mods.plan.head != nullptr) {
+    if (plan_scratch == nullptr) return fail(ACCT_ERR_NULL, "plan_scratch is NULL");
+    p.plan_stats = static_cast<unsigned int*>(plan_scratch);
+    cudaError_t me = cudaMemsetAsync(plan_scratch, 0, 2 * sizeof(unsigned int), s);
+    if (me != cudaSuccess) return fail_cuda(me, "zero-filling the plan scratch");
+  }
   // one helper pass before the main kernel: row sums, and the zero-fill of the accumulator and the turn counters
   cudaError_t e = launch_bwd_delta(a->o, g->d_o, delta, static_cast<int64_t>(rows), a->D, st.o, st_do, a->N, a->S_q, bf16,
-                                   s, dq_acc, dq_order, static_cast<int64_t>(q_tiles));
+                                   s, dq_acc, dq_order, static_cast<int64_t>(q_tiles), const_cast<unsigned int*>(p.plan_stats));
   if (e != cudaSuccess) return fail_cuda(e, "launching the row-sum kernel");
   p.lse = a->lse; p.delta = delta; p.dq_acc = dq_acc;
   p.dq_order = (a->flags & ACCT_FLAG_DETERMINISTIC) ? dq_order : nullptr;
@@ -527,7 +586,6 @@ int acct_fa_bwd_strided(const acct_fa_args* a, const acct_fa_bwd_io* g, const in
   p.B = a->B; p.N = a->N; p.S_q = a->S_q; p.S_k = a->S_k; p.D = a->D;
   p.kv_group = a->N / kv_heads(a);
   p.scale = a->scale; p.scale_log2 = a->scale * kLog2e;
-  p.mods = make_mods(a);
   p.status = dev->status;
   if (g->ev_kernel_start != nullptr) {
     e = cudaEventRecord(static_cast<cudaEvent_t>(g->ev_kernel_start), s);

@@ -81,6 +81,10 @@ struct BwdShared {
   volatile uint32_t abort_flag;
   int item[2];
   BwdItem decoded[2];            // the same two items, decoded by the producer (see next_item)
+  // The Q tiles that take part, per item (mask plan).  Read for as long as the item's steps last, so a list outlives the
+  // item's mailbox slot: item k + 1 is published once every role has read item k - 1, which the compute warps, the first
+  // to do so, do at the end of the last step of item k - 2 (the list that is overwritten).
+  uint8_t q_list[3][kPlanTiles];
   alignas(16) float lse2[2][kTile];   // L * log2(e) per query of the tile (+inf for rows past S_q); read as float4
   alignas(16) float delta[2][kTile];
 };
@@ -157,7 +161,8 @@ __device__ __noinline__ void mask_prepass(const ScoreMods& mods, uint32_t t_st, 
 // With an ordered dQ reduction the CTA of tile j waits for the CTAs of the later tiles (j' > j) that touch the same Q
 // tile, so those must never be started after it: tiles are then handed out in descending order, and every wait
 // points at an item that was taken earlier, i.e. is being worked on or finished, however many tiles a slice has.
-__device__ __forceinline__ BwdItem decode_item(const BwdParams& p, int w) {
+// With a mask plan the item's Q tiles are those of its words of the plan, listed in slot k % 3.
+__device__ __forceinline__ BwdItem decode_item(const BwdParams& p, int w, int k, bool planned, uint8_t (*q_list)[kPlanTiles]) {
   const ScoreMods& mods = p.mods;
   BwdItem it;
   const int n_kv = p.N / p.kv_group;
@@ -182,8 +187,26 @@ __device__ __forceinline__ BwdItem decode_item(const BwdParams& p, int w) {
   if (it.j * kTile >= it.kv_len) i_hi = i_lo - 1;
   it.i_lo = i_lo;
   it.n_per = max(0, i_hi - i_lo + 1);
+  if (planned) {      // (no band, no triangle, no valid lengths: all Q tiles up to here)
+    const int mb = mods.mask_batch > 1 ? it.b : 0;
+    const uint4* words = reinterpret_cast<const uint4*>(mods.plan.need_t + (static_cast<int64_t>(mb) * n_j + it.j) * kPlanWords);
+    const uint4 w0 = words[0], w1 = words[1];
+    const uint32_t bits[kPlanWords] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+    int n = 0;
+#pragma unroll
+    for (int x = 0; x < kPlanWords; ++x)
+      for (uint32_t left = bits[x]; left != 0u; left &= left - 1)
+        q_list[k % 3][n++] = static_cast<uint8_t>(x * 32 + __ffs(left) - 1);
+    it.i_lo = n > 0 ? q_list[k % 3][0] : 0;
+    it.n_per = n;
+  }
   it.n_iter = it.n_per * p.kv_group;
   return it;
+}
+
+// Q tile number m (0 .. n_per - 1) of a CTA's k-th item
+__device__ __forceinline__ int q_tile(const BwdShared& sh, const BwdItem& it, int k, bool planned, int m) {
+  return planned ? sh.q_list[k % 3][m] : it.i_lo + m;
 }
 
 // Every role learns its CTA's k-th work item here: its number and, decoded by the producer (the integer divisions of
@@ -245,6 +268,12 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
   const ScoreMods& mods = p.mods;
   const int total_items = ((p.S_k + kTile - 1) / kTile) * p.B * (p.N / p.kv_group);
 
+  // the mask plan, where the operands of this call allow it (every role comes to the same answer)
+  bool planned = false;
+  if constexpr (MASKED) if (mods.plan.head != nullptr)
+    planned = plan_holds(mods.plan.head, p.scale) && __uint_as_float(p.plan_stats[0]) < kPlanMaxNorm2 &&
+              __uint_as_float(p.plan_stats[1]) < kPlanMaxNorm2;
+
   if ((smem_u32(smem) & 1023u) != 0u) {          // the swizzled tiles need a 1024-byte aligned base
     if (tid == 0) atomicMax(p.status, DEV_BAD_SMEM_BASE);
     return;
@@ -293,9 +322,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
         // that the counter's latency -- a global atomic next to 148 SMs' reduce traffic -- is not on their path.
         int w_cur = static_cast<int>(atomicAdd(p.work_counter, 1u));
         int w_nxt = total_items;
-        auto publish = [&](int slot, int w) {
+        auto publish = [&](int k, int w) {
+          const int slot = k & 1;
           sh.item[slot] = w;
-          if (w < total_items) sh.decoded[slot] = decode_item(p, w);
+          if (w < total_items) sh.decoded[slot] = decode_item(p, w, k, planned, sh.q_list);
           mbar_arrive(&sh.item_full[slot]);      // (release: the stores above are visible to whoever sees the phase)
         };
         publish(0, w_cur);
@@ -307,7 +337,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
           auto publish_next = [&]() {
             if (k >= 1) mbar_wait(&sh.item_empty[(k + 1) & 1], ((k - 1) >> 1) & 1, abort_flag, p.status, DEV_TIMEOUT_SYNC);
             w_nxt = *abort_flag == 0u ? static_cast<int>(atomicAdd(p.work_counter, 1u)) : total_items;
-            publish((k + 1) & 1, w_nxt);
+            publish(k + 1, w_nxt);
             published = true;
           };
           if (it.n_iter > 0 && *abort_flag == 0u) {
@@ -317,7 +347,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
             for (int nb = 0; nb < NB; ++nb) tma_load_4d(sK + nb * 16384, &p.map_k, &sh.kv_full, nb * 64, it.j * kTile, it.h_kv, it.b);
             for (int nb = 0; nb < NB; ++nb) tma_load_4d(sV + nb * 16384, &p.map_v, &sh.kv_full, nb * 64, it.j * kTile, it.h_kv, it.b);
             for (int n = 0; n < it.n_iter; ++n) {
-              const int i = it.i_lo + n % it.n_per, h = it.h_kv * p.kv_group + n / it.n_per;
+              const int i = q_tile(sh, it, k, planned, n % it.n_per), h = it.h_kv * p.kv_group + n / it.n_per;
               const int gn = g0 + n;
               const int st = gn % kStages;
               // the Q stage is free once the dK product of two tiles ago has finished
@@ -452,7 +482,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
     if (w >= total_items) break;
     const int b = it.b, j = it.j, kv_len = it.kv_len;
     auto head_of = [&](int n) { return it.h_kv * p.kv_group + n / max(it.n_per, 1); };
-    auto tile_of = [&](int n) { return it.i_lo + n % max(it.n_per, 1); };
+    auto tile_of = [&](int n) { return q_tile(sh, it, k, planned, n % max(it.n_per, 1)); };
     for (int n = 0; n < it.n_iter; ++n) {
       const int q_base = tile_of(n) * kTile;
       const int h = head_of(n);
@@ -599,10 +629,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
     const BwdItem it = it_next;
     int next_no = total_items;
     bool next_known = false;
-    const int b = it.b, j = it.j, kv_len = it.kv_len, i_lo = it.i_lo, n_per = it.n_per, n_iter = it.n_iter;
+    const int b = it.b, j = it.j, kv_len = it.kv_len, n_per = it.n_per, n_iter = it.n_iter;
     const int bh_kv = it.bh_kv;
     auto head_of = [&](int n) { return it.h_kv * p.kv_group + n / max(n_per, 1); };
-    auto tile_of = [&](int n) { return i_lo + n % max(n_per, 1); };
+    auto tile_of = [&](int n) { return q_tile(sh, it, k, planned, n % max(n_per, 1)); };
     const int kv_idx = j * kTile + r;
     const bool kv_ok = kv_idx < kv_len;
     // alibi term of this key row in log2 units for query head h; -inf removes a key row that does not exist
@@ -616,7 +646,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
       return v;
     };
     float bias = kNegInf;
-    float bias_first = kNegInf;          // bias_of(head_of(0)), from the value requested ahead
+    float bias_first = kNegInf;          // bias_of() of the first head, from the value requested ahead
     if (kv_ok) {
       bias_first = 0.f;
       if (mods.alibi != nullptr)
@@ -631,7 +661,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
     float nxt_lse = 0.f, nxt_dlt = 0.f;
     bool nxt_ok = false;
     if (hf == 0 && n_iter > 0) {
-      const int q_row = i_lo * kTile + r;
+      const int q_row = it.i_lo * kTile + r;
       const bool q_ok = q_row < p.S_q;
       // (buffer g0 & 1 was last read for the step before last, whose dS part every thread finished before the
       // products this thread has since waited for could be issued)
@@ -644,9 +674,9 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
     const uint8_t* tile_class = nullptr;
     const int tiles_k = (p.S_k + kTile - 1) / kTile;
     if constexpr (MASKED) if (mods.mask_kind == 1 && mods.mask_tiles != nullptr)
-      tile_class = mods.mask_tiles + static_cast<int64_t>(mods.mask_batch > 1 ? b : 0) * ((p.S_q + kTile - 1) / kTile) * tiles_k + j;
+      tile_class = (planned ? mods.plan.cls : mods.mask_tiles) + static_cast<int64_t>(mods.mask_batch > 1 ? b : 0) * ((p.S_q + kTile - 1) / kTile) * tiles_k + j;
     int mask_class = 1, mask_class_next = 1;
-    if (tile_class != nullptr && n_iter > 0) mask_class_next = tile_class[static_cast<int64_t>(tile_of(0)) * tiles_k];
+    if (tile_class != nullptr && n_iter > 0) mask_class_next = tile_class[static_cast<int64_t>(it.i_lo) * tiles_k];
 
     for (int n = 0; n < n_iter; ++n) {
       const int i = tile_of(n);
@@ -656,6 +686,11 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
       if (n % max(n_per, 1) == 0) bias = n == 0 ? bias_first : bias_of(head_of(n));   // first tile of a query head
       mask_class = mask_class_next;
       if (tile_class != nullptr && n + 1 < n_iter) mask_class_next = tile_class[static_cast<int64_t>(tile_of(n + 1)) * tiles_k];
+      // class 3 (mask plan): a bit per position, set = masked; this key's bits for the half's 64 queries
+      uint2 key_bits = make_uint2(0u, 0u);
+      if constexpr (MASKED) if (mask_class == 3)
+        key_bits = *reinterpret_cast<const uint2*>(
+            mods.plan.bits + (tile_class + static_cast<int64_t>(i) * tiles_k - mods.plan.cls) * kPlanBitWords + kTile * 4 + r * 4 + hf * 2);
       // ---- P part: needs S^T only
       mbar_wait(&sh.st_full, gn & 1, abort_flag, p.status, DEV_TIMEOUT_MMA);
       tc_fence_after_sync();
@@ -681,7 +716,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
       // A mask tile that is all 0 is not read; one that is all 1 adds one constant to every score of the tile,
       // which joins the key row's bias; any other tile is read.
       const bool mask_const = MASKED && mods.mask_kind == 1 && mask_class == 2;
-      const bool use_mask = MASKED && ((mods.mask_kind == 1 && mask_class != 0 && !mask_const) || (mods.mask_kind == 2 && i == j));
+      const bool use_mask = MASKED && ((mods.mask_kind == 1 && mask_class == 1) || (mods.mask_kind == 2 && i == j));
       const float tile_bias = mask_const ? bias - 10000.0f * kLog2e : bias;
       const bool diag = mods.causal && (q_base < j * kTile + kTile - 1);
       // TriangleAttention row groups: the rows of this Q tile see keys below the end of their group; the smallest
@@ -713,6 +748,11 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
             u8_keep_load(mods.drop, static_cast<int64_t>(bh) * p.S_q, q_base + c * 32, p.S_q - 1, p.S_k, kv_idx - lane, lane, raw8);
           if (diag) p_fast<true>(s[cc], lse2 + c * 32, p.scale_log2, tile_bias, kv_idx, q_base + c * 32, pr[cc]);
           else p_fast<false>(s[cc], lse2 + c * 32, p.scale_log2, tile_bias, kv_idx, q_base + c * 32, pr[cc]);
+          if constexpr (MASKED) if (mask_class == 3) {
+            const uint32_t word = cc == 0 ? key_bits.x : key_bits.y;
+#pragma unroll
+            for (int e = 0; e < 32; ++e) pr[cc][e] = ((word >> e) & 1u) ? 0.f : pr[cc][e];
+          }
           uint32_t pk[16];
           if constexpr (DROP == 1 || DROP == 3) {
             if constexpr (DROP == 1) keep_bits[cc] = philox_keep_column(mods, bh, q_base + c * 32, p.S_q - 1, kv_idx, lane);
@@ -930,8 +970,10 @@ struct RowStrides {
 // launch: flash_attention_bwd.py:55-57).
 template <bool BF16, int LPR>
 __global__ void bwd_delta_kernel(const void* o, const void* d_o, float* delta, int64_t rows, int D, RowStrides so,
-                                 RowStrides sdo, int N, int S_q, float* zero_acc, unsigned int* counters, int64_t n_counters) {
+                                 RowStrides sdo, int N, int S_q, float* zero_acc, unsigned int* counters, int64_t n_counters,
+                                 unsigned int* plan_stats) {
   constexpr int RPW = 32 / LPR;
+  unsigned int most_do2 = 0u, most_delta = 0u;     // (as bits: a NaN is larger than everything)
   const int lane = threadIdx.x & 31;
   const int sub = lane % LPR, rsub = lane / LPR;
   const int64_t warp_global = static_cast<int64_t>(blockIdx.x) * (blockDim.x / 32) + (threadIdx.x >> 5);
@@ -941,7 +983,7 @@ __global__ void bwd_delta_kernel(const void* o, const void* d_o, float* delta, i
     counters[c] = 0u;
   for (int64_t row0 = warp_global * RPW; row0 < rows; row0 += warps_total * RPW) {
     const int64_t row = row0 + rsub;
-    float acc = 0.f;
+    float acc = 0.f, do2 = 0.f;
     if (row < rows && sub * 8 < D) {
       if (zero_acc != nullptr) {
         float4* z = reinterpret_cast<float4*>(zero_acc + row * D + sub * 8);
@@ -952,24 +994,28 @@ __global__ void bwd_delta_kernel(const void* o, const void* d_o, float* delta, i
       const int64_t bb = bh / N, hh = bh % N, rr = row % S_q;
       const uint4 a = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(o) + bb * so.b + hh * so.h + rr * so.s + sub * 8);
       const uint4 g = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(d_o) + bb * sdo.b + hh * sdo.h + rr * sdo.s + sub * 8);
-      const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, gw[4] = {g.x, g.y, g.z, g.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        float2 x, y;
-        if constexpr (BF16) {
-          x = make_float2(__uint_as_float(aw[e] << 16), __uint_as_float(aw[e] & 0xffff0000u));
-          y = make_float2(__uint_as_float(gw[e] << 16), __uint_as_float(gw[e] & 0xffff0000u));
-        } else {
-          x = __half22float2(*reinterpret_cast<const __half2*>(&aw[e]));
-          y = __half22float2(*reinterpret_cast<const __half2*>(&gw[e]));
-        }
-        acc = fmaf(x.x, y.x, acc);
-        acc = fmaf(x.y, y.y, acc);
-      }
+      acc = dot8<BF16>(a, g, 0.f);
+      if (plan_stats != nullptr) do2 = dot8<BF16>(g, g, 0.f);
     }
 #pragma unroll
     for (int off2 = LPR / 2; off2 > 0; off2 >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off2);
     if (sub == 0 && row < rows) delta[row] = acc;
+    if (plan_stats != nullptr) {
+#pragma unroll
+      for (int off2 = LPR / 2; off2 > 0; off2 >>= 1) do2 += __shfl_xor_sync(0xffffffffu, do2, off2);
+      most_do2 = max(most_do2, __float_as_uint(do2) & 0x7fffffffu);
+      most_delta = max(most_delta, __float_as_uint(acc) & 0x7fffffffu);
+    }
+  }
+  if (plan_stats != nullptr) {
+    __shared__ unsigned int block_max[2];
+    if (threadIdx.x < 2) block_max[threadIdx.x] = 0u;
+    __syncthreads();
+    most_do2 = __reduce_max_sync(0xffffffffu, most_do2);
+    most_delta = __reduce_max_sync(0xffffffffu, most_delta);
+    if (lane == 0) { atomicMax(&block_max[0], most_do2); atomicMax(&block_max[1], most_delta); }
+    __syncthreads();
+    if (threadIdx.x < 2) atomicMax(&plan_stats[threadIdx.x], block_max[threadIdx.x]);
   }
 }
 
@@ -994,6 +1040,7 @@ cudaError_t launch_fa_bwd(const BwdParams& p, bool bf16, int sm_count, cudaStrea
   // persistent CTAs, one per SM (tensor memory and shared memory admit no more), fewer if there is less work
   const long long items = static_cast<long long>((p.S_k + kTile - 1) / kTile) * p.B * (p.N / p.kv_group);
   dim3 grid(static_cast<unsigned>(items < sm_count ? items : sm_count));
+  static_assert(5 * 32768 + 2 * 32768 + sizeof(BwdShared) <= 232448, "shared memory of a thread block at head_dim 128");
   // (row groups of a multiple of 128 rows never cut a tile: the tile ranges alone take care of them)
   const bool masked = p.mods.mask_kind != 0 || (p.mods.tri_block > 0 && p.mods.tri_block % kTile != 0);
   const bool drop_u8_bits = p.mods.drop != nullptr && p.mods.drop_dtype == 2 /*U8*/ && p.S_k % 4 == 0 &&
@@ -1016,7 +1063,7 @@ cudaError_t launch_fa_bwd(const BwdParams& p, bool bf16, int sm_count, cudaStrea
 
 cudaError_t launch_bwd_delta(const void* o, const void* d_o, float* delta, int64_t rows, int D, const int64_t (&o_stride)[3],
                              const int64_t (&do_stride)[3], int N, int S_q, bool bf16, cudaStream_t stream,
-                             float* zero_acc, unsigned int* counters, int64_t n_counters) {
+                             float* zero_acc, unsigned int* counters, int64_t n_counters, unsigned int* plan_stats) {
   const int lpr = D <= 64 ? 8 : (D <= 128 ? 16 : 32);       // lanes per row
   const int warps = 8;
   const int64_t rows_per_block = static_cast<int64_t>(warps) * (32 / lpr);
@@ -1028,7 +1075,8 @@ cudaError_t launch_bwd_delta(const void* o, const void* d_o, float* delta, int64
   auto kern = lpr == 8 ? (bf16 ? bwd_delta_kernel<true, 8> : bwd_delta_kernel<false, 8>)
               : lpr == 16 ? (bf16 ? bwd_delta_kernel<true, 16> : bwd_delta_kernel<false, 16>)
                           : (bf16 ? bwd_delta_kernel<true, 32> : bwd_delta_kernel<false, 32>);
-  kern<<<static_cast<unsigned>(blocks), warps * 32, 0, stream>>>(o, d_o, delta, rows, D, so, sdo, N, S_q, zero_acc, counters, n_counters);
+  kern<<<static_cast<unsigned>(blocks), warps * 32, 0, stream>>>(o, d_o, delta, rows, D, so, sdo, N, S_q, zero_acc, counters, n_counters,
+                                                           plan_stats);
   return cudaGetLastError();
 }
 

@@ -69,6 +69,26 @@ __device__ __forceinline__ float load_mask_value(const void* base, int dtype, in
   return __half2float(reinterpret_cast<const __half*>(base)[idx]);
 }
 
+// acc + the dot product of eight 16-bit pairs
+template <bool BF16>
+__device__ __forceinline__ float dot8(const uint4& a, const uint4& g, float acc) {
+  const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, gw[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    float2 x, y;
+    if constexpr (BF16) {
+      x = make_float2(__uint_as_float(aw[e] << 16), __uint_as_float(aw[e] & 0xffff0000u));
+      y = make_float2(__uint_as_float(gw[e] << 16), __uint_as_float(gw[e] & 0xffff0000u));
+    } else {
+      x = __half22float2(*reinterpret_cast<const __half2*>(&aw[e]));
+      y = __half22float2(*reinterpret_cast<const __half2*>(&gw[e]));
+    }
+    acc = fmaf(x.x, y.x, acc);
+    acc = fmaf(x.y, y.y, acc);
+  }
+  return acc;
+}
+
 // 32 consecutive values (elements idx0 .. idx0+31 of a u8 / f16 / bf16 array) as floats, times `mul`.
 // `vec` (uniform): idx0 is a multiple of 16 elements and all 32 elements exist, so 128-bit loads are used;
 // otherwise element loads, with elements at or past `n_valid` read as 0.

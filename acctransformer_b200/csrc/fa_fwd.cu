@@ -69,6 +69,7 @@ struct FwdShared {
   uint64_t s_full[2], p_half[2], p_ready[2], o_done[2];
   uint32_t tmem_base;
   volatile uint32_t abort_flag;
+  uint32_t need[2][kPlanWords];           // K/V tiles of each Q tile that the mask plan leaves (all ones without a plan)
   alignas(16) float alibi[2][2][kTile];   // [softmax group][tile parity]: alibi row of the K/V tile, log2 units
 };
 
@@ -118,14 +119,53 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
   int kv_len = p.S_k;
   if (mods.seq_lens != nullptr) kv_len = min(p.S_k, max(0, mods.seq_lens[b]));
 
-  const TileRange r0 = kv_tile_range(NQ * pair, p.S_q, kv_len, mods);
+  TileRange r0 = kv_tile_range(NQ * pair, p.S_q, kv_len, mods);
   TileRange r1 = kv_tile_range(NQ * pair + 1, p.S_q, kv_len, mods);
   if (NQ == 1) { r1.lo = 0; r1.hi = -1; }
+  // Tiles that the mask plan leaves out: every role walks the same bits.  The ranges shrink to the first and last tile
+  // needed, and the others are skipped one by one (next_tile, needed).
+  const bool planned = (MODS & 1) != 0 && mods.plan.head != nullptr && plan_holds(mods.plan.head, p.scale);
+  if constexpr ((MODS & 1) != 0) if (planned) {
+    const int tiles_q = (p.S_q + kTile - 1) / kTile;
+    const uint32_t* rows = mods.plan.need + static_cast<int64_t>(mods.mask_batch > 1 ? b : 0) * tiles_q * kPlanWords;
+    auto shrink = [&](int i, TileRange& r, uint32_t* out) {
+      if (r.lo > r.hi) return;                   // (an absent second Q tile)
+      int lo = kPlanTiles, hi = -1;
+#pragma unroll
+      for (int x = 0; x < kPlanWords; ++x) {
+        const uint32_t bits = rows[i * kPlanWords + x];
+        if (tid == 0) out[x] = bits;
+        if (bits != 0u) {
+          if (hi < 0) lo = x * 32 + __ffs(bits) - 1;
+          hi = x * 32 + 31 - __clz(bits);
+        }
+      }
+      r.lo = lo; r.hi = hi;
+    };
+    if (tid < 2 * kPlanWords) sh.need[tid / kPlanWords][tid % kPlanWords] = 0u;
+    __syncwarp();                                // (thread 0 of the same warp fills in what follows)
+    shrink(NQ * pair, r0, sh.need[0]);
+    shrink(NQ * pair + 1, r1, sh.need[1]);
+  }
+  auto needed = [&](int qt, const TileRange& r, int j) {
+    return j >= r.lo && j <= r.hi && (!planned || ((sh.need[qt][j >> 5] >> (j & 31)) & 1u) != 0u);
+  };
+  // the tile after j that Q tile qt needs (r.hi is needed, so the walk ends), and the same for either Q tile
+  auto next_tile = [&](int qt, const TileRange& r, int j) {
+    ++j;
+    if constexpr ((MODS & 1) != 0) if (planned) while (j < r.hi && !needed(qt, r, j)) ++j;
+    return j;
+  };
   const bool any0 = r0.lo <= r0.hi, any1 = r1.lo <= r1.hi;
   int cta_lo = 0, cta_hi = -1;
   if (any0 && any1) { cta_lo = min(r0.lo, r1.lo); cta_hi = max(r0.hi, r1.hi); }
   else if (any0) { cta_lo = r0.lo; cta_hi = r0.hi; }
   else if (any1) { cta_lo = r1.lo; cta_hi = r1.hi; }
+  auto next_any = [&](int j) {
+    ++j;
+    if constexpr ((MODS & 1) != 0) if (planned) while (j < cta_hi && !needed(0, r0, j) && !needed(1, r1, j)) ++j;
+    return j;
+  };
 
   if (tid == 0) {
     mbar_init(&sh.q_full, 1);
@@ -158,7 +198,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
           tma_load_4d(sQ + qt * kTileBytes + nb * 16384, &p.map_q, &sh.q_full, nb * 64,
                       (NQ * pair + qt) * kTile, h, b);
       int it = 0;
-      for (int j = cta_lo; j <= cta_hi; ++j, ++it) {
+      for (int j = cta_lo; j <= cta_hi; j = next_any(j), ++it) {
         const int st = it % kSt;
         const uint32_t reuse_parity = ((it / kSt) - 1) & 1;
         if (it >= kSt) mbar_wait(&sh.k_empty[st], reuse_parity, abort_flag, p.status, DEV_TIMEOUT_SYNC);
@@ -210,19 +250,21 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
       // prologue: scores of the first K/V tile
       mbar_wait(&sh.k_full[0], 0, abort_flag, p.status, DEV_TIMEOUT_TMA);
       for (int qt = 0; qt < 2; ++qt)
-        if (cta_lo >= rng[qt].lo && cta_lo <= rng[qt].hi) issue_s(qt, 0);
+        if (needed(qt, rng[qt], cta_lo)) issue_s(qt, 0);
       if (elect_one()) umma_commit(&sh.k_empty[0]);
       mbar_wait(&sh.v_full[0], 0, abort_flag, p.status, DEV_TIMEOUT_TMA);
       int it = 0;
-      for (int j = cta_lo; j <= cta_hi; ++j, ++it) {
+      int jn;
+      for (int j = cta_lo; j <= cta_hi; j = jn, ++it) {
+        jn = next_any(j);
         const int st = it % kSt;
         const int stn = (it + 1) % kSt;
         const uint32_t full_parity_n = ((it + 1) / kSt) & 1;
-        const bool more = j + 1 <= cta_hi;
-        bool k_seen = false;   // K tile j+1 seen full
+        const bool more = jn <= cta_hi;
+        bool k_seen = false;   // the next K tile seen full
         for (int qt = 0; qt < 2; ++qt) {
-          const bool pv = j >= rng[qt].lo && j <= rng[qt].hi;
-          const bool sn = more && j + 1 >= rng[qt].lo && j + 1 <= rng[qt].hi;
+          const bool pv = needed(qt, rng[qt], j);
+          const bool sn = more && needed(qt, rng[qt], jn);
           const uint32_t t_s = tmem + kColS + qt * 128, t_o = tmem + kColO + qt * DPAD;
           const uint32_t v0 = vt_lo + st * kTileUnits;
           if (pv) {
@@ -297,7 +339,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
     // before the wait for S, so that its latency is not on the path.
     const uint8_t* tile_class = nullptr;
     if constexpr ((MODS & 1) != 0) if (mods.mask_kind == 1 && mods.mask_tiles != nullptr)
-      tile_class = mods.mask_tiles + (static_cast<int64_t>(mods.mask_batch > 1 ? b : 0) * ((p.S_q + kTile - 1) / kTile) +
+      tile_class = (planned ? mods.plan.cls : mods.mask_tiles) + (static_cast<int64_t>(mods.mask_batch > 1 ? b : 0) * ((p.S_q + kTile - 1) / kTile) +
                                       min(q_tile, (p.S_q - 1) / kTile)) * ((p.S_k + kTile - 1) / kTile);
     int mask_class = 1, mask_class_next = 1;
     if (tile_class != nullptr && rng.lo <= rng.hi) mask_class_next = tile_class[rng.lo];
@@ -310,20 +352,26 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
 
     float m_run = kNegInf, l_run = 0.f;
     int n = 0;
-    for (int j = rng.lo; j <= rng.hi; ++j, ++n) {
+    int j_next;
+    for (int j = rng.lo; j <= rng.hi; j = j_next, ++n) {
+      j_next = next_tile(qt, rng, j);
       mask_class = mask_class_next;
-      if (tile_class != nullptr && j < rng.hi) mask_class_next = tile_class[j + 1];
+      if (tile_class != nullptr && j < rng.hi) mask_class_next = tile_class[j_next];
       if constexpr ((MODS & 2) != 0) if (mods.alibi != nullptr) {
         al_raw = al_raw_next;
-        if (j < rng.hi) al_raw_next = alibi_raw[min((j + 1) * kTile + row_in_tile, p.S_k - 1)];
+        if (j < rng.hi) al_raw_next = alibi_raw[min(j_next * kTile + row_in_tile, p.S_k - 1)];
       }
+      // class 3 (mask plan): a bit per position, set = masked; this row's 128, requested ahead of the scores
+      uint4 row_bits = make_uint4(0u, 0u, 0u, 0u);
+      if constexpr ((MODS & 1) != 0) if (mask_class == 3)
+        row_bits = reinterpret_cast<const uint4*>(mods.plan.bits + (tile_class + j - mods.plan.cls) * kPlanBitWords)[row_in_tile];
       mbar_wait(&sh.s_full[qt], n & 1, abort_flag, p.status, DEV_TIMEOUT_MMA);
       tc_fence_after_sync();
       const int col_base = j * kTile;
       // a mask tile that is all 1 adds one constant to every score of the tile: without alibi it is folded into
       // the exponent's offset below and the tile takes the plain path
       const bool mask_const = (MODS & 1) != 0 && mods.mask_kind == 1 && mask_class == 2 && !has_alibi;
-      const bool use_mask = (MODS & 1) != 0 && ((mods.mask_kind == 1 && mask_class != 0 && !mask_const) ||
+      const bool use_mask = (MODS & 1) != 0 && ((mods.mask_kind == 1 && (mask_class == 1 || (mask_class == 2 && !mask_const))) ||
                                                 (mods.mask_kind == 2 && j == q_tile));
       const float tile_add = mask_const ? -10000.0f * kLog2e : 0.f;
       const bool generic = GENERIC && (use_mask || has_alibi);
@@ -441,6 +489,15 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
 #pragma unroll
           for (int i = 0; i < 32; ++i)
             s[c][i] = (col_base + c * 32 + i >= bound) ? __float_as_uint(kNegInf) : s[c][i];
+      }
+
+      if constexpr ((MODS & 1) != 0) if (mask_class == 3) {
+        const uint32_t words[4] = {row_bits.x, row_bits.y, row_bits.z, row_bits.w};
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            s[c][i] = ((words[c] >> i) & 1u) ? __float_as_uint(kNegInf) : s[c][i];
       }
 
       // One 32-column chunk: P = exp2(x * mult - m) packed to 16 bits, row sum (before dropout) into `l4`.

@@ -33,8 +33,10 @@ using torch::autograd::SavedVariable;
 using torch::autograd::variable_list;
 
 struct Library {
-  decltype(&acct_fa_fwd) fa_fwd;
-  decltype(&acct_fa_bwd_strided) fa_bwd;
+  decltype(&acct_fa_fwd_planned) fa_fwd;
+  decltype(&acct_fa_bwd_planned) fa_bwd;
+  decltype(&acct_mask_plan_bytes) mask_plan_bytes;
+  decltype(&acct_mask_plan) mask_plan;
   decltype(&acct_fa_bwd_workspace_bytes) fa_bwd_workspace_bytes;
   decltype(&acct_infer_prefill) infer_prefill;
   decltype(&acct_infer_decode) infer_decode;
@@ -187,7 +189,7 @@ void check_fa_inputs(const Tensor& q, const Tensor& k, const Tensor& v, Tensor& 
 // kernels can (head_dim contiguous, strides and address multiples of 16 bytes): behind a transpose back to
 // [B, S, N*D] it is a strided view, and copying it would be one more pass over memory.
 struct FaBackward : public torch::autograd::Node {
-  SavedVariable q_, k_, v_, o_, lse_, mask_, drop_, alibi_, tiles_;
+  SavedVariable q_, k_, v_, o_, lse_, mask_, drop_, alibi_, tiles_, plan_;
   FaConfig cfg;
   bool released = false;
 
@@ -198,7 +200,8 @@ struct FaBackward : public torch::autograd::Node {
     Tensor d_o = grads[0];
     if (!d_o.defined()) return out;
     const Tensor q = q_.unpack(), k = k_.unpack(), v = v_.unpack(), o = o_.unpack(shared_from_this()), lse = lse_.unpack();
-    const Tensor mask = mask_.unpack(), drop = drop_.unpack(), alibi = alibi_.unpack(), tiles = tiles_.unpack();
+    const Tensor mask = mask_.unpack(), drop = drop_.unpack(), alibi = alibi_.unpack(), tiles = tiles_.unpack(),
+                 plan = plan_.unpack();
     at::AutoDispatchBelowADInplaceOrView below;
     c10::cuda::OptionalCUDAGuard guard(q.device());
     int64_t ds[3] = {d_o.stride(0), d_o.stride(1), d_o.stride(2)};
@@ -214,13 +217,15 @@ struct FaBackward : public torch::autograd::Node {
     const auto dt = q.scalar_type();
     Tensor dq = empty_like_shape(q.sizes(), dt, q), dk = empty_like_shape(k.sizes(), dt, q), dv = empty_like_shape(v.sizes(), dt, q);
     const size_t nbytes = g_lib.fa_bwd_workspace_bytes(&a);
-    Tensor ws = empty_like_shape({static_cast<int64_t>(nbytes)}, at::kByte, q);
+    const int64_t own = (nbytes + 15) / 16 * 16;      // behind it 16 bytes for the statistics that go with a mask plan
+    Tensor ws = empty_like_shape({own + 16}, at::kByte, q);
     acct_fa_bwd_io g;
     memset(&g, 0, sizeof(g));
     g.d_o = d_o.const_data_ptr();
     g.dq = dq.data_ptr(); g.dk = dk.data_ptr(); g.dv = dv.data_ptr();
     g.workspace = ws.data_ptr(); g.workspace_bytes = nbytes;
-    check(g_lib.fa_bwd(&a, &g, ds, stream_of(q)));
+    check(g_lib.fa_bwd(&a, &g, ds, plan.defined() ? plan.const_data_ptr() : nullptr, static_cast<uint8_t*>(ws.data_ptr()) + own,
+                       stream_of(q)));
     out[0] = std::move(dq); out[1] = std::move(dk); out[2] = std::move(dv);
     return out;
   }
@@ -228,7 +233,7 @@ struct FaBackward : public torch::autograd::Node {
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
     released = true;
-    for (SavedVariable* s : {&q_, &k_, &v_, &o_, &lse_, &mask_, &drop_, &alibi_, &tiles_}) s->reset_data();
+    for (SavedVariable* s : {&q_, &k_, &v_, &o_, &lse_, &mask_, &drop_, &alibi_, &tiles_, &plan_}) s->reset_data();
   }
 
   std::string name() const override { return "FlashAttentionBackward"; }
@@ -274,8 +279,10 @@ PyObject* py_init(PyObject*, PyObject* path) {
     TORCH_CHECK(f != nullptr, p, " has no ", name);
     return f;
   };
-  g_lib.fa_fwd = reinterpret_cast<decltype(g_lib.fa_fwd)>(sym("acct_fa_fwd"));
-  g_lib.fa_bwd = reinterpret_cast<decltype(g_lib.fa_bwd)>(sym("acct_fa_bwd_strided"));
+  g_lib.fa_fwd = reinterpret_cast<decltype(g_lib.fa_fwd)>(sym("acct_fa_fwd_planned"));
+  g_lib.fa_bwd = reinterpret_cast<decltype(g_lib.fa_bwd)>(sym("acct_fa_bwd_planned"));
+  g_lib.mask_plan_bytes = reinterpret_cast<decltype(g_lib.mask_plan_bytes)>(sym("acct_mask_plan_bytes"));
+  g_lib.mask_plan = reinterpret_cast<decltype(g_lib.mask_plan)>(sym("acct_mask_plan"));
   g_lib.fa_bwd_workspace_bytes = reinterpret_cast<decltype(g_lib.fa_bwd_workspace_bytes)>(sym("acct_fa_bwd_workspace_bytes"));
   g_lib.infer_prefill = reinterpret_cast<decltype(g_lib.infer_prefill)>(sym("acct_infer_prefill"));
   g_lib.infer_decode = reinterpret_cast<decltype(g_lib.infer_decode)>(sym("acct_infer_decode"));
@@ -306,7 +313,7 @@ PyObject* py_fa_apply(PyObject*, PyObject* const* args, Py_ssize_t n) {
     c.offset = PyLong_AsUnsignedLongLongMask(args[16]);
     if (PyErr_Occurred()) throw python_error();
   }
-  Tensor o, lse;
+  Tensor o, lse, plan;
   // as a Python autograd Function without a `jvp` does; a tangent would be dropped silently otherwise
   for (const Tensor* t : {&q, &k, &v, &std::as_const(mask), &std::as_const(drop), &std::as_const(alibi)})
     TORCH_CHECK_NOT_IMPLEMENTED(!t->defined() || !t->_fw_grad(/*level=*/0).defined(),
@@ -322,7 +329,12 @@ PyObject* py_fa_apply(PyObject*, PyObject* const* args, Py_ssize_t n) {
       lse = empty_like_shape(q.sizes().slice(0, 3), at::kFloat, q);
       acct_fa_args a;
       fill_args(a, q, k, v, o, lse, mask, drop, alibi, tiles, c);
-      check(g_lib.fa_fwd(&a, stream_of(q)));
+      const size_t plan_bytes = g_lib.mask_plan_bytes(&a);
+      if (plan_bytes > 0) {
+        plan = empty_like_shape({static_cast<int64_t>(plan_bytes)}, at::kByte, q);
+        check(g_lib.mask_plan(&a, plan.data_ptr(), stream_of(q)));
+      }
+      check(g_lib.fa_fwd(&a, plan.defined() ? plan.const_data_ptr() : nullptr, stream_of(q)));
     }
     // (an optional input may require a gradient too: it gets none, but the output is part of the graph)
     if (torch::autograd::compute_requires_grad(inputs)) {
@@ -336,6 +348,7 @@ PyObject* py_fa_apply(PyObject*, PyObject* const* args, Py_ssize_t n) {
       node->drop_ = SavedVariable(drop, false);
       node->alibi_ = SavedVariable(alibi, false);
       node->tiles_ = SavedVariable(tiles, false);
+      node->plan_ = SavedVariable(plan, false);
       torch::autograd::set_history(o, node);
       node->o_ = SavedVariable(o, true);
       node->lse_ = SavedVariable(lse, false);

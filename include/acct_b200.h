@@ -222,6 +222,19 @@ ACCT_API int acct_fa_bwd(const acct_fa_args* a, const acct_fa_bwd_io* g, void* s
  * projection reads, the gradient arrives as such a view and need not be copied first. */
 ACCT_API int acct_fa_bwd_strided(const acct_fa_args* a, const acct_fa_bwd_io* g, const int64_t* d_o_stride, void* stream);
 
+/* Which 128x128 tiles of a mask tensor a forward and backward need not compute at all.  In a row that has an unmasked key,
+ * the probabilities of a tile that is all 1 are exactly 0, so leaving the tile out changes no result as long as the scores
+ * stay within a few thousand and every operand is finite; both are checked on the GPU, and where they fail every tile is
+ * computed.  acct_mask_plan_bytes: size of the plan, 0 where none applies (it takes an ACCT_MASK_FULL mask with mask_tiles
+ * and no causal, alibi, band, seq_lens, tri_block or dropout_mask, at most 32 768 positions, and enough work to pay for the
+ * plan's passes).  acct_mask_plan enqueues its passes over the mask's classes and q, k, v of `a` (device memory, 16-byte
+ * aligned); the plan is good for calls with the same `a`.  plan_scratch: 8 bytes of device memory of the call's own. */
+ACCT_API size_t acct_mask_plan_bytes(const acct_fa_args* a);
+ACCT_API int acct_mask_plan(const acct_fa_args* a, void* plan, void* stream);
+ACCT_API int acct_fa_fwd_planned(const acct_fa_args* a, const void* plan, void* stream);
+ACCT_API int acct_fa_bwd_planned(const acct_fa_args* a, const acct_fa_bwd_io* g, const int64_t* d_o_stride, const void* plan,
+                                 void* plan_scratch, void* stream);
+
 /* Inference op  y = softmax(scale * q k^T) v.
  *
  * Replaces  FlashAttentionTik(q, k, v) -> y
