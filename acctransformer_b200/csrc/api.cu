@@ -532,6 +532,8 @@ int acct_fa_bwd_planned(const acct_fa_args* a, const acct_fa_bwd_io* g, const in
   const bool bf16 = a->dtype == ACCT_BF16;
   const size_t rows = static_cast<size_t>(a->B) * a->N * a->S_q;
   float* delta = static_cast<float*>(g->workspace);
+  // up to 160 columns one CTA holds dK and dV whole; with an ordered dQ reduction the split-width kernel does it
+  const bool mid = a->D > 128 && a->D <= kMidHeadDim && !(a->flags & ACCT_FLAG_DETERMINISTIC);
   const bool wide = a->D > 128;      // the split-width kernel: 64-row Q / dO boxes, 64-row dQ box, 2 counters per tile
   const size_t q_tiles = static_cast<size_t>(a->B) * a->N * ((a->S_q + kTile - 1) / kTile) * (wide ? 2 : 1) + 1;   // + work counter
   const size_t order_bytes = ((q_tiles * 4 + 255) / 256) * 256;
@@ -553,8 +555,8 @@ int acct_fa_bwd_planned(const acct_fa_args* a, const acct_fa_bwd_io* g, const in
   t.dtype = ACCT_F32; t.ptr = dq_acc;
   t.strides[0] = a->D; t.strides[1] = static_cast<int64_t>(a->S_q) * a->D;
   t.strides[2] = static_cast<int64_t>(a->N) * a->S_q * a->D;
-  if ((rc = make_tmap_4d(&p.map_dq, t, wide ? 64 : kTile))) return rc;
-  if (!wide && !(a->flags & ACCT_FLAG_GRAD_F32)) {
+  if ((rc = make_tmap_4d(&p.map_dq, t, mid ? 32 : wide ? 64 : kTile))) return rc;
+  if ((!wide || mid) && !(a->flags & ACCT_FLAG_GRAD_F32)) {
     // 16-bit dk, dv, packed [B,N_kv,S_k,D]: the kernel writes a tile through shared memory and one TMA store
     const int n_kv = kv_heads(a);
     t.dtype = a->dtype;
@@ -591,7 +593,7 @@ int acct_fa_bwd_planned(const acct_fa_args* a, const acct_fa_bwd_io* g, const in
     e = cudaEventRecord(static_cast<cudaEvent_t>(g->ev_kernel_start), s);
     if (e != cudaSuccess) return fail_cuda(e, "recording the kernel-start event");
   }
-  e = wide ? launch_fa_bwd_wide(p, bf16, s) : launch_fa_bwd(p, bf16, dev->info.sm_count, s);
+  e = mid ? launch_fa_bwd_mid(p, bf16, s) : wide ? launch_fa_bwd_wide(p, bf16, s) : launch_fa_bwd(p, bf16, dev->info.sm_count, s);
   if (e != cudaSuccess) return fail_cuda(e, "launching the backward kernel");
   if (g->ev_kernel_stop != nullptr) {
     e = cudaEventRecord(static_cast<cudaEvent_t>(g->ev_kernel_stop), s);

@@ -89,25 +89,6 @@ struct BwdShared {
   alignas(16) float delta[2][kTile];
 };
 
-// P = exp2(s*scale + bias - L) for 32 consecutive queries of one key row; `bias` is -inf for key rows
-// that do not exist, L is +inf for query rows that do not exist: both give exactly 0.
-template <bool DIAG>
-__device__ __forceinline__ void p_fast(const uint32_t (&s)[32], const float* lse2c, float scale_log2, float bias,
-                                       int kv_idx, int q0, float (&pr)[32]) {
-#pragma unroll
-  for (int e4 = 0; e4 < 8; ++e4) {
-    const float4 L = *reinterpret_cast<const float4*>(lse2c + 4 * e4);
-    const float l[4] = {L.x, L.y, L.z, L.w};
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int e = 4 * e4 + u;
-      float v = ex2(fmaf(__uint_as_float(s[e]), scale_log2, bias) - l[u]);
-      if (DIAG) v = (kv_idx > q0 + e) ? 0.f : v;
-      pr[e] = v;
-    }
-  }
-}
-
 // Pass over one half (64 query columns) of a thread's S^T row in tensor memory, for the tiles that need it: the
 // mask term is added in score units (the common code multiplies by the scale afterwards) and (key, query) pairs
 // outside the query's TriangleAttention row group become -inf.  Loads use clamped (always valid) addresses so

@@ -1,9 +1,28 @@
-// Device helpers shared by the two backward kernels (head_dim <= 128 and head_dim in (128, 256]).
+// Device helpers shared by the backward kernels.
 #pragma once
 #include "fa_common.cuh"
 #include "fa_kernels.cuh"
 
 namespace acct {
+
+// P = exp2(s*scale + bias - L) for 32 consecutive queries of one key row; `bias` is -inf for key rows
+// that do not exist, L is +inf for query rows that do not exist: both give exactly 0.
+template <bool DIAG>
+__device__ __forceinline__ void p_fast(const uint32_t (&s)[32], const float* lse2c, float scale_log2, float bias,
+                                       int kv_idx, int q0, float (&pr)[32]) {
+#pragma unroll
+  for (int e4 = 0; e4 < 8; ++e4) {
+    const float4 L = *reinterpret_cast<const float4*>(lse2c + 4 * e4);
+    const float l[4] = {L.x, L.y, L.z, L.w};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int e = 4 * e4 + u;
+      float v = ex2(fmaf(__uint_as_float(s[e]), scale_log2, bias) - l[u]);
+      if (DIAG) v = (kv_idx > q0 + e) ? 0.f : v;
+      pr[e] = v;
+    }
+  }
+}
 
 // Keep bits of in-kernel dropout for one key row and 32 consecutive queries q0 .. q0+31 (bit e = query q0 + e).
 // The generator works on (query, 16 consecutive keys); the 32 lanes of a warp hold 32 consecutive key rows, i.e.

@@ -92,7 +92,7 @@ struct alignas(64) FwdParams {
 struct alignas(64) BwdParams {
   CUtensorMap map_q, map_k, map_v, map_do;
   CUtensorMap map_dq;               // fp32 dQ accumulator [B,N,S_q,D], box 32 x 128
-  CUtensorMap map_dk, map_dv;       // 16-bit dk, dv [B,N_kv,S_k,D], box 64 x 128 (unused with fp32 gradients and above head_dim 128)
+  CUtensorMap map_dk, map_dv;       // 16-bit dk, dv [B,N_kv,S_k,D], box 64 x 128 (unused with fp32 gradients and above head_dim 160)
   const float* lse;                 // [B,N,S_q]
   const float* delta;               // [B,N,S_q]  rowsum(dO * O)
   float* dq_acc;                    // [B,N,S_q,D] fp32, zeroed before launch
@@ -157,6 +157,9 @@ cudaError_t launch_fa_fwd(const FwdParams& p, bool bf16, int sm_count, cudaStrea
 cudaError_t launch_fa_bwd(const BwdParams& p, bool bf16, int sm_count, cudaStream_t stream);
 // head_dim in (128, 256]: Q / dO maps with 64-row boxes, the dQ map with a 32 x 64 box, two turn counters per Q tile
 cudaError_t launch_fa_bwd_wide(const BwdParams& p, bool bf16, cudaStream_t stream);
+// head_dim in (128, 160], dQ in any order: like the above with a 32 x 32 box of the dQ map, and dk, dv maps
+constexpr int kMidHeadDim = 160;
+cudaError_t launch_fa_bwd_mid(const BwdParams& p, bool bf16, cudaStream_t stream);
 // writes the {0,1} mask the kernels' in-kernel dropout uses, [units, S_q, S_k] uint8 (units = B*N)
 cudaError_t launch_dropout_mask(unsigned char* mask, int units, int S_q, int S_k, unsigned int seed_lo, unsigned int seed_hi,
                                 unsigned int offset, unsigned int threshold, cudaStream_t stream);
