@@ -6,7 +6,10 @@
 //   warps 4-7   softmax group for Q tile 1
 //   warp  8     TMA producer: Q once, then K_j / V_j into a two-stage ring
 //   warp  9     MMA issuer (one elected thread): S = Q K^T and O += P V on tcgen05
-// Tensor memory (512 columns): S0 | S1 | O0 | O1, 128 columns each.  The 16-bit probabilities are
+// Above head_dim 128 a CTA owns one Q tile, whose scores run a tile ahead into a second S buffer; up to 64 two Q tiles
+// share three S buffers, so that their scores run ahead too.
+// Tensor memory (512 columns): S0 | S1 | O0 | O1, 128 columns each (S0 | S1 | O 256 above head_dim 128, S0 | S1 | S2 |
+// O0 64 | O1 64 up to 64).  The 16-bit probabilities are
 // written back over the first 64 columns of their own S buffer and feed the second MMA straight
 // from tensor memory.  While one group runs softmax on its tile the tensor pipe works on the other
 // group's tile, so the two overlap.  A softmax thread pulls its whole 128-entry score row into
@@ -66,7 +69,10 @@ struct FwdShared {
   uint64_t q_full;
   uint64_t k_full[kStages], k_empty[kStages];
   uint64_t v_full[kStages], v_empty[kStages];
-  uint64_t s_full[2], p_half[2], p_ready[2], o_done[2];
+  // Scores are ready: per Q tile and, where they run ahead, per turn of three of its tiles (a group that has not had a tile
+  // for a while would not know which use of a shared buffer it sees).  P is ready: per S buffer (MMA sees every use).
+  uint64_t s_full[2][3], p_half[3], p_ready[3];
+  uint64_t o_done[2];                          // per Q tile: the last P V (every P V where the scores run ahead)
   uint32_t tmem_base;
   volatile uint32_t abort_flag;
   uint32_t need[2][kPlanWords];           // K/V tiles of each Q tile that the mask plan leaves (all ones without a plan)
@@ -86,7 +92,12 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
   // CTA then owns ONE Q tile (softmax group 1 idles) and K and V have one stage each.
   constexpr int NQ = DPAD > 128 ? 1 : 2;        // Q tiles per CTA
   constexpr int kSt = DPAD > 128 ? 1 : kStages;  // K/V stages
-  constexpr uint32_t kColS = 0, kColO = NQ * 128;
+  // Where tensor memory has room, the scores run ahead of P V: one Q tile has two S buffers (8 x 8 heads of 160, 1 024 tokens:
+  // 104 -> 77 us; prefill 4 x 16 heads, 2 048 tokens: 299 -> 202 us), two Q tiles of head_dim up to 64 have three between
+  // them (2 x 8 heads of 40, 4 096 tokens: 115.6 -> 112.7 us; with a mask or alibi it gains nothing: documents of 1 500 tokens
+  // 109 -> 113 us).
+  constexpr bool kAhead = DPAD == 64 && MODS == 0;
+  constexpr uint32_t kColS = 0, kColO = kAhead ? 384 : 256;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -173,10 +184,10 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
       mbar_init(&sh.k_full[s], 1); mbar_init(&sh.k_empty[s], 1);
       mbar_init(&sh.v_full[s], 1); mbar_init(&sh.v_empty[s], 1);
     }
-    for (int q = 0; q < 2; ++q) {
-      mbar_init(&sh.s_full[q], 1); mbar_init(&sh.p_half[q], 128); mbar_init(&sh.p_ready[q], 128);
-      mbar_init(&sh.o_done[q], 1);
+    for (int s = 0; s < 3; ++s) {
+      mbar_init(&sh.s_full[0][s], 1); mbar_init(&sh.s_full[1][s], 1); mbar_init(&sh.p_half[s], 128); mbar_init(&sh.p_ready[s], 128);
     }
+    mbar_init(&sh.o_done[0], 1); mbar_init(&sh.o_done[1], 1);
     sh.abort_flag = 0;
     mbar_fence_init();
   }
@@ -192,23 +203,39 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
     reg_dealloc<kRegsControl>();
     if (cta_hi >= cta_lo && elect_one()) {
       prefetch_tmap(&p.map_q); prefetch_tmap(&p.map_k); prefetch_tmap(&p.map_v); prefetch_tmap(&p.map_o);
-      mbar_expect_tx(&sh.q_full, NQ * kTileBytes);
+      const int blocks = NQ == 1 ? (p.D + 63) / 64 : NB;    // 64-column blocks that hold anything
+      const uint32_t tile_bytes = blocks * 16384u;
+      mbar_expect_tx(&sh.q_full, NQ * tile_bytes);
       for (int qt = 0; qt < NQ; ++qt)
-        for (int nb = 0; nb < NB; ++nb)
+        for (int nb = 0; nb < blocks; ++nb)
           tma_load_4d(sQ + qt * kTileBytes + nb * 16384, &p.map_q, &sh.q_full, nb * 64,
                       (NQ * pair + qt) * kTile, h, b);
-      int it = 0;
-      for (int j = cta_lo; j <= cta_hi; j = next_any(j), ++it) {
+      auto load_k = [&](int it, int j) {
         const int st = it % kSt;
-        const uint32_t reuse_parity = ((it / kSt) - 1) & 1;
-        if (it >= kSt) mbar_wait(&sh.k_empty[st], reuse_parity, abort_flag, p.status, DEV_TIMEOUT_SYNC);
-        mbar_expect_tx(&sh.k_full[st], kTileBytes);
-        for (int nb = 0; nb < NB; ++nb)
+        if (it >= kSt) mbar_wait(&sh.k_empty[st], ((it / kSt) - 1) & 1, abort_flag, p.status, DEV_TIMEOUT_SYNC);
+        mbar_expect_tx(&sh.k_full[st], tile_bytes);
+        for (int nb = 0; nb < blocks; ++nb)
           tma_load_4d(sK + st * kTileBytes + nb * 16384, &p.map_k, &sh.k_full[st], nb * 64, j * kTile, h_kv, b);
-        if (it >= kSt) mbar_wait(&sh.v_empty[st], reuse_parity, abort_flag, p.status, DEV_TIMEOUT_SYNC);
-        mbar_expect_tx(&sh.v_full[st], kTileBytes);
-        for (int nb = 0; nb < NB; ++nb)
+      };
+      auto load_v = [&](int it, int j) {
+        const int st = it % kSt;
+        if (it >= kSt) mbar_wait(&sh.v_empty[st], ((it / kSt) - 1) & 1, abort_flag, p.status, DEV_TIMEOUT_SYNC);
+        mbar_expect_tx(&sh.v_full[st], tile_bytes);
+        for (int nb = 0; nb < blocks; ++nb)
           tma_load_4d(sV + st * kTileBytes + nb * 16384, &p.map_v, &sh.v_full[st], nb * 64, j * kTile, h_kv, b);
+      };
+      if constexpr (NQ == 1) {
+        // the scores run a tile ahead of P V: K of the next tile before V of this one
+        int it = 0, j_before = 0;
+        for (int j = cta_lo; j <= cta_hi; j = next_any(j), ++it) {
+          load_k(it, j);
+          if (it > 0) load_v(it - 1, j_before);
+          j_before = j;
+        }
+        load_v(it - 1, j_before);
+      } else {
+        int it = 0;
+        for (int j = cta_lo; j <= cta_hi; j = next_any(j), ++it) { load_k(it, j); load_v(it, j); }
       }
     }
   } else if (warp == 9) {
@@ -221,7 +248,10 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
     reg_dealloc<kRegsControl>();
     if (cta_hi >= cta_lo) {
       const uint32_t idesc_s = make_idesc(BF16, 128, 128, false, false);
-      const uint32_t idesc_o = make_idesc(BF16, 128, DPAD, false, true);
+      // steps of the contraction over head_dim, and 16-column groups of O, that hold anything (only the widest kernel has
+      // many to save: a test before every MMA cost head_dim 128 one to four percent)
+      const int k_steps = NQ == 1 ? (p.D + 15) / 16 : DPAD / 16;
+      const uint32_t idesc_o = make_idesc(BF16, 128, k_steps * 16, false, true);
       const uint64_t kmajor = make_sdesc_base(16, 1024);
       const uint64_t mnmajor = make_sdesc_base(16384, 1024);
       const uint32_t k_hi = static_cast<uint32_t>(kmajor >> 32), k_lo = static_cast<uint32_t>(kmajor);
@@ -235,22 +265,122 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
       constexpr uint32_t kTileUnits = kTileBytes >> 4;
       mbar_wait(&sh.q_full, 0, abort_flag, p.status, DEV_TIMEOUT_TMA);
 
-      auto issue_s = [&](int qt, int st) {
+      auto issue_s = [&](int qt, int buf, int st, int turn) {
         const uint32_t a0 = q_lo + qt * kTileUnits, b0 = kt_lo + st * kTileUnits;
         if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < DPAD / 16; ++kk) {
             const uint32_t off = (kk >> 2) * 1024u + (kk & 3) * 2u;   // 16-byte units
-            umma_ss_lohi(tmem + kColS + qt * 128, a0 + off, k_hi, b0 + off, k_hi, idesc_s, kk > 0);
+            if (NQ > 1 || kk < k_steps) umma_ss_lohi(tmem + kColS + buf * 128, a0 + off, k_hi, b0 + off, k_hi, idesc_s, kk > 0);
           }
-          umma_commit(&sh.s_full[qt]);
+          umma_commit(&sh.s_full[qt][turn]);
         }
       };
 
+      if constexpr (NQ == 1) {
+        // One Q tile, two S buffers: the scores of the next tile are issued before this tile's P V, so that the softmax
+        // group finds them when it is through with this one.
+        mbar_wait(&sh.k_full[0], 0, abort_flag, p.status, DEV_TIMEOUT_TMA);
+        issue_s(0, 0, 0, 0);
+        if (elect_one()) umma_commit(&sh.k_empty[0]);
+        int it = 0, jn;
+        for (int j = cta_lo; j <= cta_hi; j = jn, ++it) {
+          jn = next_any(j);
+          const int buf = it & 1;
+          if (jn <= cta_hi) {       // (its buffer's P was consumed by the P V before this one: the tensor pipe runs in order)
+            mbar_wait(&sh.k_full[0], (it + 1) & 1, abort_flag, p.status, DEV_TIMEOUT_TMA);
+            tc_fence_after_sync();
+            issue_s(0, buf ^ 1, 0, buf ^ 1);
+            if (elect_one()) umma_commit(&sh.k_empty[0]);
+          }
+          mbar_wait(&sh.v_full[0], it & 1, abort_flag, p.status, DEV_TIMEOUT_TMA);
+          mbar_wait(&sh.p_half[buf], (it >> 1) & 1, abort_flag, p.status, DEV_TIMEOUT_SYNC);
+          tc_fence_after_sync();
+          const uint32_t t_s = tmem + kColS + buf * 128, t_o = tmem + kColO;
+          if (elect_one()) {
+#pragma unroll
+            for (int kk = 0; kk < kTile / 32; ++kk)
+              umma_ts_lohi(t_o, t_s + kk * 8, vt_lo + kk * 128u, mn_hi, idesc_o, it > 0 || kk > 0);
+          }
+          mbar_wait(&sh.p_ready[buf], (it >> 1) & 1, abort_flag, p.status, DEV_TIMEOUT_SYNC);
+          tc_fence_after_sync();
+          if (elect_one()) {
+#pragma unroll
+            for (int kk = kTile / 32; kk < kTile / 16; ++kk)
+              umma_ts_lohi(t_o, t_s + kk * 8, vt_lo + kk * 128u, mn_hi, idesc_o, true);
+            umma_commit(&sh.o_done[0]);
+            umma_commit(&sh.v_empty[0]);
+          }
+        }
+      } else if constexpr (kAhead) {
+        // Two Q tiles, three S buffers taken in turn: the scores of (tile, Q tile) number t + 3 are issued as soon as the
+        // P V of number t has consumed its buffer, so a softmax group that is through with a tile finds the next one.
+        auto advance = [&](int& j, int& qt) {          // in the order (first K/V tile, Q tile 0), (.., Q tile 1), ..
+          do {
+            if (qt == 0) { qt = 1; } else { qt = 0; j = next_any(j); }
+          } while (j <= cta_hi && !needed(qt, qt == 0 ? r0 : r1, j));
+        };
+        int js = cta_lo, qs = 0, it_k = 0, buf_s = 0, turn0 = 0, turn1 = 0;   // next scores
+        bool k_new = true;
+        if (!needed(0, r0, js)) advance(js, qs);
+        auto next_scores = [&]() {
+          if (js > cta_hi) return;
+          const int st = it_k % kSt;
+          if (k_new) {
+            mbar_wait(&sh.k_full[st], (it_k / kSt) & 1, abort_flag, p.status, DEV_TIMEOUT_TMA);
+            tc_fence_after_sync();
+          }
+          int& turn = qs == 0 ? turn0 : turn1;
+          issue_s(qs, buf_s, st, turn);
+          turn = turn == 2 ? 0 : turn + 1;
+          buf_s = buf_s == 2 ? 0 : buf_s + 1;
+          const int j = js;
+          advance(js, qs);
+          k_new = js != j;
+          if (k_new) {
+            if (elect_one()) umma_commit(&sh.k_empty[st]);
+            ++it_k;
+          }
+        };
+        for (int i = 0; i < 3; ++i) next_scores();
+        int jp = cta_lo, qp = 0, it_v = 0, buf = 0;    // next P V
+        uint32_t parity = 0;
+        bool v_new = true, fresh0 = true, fresh1 = true;   // no P V into O of the Q tile yet
+        if (!needed(0, r0, jp)) advance(jp, qp);
+        while (jp <= cta_hi) {
+          const int st = it_v % kSt;
+          const uint32_t t_s = tmem + kColS + buf * 128, t_o = tmem + kColO + qp * DPAD, v0 = vt_lo + st * kTileUnits;
+          if (v_new) mbar_wait(&sh.v_full[st], (it_v / kSt) & 1, abort_flag, p.status, DEV_TIMEOUT_TMA);
+          mbar_wait(&sh.p_half[buf], parity, abort_flag, p.status, DEV_TIMEOUT_SYNC);
+          tc_fence_after_sync();
+          const bool first = qp == 0 ? fresh0 : fresh1;
+          if (elect_one()) {
+#pragma unroll
+            for (int kk = 0; kk < kTile / 32; ++kk)
+              umma_ts_lohi(t_o, t_s + kk * 8, v0 + kk * 128u, mn_hi, idesc_o, !first || kk > 0);
+          }
+          mbar_wait(&sh.p_ready[buf], parity, abort_flag, p.status, DEV_TIMEOUT_SYNC);
+          tc_fence_after_sync();
+          const int j = jp, qt = qp;
+          if (qt == 0) fresh0 = false; else fresh1 = false;
+          advance(jp, qp);
+          v_new = jp != j;
+          if (elect_one()) {
+#pragma unroll
+            for (int kk = kTile / 32; kk < kTile / 16; ++kk)
+              umma_ts_lohi(t_o, t_s + kk * 8, v0 + kk * 128u, mn_hi, idesc_o, true);
+            umma_commit(&sh.o_done[qt]);
+            if (v_new) umma_commit(&sh.v_empty[st]);
+          }
+          if (v_new) ++it_v;
+          if (++buf == 3) { buf = 0; parity ^= 1u; }
+          next_scores();
+        }
+      } else {
       // prologue: scores of the first K/V tile
       mbar_wait(&sh.k_full[0], 0, abort_flag, p.status, DEV_TIMEOUT_TMA);
-      for (int qt = 0; qt < 2; ++qt)
-        if (needed(qt, rng[qt], cta_lo)) issue_s(qt, 0);
+      for (int qt = 0; qt < NQ; ++qt)
+        if (needed(qt, rng[qt], cta_lo)) issue_s(qt, qt, 0, 0);
       if (elect_one()) umma_commit(&sh.k_empty[0]);
       mbar_wait(&sh.v_full[0], 0, abort_flag, p.status, DEV_TIMEOUT_TMA);
       int it = 0;
@@ -295,7 +425,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
             // every commit costs this thread 80-95 cycles in which it issues nothing
             ++n_done[qt];
           }
-          if (sn) issue_s(qt, stn);
+          if (sn) issue_s(qt, qt, stn, 0);
         }
         if (elect_one()) {
           umma_commit(&sh.v_empty[st]);
@@ -305,6 +435,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
           // the next V tile, waited for while the MMAs just issued still execute
           mbar_wait(&sh.v_full[stn], full_parity_n, abort_flag, p.status, DEV_TIMEOUT_TMA);
         }
+      }
       }
     }
   } else if (warp >= 10) {
@@ -318,7 +449,6 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
     const int row_in_tile = tid & 127;
     const int q_row = q_tile * kTile + row_in_tile;
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const uint32_t t_s = tmem + lane_base + kColS + qt * 128;
     const uint32_t t_o = tmem + lane_base + kColO + qt * DPAD;
     constexpr bool GENERIC = MODS != 0;
     const bool has_alibi = (MODS & 2) != 0 && (mods.alibi != nullptr || mods.alibi_slopes != nullptr);
@@ -365,7 +495,21 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
       uint4 row_bits = make_uint4(0u, 0u, 0u, 0u);
       if constexpr ((MODS & 1) != 0) if (mask_class == 3)
         row_bits = reinterpret_cast<const uint4*>(mods.plan.bits + (tile_class + j - mods.plan.cls) * kPlanBitWords)[row_in_tile];
-      mbar_wait(&sh.s_full[qt], n & 1, abort_flag, p.status, DEV_TIMEOUT_MMA);
+      // S buffer of this tile, and which barrier and phase say that its scores are there
+      int buf = qt, turn = 0;
+      uint32_t s_parity = n & 1;
+      if constexpr (NQ == 1) { buf = turn = n & 1; s_parity = (n >> 1) & 1; }
+      if constexpr (kAhead) {
+        // its number in the order of the MMA warp: this group's tiles before it, and the other's (its tile of the same j
+        // comes before for Q tile 1)
+        const TileRange& other = qt == 0 ? r1 : r0;
+        const int before = max(0, min(j + qt - other.lo, other.hi - other.lo + 1));
+        buf = static_cast<uint32_t>(n + before) % 3u;
+        turn = static_cast<uint32_t>(n) % 3u;
+        s_parity = (static_cast<uint32_t>(n) / 3u) & 1u;
+      }
+      const uint32_t t_s = tmem + lane_base + kColS + buf * 128;
+      mbar_wait(&sh.s_full[qt][turn], s_parity, abort_flag, p.status, DEV_TIMEOUT_MMA);
       tc_fence_after_sync();
       const int col_base = j * kTile;
       // a mask tile that is all 1 adds one constant to every score of the tile: without alibi it is folded into
@@ -599,10 +743,16 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
         m_run = m_new;
         l_run *= alpha;
       }
+      if constexpr (NQ == 1 || kAhead) if (n > 0) {
+        // (for every tile, so that no phase goes by unseen; the P V of the tile before is long issued)
+        mbar_wait(&sh.o_done[qt], (n - 1) & 1, abort_flag, p.status, DEV_TIMEOUT_MMA);
+        tc_fence_after_sync();
+      }
       if (n > 0 && any_grow) {
-        // O of the previous tiles is complete (the S MMA just waited for was issued after their P V)
+        // O of the previous tiles is complete: the S MMA just waited for was issued after their P V, or, where the scores
+        // run ahead, that P V has been waited for
 #pragma unroll 1
-        for (int c = 0; c < DPAD / 32; ++c) {
+        for (int c = 0; c < DPAD / 32 && (NQ > 1 || c * 32 < p.D); ++c) {
           uint32_t r[32];
           tmem_ld32(t_o + c * 32, r);
           tmem_wait_ld();
@@ -627,7 +777,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
         tmem_st16(t_s + 16, pk);
         tmem_wait_st();
         tc_fence_before_sync();
-        mbar_arrive(&sh.p_half[qt]);
+        mbar_arrive(&sh.p_half[buf]);
       }
       {
         // the second half as one store: the exponentials of chunk 3 overlap the tail of chunk 2
@@ -645,14 +795,14 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
       }
       tmem_wait_st();
       tc_fence_before_sync();
-      mbar_arrive(&sh.p_ready[qt]);
+      mbar_arrive(&sh.p_ready[buf]);
     }
 
     // epilogue: O / l through this group's (now dead) Q tile in shared memory and a TMA store, which
     // clips rows past S_q and columns past D; L = m + ln l straight to global memory
     if (qt < NQ && q_tile * kTile < p.S_q) {
       if (n > 0) {
-        mbar_wait(&sh.o_done[qt], 0, abort_flag, p.status, DEV_TIMEOUT_MMA);
+        mbar_wait(&sh.o_done[qt], NQ == 1 || kAhead ? (n - 1) & 1 : 0, abort_flag, p.status, DEV_TIMEOUT_MMA);
         tc_fence_after_sync();
       } else if (cta_hi >= cta_lo) {
         // no K/V tile for this Q tile, but its TMA load was issued: let it land before the tile is reused
@@ -661,7 +811,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
       const float inv_l = (n > 0 && l_run > 0.f) ? 1.0f / l_run : 0.f;
       uint8_t* stage = sQ + qt * kTileBytes;
 #pragma unroll 1
-      for (int c = 0; c < DPAD / 32; ++c) {
+      for (int c = 0; c < DPAD / 32 && (NQ > 1 || c * 32 < p.D); ++c) {
         uint32_t r[32];
         if (n > 0) { tmem_ld32(t_o + c * 32, r); tmem_wait_ld(); }
         else {
