@@ -268,7 +268,9 @@ unsigned int dropout_threshold(float keep_prob) {
 
 // A mask plan pays where a mask tensor with a summary is the only thing that limits the scores and there is enough work:
 // its passes cost 8 us and one read of q, k and v, a tile pair of forward and backward about 6 us on its SM.  3 000 tokens of
-// four documents, 2 x 32 heads of 128 (36 864 tile pairs): forward and backward 1 476 -> 479 us.  A band, valid lengths, row groups and alibi set limits or add terms that the bounds do not
+// four documents, 2 x 32 heads of 128 (36 864 tile pairs): forward and backward 1 476 -> 479 us.  At the line, 32 heads and 2 048
+// tokens of four documents (8 192 pairs), 392 -> 213 us; far below it launches are what a call costs, and three more of them
+// would be added.  A band, valid lengths, row groups and alibi set limits or add terms that the bounds do not
 // cover; a dropout tensor may hold any factor.
 constexpr int64_t kPlanMinTilePairs = 8192;
 constexpr int64_t kPlanMaxMaskTiles = 16384;      // 64 MB of bits (an eighth of the mask's own size in 16 bits, twice)

@@ -1,4 +1,5 @@
-// FlashAttention-2 backward for head_dim in (128, 256] on sm_100a.
+// FlashAttention-2 backward for head_dim in (160, 256] on sm_100a, and in (128, 160] where dQ is summed in a fixed order
+// (without that, fa_bwd_mid.cu takes those widths).
 //
 // At these widths the dK and dV accumulators of one 128-row K/V tile would fill tensor memory on their own
 // (2 x 256 columns), and full-width K, V, Q and dO tiles would not fit shared memory.  So the work of one K/V tile is
@@ -15,7 +16,7 @@
 // 40 for an unsplit product, the price of fitting.  Tensor memory: S^T 64 | dP^T 64 | dQ^T 64 | (64 unused) |
 // dK half 128 | dV half 128.  Shared memory: K and V whole (2 x 64 KB), one Q and one dO sub-tile of 64 rows
 // (2 x 32 KB, single-buffered), dS^T (16 KB), dQ staging (16 KB).  The single Q / dO buffers make this kernel
-// latency-bound: it exists so that every head_dim the reference cell accepts (up to 256,
+// latency-bound (at head_dim 160 three times slower than fa_bwd_mid.cu): it exists so that every head_dim the reference cell accepts (up to 256,
 // train/acctransformer/flash_attention/nn/layer/flash_attention.py:26,105-106) trains; the head_dim <= 128 kernel
 // is the optimised one.  Mask, alibi, dropout (both forms), band, row groups and valid lengths are all handled on
 // one general path, element by element.
