@@ -260,7 +260,8 @@ def mask_tile_classes(attn_mask):
     if m.dim() == 2:
         m = m.unsqueeze(0)
     lib = load()
-    tiles = torch.empty((m.shape[0], -(-m.shape[1] // 128), -(-m.shape[2] // 128)), dtype=torch.uint8, device=m.device)
+    with torch.inference_mode(False):      # (remembered beyond a call under inference mode, so not an inference tensor)
+        tiles = torch.empty((m.shape[0], -(-m.shape[1] // 128), -(-m.shape[2] // 128)), dtype=torch.uint8, device=m.device)
     assert tiles.numel() == lib.acct_mask_tiles_bytes(m.shape[0], m.shape[1], m.shape[2])
     with torch.cuda.device(m.device):
         check(lib.acct_mask_classify_tiles(m.data_ptr(), _dtype_code(m, "attn_mask"), m.shape[0], m.shape[1], m.shape[2],

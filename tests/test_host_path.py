@@ -55,3 +55,27 @@ def test_forward_mode_is_refused():
     with fwad.dual_level():
         with pytest.raises(NotImplementedError):
             _layer(64)(fwad.make_dual(q, t), k, v)
+
+
+def _documents(S, dtype=torch.float16):
+    """Two documents, causal inside each: [1, S, S], 1 where a key must not be seen."""
+    pos = torch.arange(S, device="cuda")
+    doc = pos >= S // 3
+    return ((doc[:, None] != doc[None, :]) | (pos[None, :] > pos[:, None])).to(dtype)[None]
+
+
+def _grads(layer, qkv, d_o, *rest):
+    xs = [t.detach().requires_grad_() for t in qkv]
+    return torch.autograd.grad(layer(*xs, *rest), xs, d_o)
+
+
+def test_mask_first_seen_under_inference_mode_can_be_trained_with():
+    q, k, v, d_o = _inputs(1, 2, 200, 64)
+    mask = _documents(200)
+    with torch.inference_mode():
+        _layer(64)(q, k, v, mask)
+    got = _grads(_layer(64), (q, k, v), d_o, mask)
+    want = _grads(_layer(64), (q, k, v), d_o, mask.clone())
+    # (dq is a sum over two K/V tiles: no order to depend on)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
