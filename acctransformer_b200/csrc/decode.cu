@@ -379,25 +379,46 @@ __global__ void __launch_bounds__(kDecodeThreads) decode_split_kernel(const Deco
   if constexpr (CL) cluster_merge<BF16>(p, &s_part[0][0], s_pm, s_pl, DMAX, b, h_kv, kDecodeThreads);
 }
 
+// One block per query head, one thread per column, at most 64 parts: lane s of every warp holds part s (and 32 + s).  What
+// bounds it is latency, so all loads of the first 16 parts and of the running maxima and sums are out before anything
+// waits.  A whole step of 256 heads of 128 over 64 keys in 8 / 16 parts: 11.0 / 15.2 us with plain loops over the parts (9.9 /
+// 13.8 where the compiler happens to pipeline them), 9.4 / 13.0 us like this.
 template <bool BF16>
 __global__ void decode_merge_kernel(const DecodeParams p) {
-  const int unit = blockIdx.x;
-  const float* ml = p.part_ml + static_cast<int64_t>(unit) * p.splits * 2;
-  float big = -INFINITY;
-  for (int s = 0; s < p.splits; ++s) big = fmaxf(big, ml[2 * s]);
-  float lsum = 0.f;
-  for (int s = 0; s < p.splits; ++s) lsum += (ml[2 * s] == -INFINITY) ? 0.f : ml[2 * s + 1] * ex2(ml[2 * s] - big);
-  const float inv = lsum > 0.f ? 1.0f / lsum : 0.f;
-  for (int t = threadIdx.x; t < p.D; t += blockDim.x) {
-    float a = 0.f;
-    for (int s = 0; s < p.splits; ++s) {
-      const float w = (ml[2 * s] == -INFINITY) ? 0.f : ex2(ml[2 * s] - big);
-      a = fmaf(p.part_acc[(static_cast<int64_t>(unit) * p.splits + s) * p.D + t], w, a);
+  constexpr int kBatch = 16;
+  const int unit = blockIdx.x, n = p.splits, t = threadIdx.x, lane = t & 31;
+  const float* part = p.part_acc + static_cast<int64_t>(unit) * n * p.D + t;
+  const float2* ml = reinterpret_cast<const float2*>(p.part_ml) + static_cast<int64_t>(unit) * n;
+  float v[kBatch];
+  auto load = [&](int s0) {
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) v[i] = s0 + i < n && t < p.D ? part[static_cast<int64_t>(s0 + i) * p.D] : 0.f;
+  };
+  load(0);
+  const float2 none = make_float2(-INFINITY, 0.f);
+  const float2 e0 = lane < n ? ml[lane] : none, e1 = 32 + lane < n ? ml[32 + lane] : none;
+  float big = fmaxf(e0.x, e1.x);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, off));
+  const float w0 = e0.x == -INFINITY ? 0.f : ex2(e0.x - big), w1 = e1.x == -INFINITY ? 0.f : ex2(e1.x - big);
+  float a = 0.f, lsum = 0.f;
+  for (int s0 = 0; s0 < n; s0 += kBatch) {
+    if (s0 > 0) load(s0);
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      if (s0 + i >= n) break;
+      const int from = (s0 + i) & 31;
+      const float w = __shfl_sync(0xffffffffu, s0 < 32 ? w0 : w1, from);
+      const float l = __shfl_sync(0xffffffffu, s0 < 32 ? e0.y : e1.y, from);
+      lsum = fmaf(l, w, lsum);
+      a = fmaf(v[i], w, a);
     }
-    a *= inv;
-    if constexpr (BF16) reinterpret_cast<__nv_bfloat16*>(p.y)[static_cast<int64_t>(unit) * p.D + t] = __float2bfloat16(a);
-    else reinterpret_cast<__half*>(p.y)[static_cast<int64_t>(unit) * p.D + t] = __float2half(a);
   }
+  if (t >= p.D) return;
+  a *= lsum > 0.f ? 1.0f / lsum : 0.f;
+  const int64_t at = static_cast<int64_t>(unit) * p.D + t;
+  if constexpr (BF16) reinterpret_cast<__nv_bfloat16*>(p.y)[at] = __float2bfloat16(a);
+  else reinterpret_cast<__half*>(p.y)[at] = __float2half(a);
 }
 
 cudaError_t launch_merge(const DecodeParams& p, bool bf16, cudaStream_t stream) {

@@ -37,3 +37,26 @@ def test_clustered_parts_against_the_oracle(B, n_kv, group, S, D, dtype):
     # probabilities are rounded to 16 bits too (at most 2^-11 / 2^-8 of the largest |v|, about 4)
     tol = 4e-3 if dtype == "float16" else 3e-2
     assert float(np.max(np.abs(y.float().cpu().numpy() - want))) <= tol
+
+
+# the second kernel, which merges the parts where they are no cluster: batches of 16 parts, two halves of 32; empty parts
+@pytest.mark.parametrize("splits", [1, 2, 15, 16, 17, 32, 33, 49, 64])
+@pytest.mark.parametrize("group,D,dtype", [(1, 40, "float16"), (4, 128, "bfloat16"), (1, 256, "float16")])
+def test_merge_of_any_number_of_parts(splits, group, D, dtype):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from acctransformer_b200 import _lib, ops
+    dt = getattr(torch, dtype)
+    B, n_kv, S = 3, 2, 4200
+    g = torch.Generator().manual_seed(splits + D)
+    q = torch.randn(B, n_kv * group, 1, D, generator=g).to(dt)
+    k, v = (torch.randn(B, n_kv, S, D, generator=g).to(dt) for _ in range(2))
+    lens = torch.tensor([1, 2000, S], dtype=torch.int32)
+    scale = 1.0 / math.sqrt(D)
+    y = ops.infer_decode(q.cuda(), k.cuda(), v.cuda(), lens.cuda(), scale=scale, num_splits=splits)
+    torch.cuda.synchronize()
+    _lib.device_status()
+    want = ref.decode_ref(q.float().numpy(), k.float().numpy().repeat(group, axis=1), v.float().numpy().repeat(group, axis=1),
+                          lens.numpy(), scale)
+    tol = 4e-3 if dtype == "float16" else 3e-2      # as above
+    assert float(np.max(np.abs(y.float().cpu().numpy() - want))) <= tol
