@@ -75,6 +75,19 @@ void require_cuda(const char* name, const Tensor& t) {
   HOST_CHECK(t.defined() && t.is_cuda(), name, " must be a CUDA tensor (this library has no CPU path)");
 }
 
+// Every pointer that a kernel gets is checked here: a host address or one of another GPU would fault on the device.
+void require_on(const char* name, const Tensor& t, const Tensor& q) {
+  require_cuda(name, t);
+  HOST_CHECK(t.device() == q.device(), name, " must be on the device of q, ", q.device(), ", not on ", t.device());
+}
+
+// valid lengths as the kernels read them: at least one int32 per sequence
+Tensor lengths(const Tensor& lens, int64_t B, const Tensor& q) {
+  require_on("seq_lens", lens, q);
+  HOST_CHECK(lens.numel() >= B, "seq_lens must hold a length for each of ", B, " sequences, got ", lens.numel());
+  return lens.to(at::kInt).contiguous();
+}
+
 void strides3(const Tensor& t, int64_t (&out)[3]) {
   HOST_CHECK(t.stride(-1) == 1, "head_dim must be contiguous");
   for (int i = 0; i < 3; ++i) out[i] = t.stride(i);
@@ -140,7 +153,7 @@ void check_fa_inputs(const Tensor& q, const Tensor& k, const Tensor& v, Tensor& 
   const Tensor* qkv[3] = {&q, &k, &v};
   const char* names[3] = {"q", "k", "v"};
   for (int i = 0; i < 3; ++i) {
-    require_cuda(names[i], *qkv[i]);
+    require_on(names[i], *qkv[i], q);
     HOST_CHECK(qkv[i]->dim() == 4, names[i], " must be [B, N, S, D]");
   }
   const auto dt = q.scalar_type();
@@ -150,7 +163,7 @@ void check_fa_inputs(const Tensor& q, const Tensor& k, const Tensor& v, Tensor& 
   HOST_CHECK(k.size(0) == B && k.size(3) == D && v.sizes() == k.sizes() && N_kv >= 1 && N % N_kv == 0, "shape mismatch: q ",
              q.sizes(), ", k ", k.sizes(), ", v ", v.sizes(), " (k and v may have fewer heads than q if their head count divides q's)");
   if (mask.defined()) {
-    require_cuda("attn_mask", mask);
+    require_on("attn_mask", mask, q);
     mask = mask.contiguous();
     if (c.mask_tile128) {
       HOST_CHECK(mask.numel() == 128 * 128, "the tile form of attn_mask must hold 128x128 elements");
@@ -162,21 +175,21 @@ void check_fa_inputs(const Tensor& q, const Tensor& k, const Tensor& v, Tensor& 
   }
   if (tiles.defined()) {
     HOST_CHECK(mask.defined() && !c.mask_tile128, "mask_tiles goes with a full attn_mask tensor");
-    require_cuda("mask_tiles", tiles);
+    require_on("mask_tiles", tiles, q);
     const int64_t mb = mask.dim() == 2 ? 1 : mask.size(0);
     HOST_CHECK(tiles.scalar_type() == at::kByte && tiles.is_contiguous() && tiles.dim() == 3 && tiles.size(0) == mb &&
                    tiles.size(1) == (S_q + 127) / 128 && tiles.size(2) == (S_k + 127) / 128,
                "mask_tiles must be a contiguous uint8 tensor as mask_tile_classes() returns it");
   }
   if (drop.defined()) {
-    require_cuda("dropout_mask", drop);
+    require_on("dropout_mask", drop, q);
     HOST_CHECK(drop.dim() == 4 && drop.size(0) == B && drop.size(1) == N && drop.size(2) == S_q && drop.size(3) == S_k,
                "dropout_mask must be [B, N, S_q, S_k]");
     HOST_CHECK(!c.has_seed, "give either dropout_mask (tensor form) or dropout_seed (in-kernel form), not both");
     drop = drop.contiguous();
   }
   if (alibi.defined()) {
-    require_cuda("alibi", alibi);
+    require_on("alibi", alibi, q);
     HOST_CHECK(alibi.dim() == 4 && alibi.size(0) == B && alibi.size(1) == N && alibi.size(2) == 1 && alibi.size(3) == S_k &&
                    alibi.scalar_type() == dt,
                "alibi must be [B, N, 1, S_k] in the dtype of q");
@@ -372,7 +385,8 @@ PyObject* py_infer_prefill(PyObject*, PyObject* const* args, Py_ssize_t n) {
   {
     pybind11::gil_scoped_release no_gil;
     at::AutoDispatchBelowADInplaceOrView below;
-    require_cuda("q", q); require_cuda("k", k); require_cuda("v", v);
+    require_cuda("q", q); require_on("k", k, q); require_on("v", v, q);
+    HOST_CHECK(k.scalar_type() == q.scalar_type() && v.scalar_type() == q.scalar_type(), "q, k, v must share one dtype");
     const int64_t rank = q.dim();
     HOST_CHECK(rank == 3 || rank == 4, "q must have rank 3 or 4");
     HOST_CHECK(k.dim() == rank && v.dim() == rank && k.sizes() == v.sizes(), "k and v must have q's rank and one shape");
@@ -392,7 +406,7 @@ PyObject* py_infer_prefill(PyObject*, PyObject* const* args, Py_ssize_t n) {
     a.causal = causal ? 1 : 0;
     a.scale = static_cast<float>(scale);
     if (lens.defined()) {
-      lens = lens.to(at::kInt).contiguous();
+      lens = lengths(lens, a.B, q);
       a.seq_lens = static_cast<const int32_t*>(lens.const_data_ptr());
     }
     check(g_lib.infer_prefill(&a, stream_of(q)));
@@ -414,7 +428,9 @@ PyObject* py_infer_decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
   {
     pybind11::gil_scoped_release no_gil;
     at::AutoDispatchBelowADInplaceOrView below;
-    require_cuda("q", q); require_cuda("k_cache", k); require_cuda("v_cache", v);
+    require_cuda("q", q); require_on("k_cache", k, q); require_on("v_cache", v, q); require_on("workspace", ws, q);
+    HOST_CHECK(k.scalar_type() == q.scalar_type() && v.scalar_type() == q.scalar_type(),
+               "q, k_cache, v_cache must share one dtype");
     HOST_CHECK(q.dim() == 4 && q.size(2) == 1, "decode takes one query token: q must be [B, N, 1, D]");
     const int64_t B = q.size(0), N = q.size(1), D = q.size(3);
     const bool paged = table.defined();
@@ -424,13 +440,19 @@ PyObject* py_infer_decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HOST_CHECK(k.strides() == v.strides(), "k_cache and v_cache must share strides");
     c10::cuda::OptionalCUDAGuard guard(q.device());
     q = q.contiguous();
-    if (!y.defined()) y = empty_like_shape(q.sizes(), q.scalar_type(), q);
+    if (y.defined()) {
+      require_on("out", y, q);
+      HOST_CHECK(y.scalar_type() == q.scalar_type() && y.is_contiguous() && y.numel() == q.numel(),
+                 "out must be a contiguous tensor with the dtype and the number of elements of q");
+    } else {
+      y = empty_like_shape(q.sizes(), q.scalar_type(), q);
+    }
     acct_decode_args a;
     memset(&a, 0, sizeof(a));
     a.dtype = q.scalar_type() == at::kHalf ? ACCT_F16 : q.scalar_type() == at::kBFloat16 ? ACCT_BF16 : -1;
     a.B = B; a.N = N; a.D = D; a.N_kv = k.size(1);
     if (paged) {
-      require_cuda("block_table", table);
+      require_on("block_table", table, q);
       table = table.to(at::kInt).contiguous();
       HOST_CHECK(table.dim() == 2 && table.size(0) == B, "block_table must be [B, max_pages]");
       a.block_table = static_cast<const int32_t*>(table.const_data_ptr());
@@ -443,7 +465,7 @@ PyObject* py_infer_decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
     a.q = q.const_data_ptr(); a.k_cache = k.const_data_ptr(); a.v_cache = v.const_data_ptr(); a.y = y.data_ptr();
     strides3(k, a.kv_stride);
     if (lens.defined()) {
-      lens = lens.to(at::kInt).contiguous();
+      lens = lengths(lens, a.B, q);
       a.seq_lens = static_cast<const int32_t*>(lens.const_data_ptr());
     }
     a.scale = static_cast<float>(scale);

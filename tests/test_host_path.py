@@ -79,3 +79,76 @@ def test_mask_first_seen_under_inference_mode_can_be_trained_with():
     # (dq is a sum over two K/V tiles: no order to depend on)
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+# operands that a kernel would read or write out of range, or not at all from where they are: errors on the host, no launch
+@pytest.mark.parametrize("what", ["lengths on the host", "too few lengths", "key dtype", "out dtype", "out too small",
+                                  "strided out", "workspace on the host", "table on the host"])
+def test_decode_refuses_what_the_kernels_cannot_reach(what):
+    from acctransformer_b200 import ops
+    q, _, _, _ = _inputs(2, 4, 1, 64)
+    k, v, _, _ = _inputs(2, 4, 64, 64)
+    kw = {"seq_lens": torch.tensor([3, 64], dtype=torch.int32, device="cuda")}
+    if what == "lengths on the host":
+        kw["seq_lens"] = kw["seq_lens"].cpu()
+    elif what == "too few lengths":
+        kw["seq_lens"] = kw["seq_lens"][:1]
+    elif what == "key dtype":
+        k, v = k.to(torch.bfloat16), v.to(torch.bfloat16)
+    elif what == "out dtype":
+        kw["out"] = torch.empty_like(q, dtype=torch.uint8)
+    elif what == "out too small":
+        kw["out"] = torch.empty_like(q[:1])
+    elif what == "strided out":
+        kw["out"] = torch.empty(2, 4, 1, 128, device="cuda", dtype=q.dtype)[..., :64]
+    elif what == "workspace on the host":
+        kw["workspace"] = ops.DecodeWorkspace(2, 4, 64, "cpu")
+    else:
+        kw["block_table"] = torch.zeros(2, 1, dtype=torch.int32)
+    with pytest.raises(ValueError):
+        ops.infer_decode(q, k, v, **kw)
+
+
+def test_decode_takes_lengths_and_out_in_any_shape():
+    from acctransformer_b200 import ops
+    q, _, _, _ = _inputs(2, 4, 1, 64)
+    k, v, _, _ = _inputs(2, 4, 64, 64)
+    want = ops.infer_decode(q, k, v, torch.tensor([3, 64], dtype=torch.int32, device="cuda"))
+    out = torch.empty(2, 4, 64, device="cuda", dtype=q.dtype)
+    got = ops.infer_decode(q, k, v, torch.tensor([[3], [64], [5]], device="cuda"), out=out)
+    assert got is out or got.data_ptr() == out.data_ptr()
+    assert torch.equal(out.view_as(want), want)
+
+
+@pytest.mark.parametrize("what", ["lengths on the host", "too few lengths", "key dtype", "value on the host"])
+def test_prefill_refuses_what_the_kernels_cannot_reach(what):
+    from acctransformer_b200 import ops
+    q, k, v, _ = _inputs(2, 2, 130, 64)
+    lens = torch.tensor([130, 7], dtype=torch.int32, device="cuda")
+    if what == "lengths on the host":
+        lens = lens.cpu()
+    elif what == "too few lengths":
+        lens = lens[:1]
+    elif what == "key dtype":
+        k, v = k.to(torch.bfloat16), v.to(torch.bfloat16)
+    else:
+        v = v.cpu()
+    with pytest.raises(ValueError):
+        ops.infer_prefill(q, k, v, seq_lens=lens)
+
+
+@pytest.mark.parametrize("what", ["key", "mask", "alibi", "dropout mask"])
+def test_training_refuses_what_the_kernels_cannot_reach(what):
+    from acctransformer_b200.flash_attention.ops.flash_attention.flash_attention_impl import get_flash_attention
+    q, k, v, _ = _inputs(1, 2, 130, 64)
+    kw = {}
+    if what == "key":
+        k = k.cpu()
+    elif what == "mask":
+        kw["attn_mask"] = torch.zeros(1, 130, 130, dtype=q.dtype)
+    elif what == "alibi":
+        kw["alibi_mask"] = torch.zeros(1, 2, 1, 130, dtype=q.dtype)
+    else:
+        kw["dropout_mask"] = torch.ones(1, 2, 130, 130, dtype=torch.uint8)
+    with pytest.raises(ValueError):
+        get_flash_attention()(q, k, v, **kw)
