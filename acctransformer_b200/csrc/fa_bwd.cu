@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
 
   // the mask plan, where the operands of this call allow it (every role comes to the same answer)
   bool planned = false;
-  if constexpr (MASKED) if (mods.plan.head != nullptr)
+  if constexpr (MASKED && DROP < 2) if (mods.plan.head != nullptr)     // (a dropout tensor excludes a plan)
     planned = plan_holds(mods.plan.head, p.scale) && __uint_as_float(p.plan_stats[0]) < kPlanMaxNorm2 &&
               __uint_as_float(p.plan_stats[1]) < kPlanMaxNorm2;
 
@@ -667,9 +667,11 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
       if (n % max(n_per, 1) == 0) bias = n == 0 ? bias_first : bias_of(head_of(n));   // first tile of a query head
       mask_class = mask_class_next;
       if (tile_class != nullptr && n + 1 < n_iter) mask_class_next = tile_class[static_cast<int64_t>(tile_of(n + 1)) * tiles_k];
-      // class 3 (mask plan): a bit per position, set = masked; this key's bits for the half's 64 queries
+      // class 3 of a plan: a bit per position, set = masked; this key's bits for the half's 64 queries (a caller's byte that
+      // is neither 0 nor 2 says "read the tile")
+      const bool bits = MASKED && planned && mask_class == 3;
       uint2 key_bits = make_uint2(0u, 0u);
-      if constexpr (MASKED) if (mask_class == 3)
+      if constexpr (MASKED) if (bits)
         key_bits = *reinterpret_cast<const uint2*>(
             mods.plan.bits + (tile_class + static_cast<int64_t>(i) * tiles_k - mods.plan.cls) * kPlanBitWords + kTile * 4 + r * 4 + hf * 2);
       // ---- P part: needs S^T only
@@ -697,7 +699,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
       // A mask tile that is all 0 is not read; one that is all 1 adds one constant to every score of the tile,
       // which joins the key row's bias; any other tile is read.
       const bool mask_const = MASKED && mods.mask_kind == 1 && mask_class == 2;
-      const bool use_mask = MASKED && ((mods.mask_kind == 1 && mask_class == 1) || (mods.mask_kind == 2 && i == j));
+      const bool use_mask = MASKED && ((mods.mask_kind == 1 && mask_class != 0 && !mask_const && !bits) || (mods.mask_kind == 2 && i == j));
       const float tile_bias = mask_const ? bias - 10000.0f * kLog2e : bias;
       const bool diag = mods.causal && (q_base < j * kTile + kTile - 1);
       // TriangleAttention row groups: the rows of this Q tile see keys below the end of their group; the smallest
@@ -729,7 +731,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_kernel(const __grid_con
             u8_keep_load(mods.drop, static_cast<int64_t>(bh) * p.S_q, q_base + c * 32, p.S_q - 1, p.S_k, kv_idx - lane, lane, raw8);
           if (diag) p_fast<true>(s[cc], lse2 + c * 32, p.scale_log2, tile_bias, kv_idx, q_base + c * 32, pr[cc]);
           else p_fast<false>(s[cc], lse2 + c * 32, p.scale_log2, tile_bias, kv_idx, q_base + c * 32, pr[cc]);
-          if constexpr (MASKED) if (mask_class == 3) {
+          if constexpr (MASKED) if (bits) {
             const uint32_t word = cc == 0 ? key_bits.x : key_bits.y;
 #pragma unroll
             for (int e = 0; e < 32; ++e) pr[cc][e] = ((word >> e) & 1u) ? 0.f : pr[cc][e];

@@ -486,6 +486,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) fa_fwd_kernel(const __grid_con
     for (int j = rng.lo; j <= rng.hi; j = j_next, ++n) {
       j_next = next_tile(qt, rng, j);
       mask_class = mask_class_next;
+      // (a caller's byte that is neither 0 nor 2 says "read the tile"; 3 means something in a plan's classes only)
+      if constexpr ((MODS & 1) != 0) if (!planned && mask_class != 0 && mask_class != 2) mask_class = 1;
       if (tile_class != nullptr && j < rng.hi) mask_class_next = tile_class[j_next];
       if constexpr ((MODS & 2) != 0) if (mods.alibi != nullptr) {
         al_raw = al_raw_next;

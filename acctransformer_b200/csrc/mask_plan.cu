@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(kPlanThreads) mask_bits_kernel(const void* mas
   const int64_t row_of_tiles = static_cast<int64_t>(mb) * gridDim.y + i, tile = row_of_tiles * gridDim.x + j;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int c = tiles[tile];
-  if (c != 1) {
+  if (c == 0 || c == 2) {                            // (any other byte: the tile is read)
     if (tid == 0) plan.cls[tile] = static_cast<uint8_t>(c);
     if (c == 0 && tid < 4) atomicOr(&plan.seen[row_of_tiles * 4 + tid], 0xffffffffu);
     return;
