@@ -73,18 +73,27 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiledFn g_encode = nullptr;
 
+using CtxGetCurrentFn = CUresult (*)(CUcontext*);
+CtxGetCurrentFn find_ctx_current() {
+  void* fn = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &fn, cudaEnableDefault, &q) != cudaSuccess) return nullptr;
+  return reinterpret_cast<CtxGetCurrentFn>(fn);
+}
+
 int init_device(PerDevice** out) {
   int dev = -1;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return fail(ACCT_ERR_NO_DEVICE, "no CUDA device: %s", cudaGetErrorString(e));
   if (dev < 0 || dev >= kMaxDevices) return fail(ACCT_ERR_NO_DEVICE, "device index %d out of range", dev);
   // A thread that has made no runtime call yet (an autograd engine's worker) has no context bound, and the driver call
-  // that encodes tensor maps needs one: bind the device's primary context once per thread and device.
-  static thread_local int t_bound = -1;
-  if (t_bound != dev) {
+  // that encodes tensor maps needs one: bind the device's primary context.  A context that is current stays so: it may be
+  // one of the caller's own, and the operands then live in it.
+  static const CtxGetCurrentFn ctx_current = find_ctx_current();
+  CUcontext ctx = nullptr;
+  if (ctx_current != nullptr && (ctx_current(&ctx) != CUDA_SUCCESS || ctx == nullptr)) {
     e = cudaSetDevice(dev);
     if (e != cudaSuccess) return fail(ACCT_ERR_NO_DEVICE, "cudaSetDevice(%d): %s", dev, cudaGetErrorString(e));
-    t_bound = dev;
   }
   PerDevice& d = g_dev[dev];
   if (d.ready.load(std::memory_order_acquire) && d.rc == 0) {

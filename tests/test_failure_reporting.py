@@ -47,3 +47,28 @@ def test_wait_that_runs_out_is_reported_once_and_the_next_call_is_clean():
     assert float(np.max(np.abs(o.float().cpu().numpy() - o_ref))) <= 2e-3
     for got, want in zip((dq, dk, dv), ref.sa_grad(q.numpy(), k.numpy(), v.numpy(), do.numpy(), causal=True, scale=scale)):
         assert float(np.max(np.abs(got.float().cpu().numpy() - want)) / np.max(np.abs(want))) <= 1e-2
+
+
+_OWN_CONTEXT = """
+import ctypes as C, sys
+cu = C.CDLL("libcuda.so.1")
+lib = C.CDLL(sys.argv[1])
+assert cu.cuInit(0) == 0
+mine, now = C.c_void_p(), C.c_void_p()
+assert cu.cuCtxCreate_v2(C.byref(mine), 0, 0) == 0
+rc = lib.acct_device_status(None)
+assert cu.cuCtxGetCurrent(C.byref(now)) == 0
+print(rc, now.value == mine.value)
+"""
+
+
+def test_context_of_the_caller_stays_current():
+    """Operands made in a driver context of the caller's own are only valid while that context is current."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import subprocess
+    import sys
+
+    from acctransformer_b200 import _lib
+    r = subprocess.run([sys.executable, "-c", _OWN_CONTEXT, _lib.LIB_PATH], capture_output=True, text=True, timeout=120)
+    assert r.stdout.split() == ["0", "True"], r.stderr
