@@ -23,6 +23,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
+#include <torch/csrc/utils/object_ptr.h>
 
 #include "../../include/acct_b200.h"
 
@@ -137,8 +138,8 @@ void fill_args(acct_fa_args& a, const Tensor& q, const Tensor& k, const Tensor& 
     a.dropout_dtype = dtype_code(drop.scalar_type(), "dropout_mask");
   }
   if (alibi.defined()) a.alibi = alibi.const_data_ptr();
-  a.prev_block_num = static_cast<int32_t>(std::min<int64_t>(c.prev, ACCT_BAND_UNBOUNDED));
-  a.next_block_num = static_cast<int32_t>(std::min<int64_t>(c.next, ACCT_BAND_UNBOUNDED));
+  a.prev_block_num = static_cast<int32_t>(c.prev);
+  a.next_block_num = static_cast<int32_t>(c.next);
   a.scale = static_cast<float>(c.scale);
   if (c.has_seed) {
     a.flags |= ACCT_FLAG_DROPOUT_PHILOX;
@@ -269,10 +270,28 @@ int64_t int_arg(PyObject* p) {
   if (v == -1 && PyErr_Occurred()) throw python_error();
   return v;
 }
-double float_arg(PyObject* p) {
-  const double v = PyFloat_AsDouble(p);
-  if (v == -1.0 && PyErr_Occurred()) throw python_error();
+// what int() and float() take, for the arguments that the Python front end passes through them
+THPObjectPtr as_int(PyObject* p) {
+  THPObjectPtr v(PyNumber_Long(p));
+  if (!v) throw python_error();
   return v;
+}
+uint64_t low_bits_arg(PyObject* p) {
+  const uint64_t v = PyLong_AsUnsignedLongLongMask(as_int(p).get());
+  if (PyErr_Occurred()) throw python_error();
+  return v;
+}
+int64_t block_count_arg(PyObject* p) {      // anything below 0 is refused by the library, anything large means unbounded
+  int overflow = 0;
+  const long long v = PyLong_AsLongLongAndOverflow(as_int(p).get(), &overflow);
+  if (v == -1 && overflow == 0 && PyErr_Occurred()) throw python_error();
+  if (overflow != 0) return overflow > 0 ? ACCT_BAND_UNBOUNDED : -1;
+  return std::max<long long>(-1, std::min<long long>(v, ACCT_BAND_UNBOUNDED));
+}
+double float_arg(PyObject* p) {
+  THPObjectPtr v(PyNumber_Float(p));
+  if (!v) throw python_error();
+  return PyFloat_AS_DOUBLE(v.get());
 }
 bool bool_arg(PyObject* p) {
   const int v = PyObject_IsTrue(p);
@@ -315,16 +334,15 @@ PyObject* py_fa_apply(PyObject*, PyObject* const* args, Py_ssize_t n) {
   c.mask_tile128 = bool_arg(args[7]);
   c.causal = bool_arg(args[8]);
   c.keep_prob = float_arg(args[9]);
-  c.prev = int_arg(args[10]);
-  c.next = int_arg(args[11]);
+  c.prev = block_count_arg(args[10]);
+  c.next = block_count_arg(args[11]);
   c.scale = float_arg(args[12]);
-  c.tri_block = int_arg(args[13]);
+  c.tri_block = static_cast<int32_t>(low_bits_arg(args[13]));
   c.deterministic = bool_arg(args[14]);
   if (args[15] != Py_None) {
     c.has_seed = true;
-    c.seed = PyLong_AsUnsignedLongLongMask(args[15]);
-    c.offset = PyLong_AsUnsignedLongLongMask(args[16]);
-    if (PyErr_Occurred()) throw python_error();
+    c.seed = low_bits_arg(args[15]);
+    c.offset = low_bits_arg(args[16]);
   }
   Tensor o, lse, plan;
   // as a Python autograd Function without a `jvp` does; a tangent would be dropped silently otherwise

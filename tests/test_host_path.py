@@ -152,3 +152,19 @@ def test_training_refuses_what_the_kernels_cannot_reach(what):
         kw["dropout_mask"] = torch.ones(1, 2, 130, 130, dtype=torch.uint8)
     with pytest.raises(ValueError):
         get_flash_attention()(q, k, v, **kw)
+
+
+def test_numbers_in_any_form_that_int_and_float_take():
+    from acctransformer_b200 import TriangleAttention
+    from acctransformer_b200.flash_attention.ops.flash_attention.flash_attention_impl import get_flash_attention
+    q, k, v, _ = _inputs(1, 2, 300, 64)
+    assert torch.equal(_layer(64, prev_block_num=1.0, next_block_num=0.0)(q, k, v), _layer(64, prev_block_num=1, next_block_num=0)(q, k, v))
+    assert torch.equal(_layer(64, prev_block_num=10 ** 30)(q, k, v), _layer(64)(q, k, v))
+    with pytest.raises(Exception, match="prev/next_block_num must be >= 0"):
+        _layer(64, prev_block_num=-1)(q, k, v)
+    mask = _documents(300)
+    assert torch.equal(TriangleAttention(block_size=128.0)(q, k, v, mask), TriangleAttention(block_size=128)(q, k, v, mask))
+    fa = get_flash_attention(scale="0.125")
+    want = get_flash_attention(scale=0.125)(q, k, v, keep_prob=0.75, dropout_seed=7, dropout_offset=2)[0]
+    assert torch.equal(fa(q, k, v, keep_prob="0.75", dropout_seed=7.0, dropout_offset=torch.tensor(2.0))[0], want)
+    assert torch.equal(fa(q, k, v, keep_prob=0.75, dropout_seed=7 + 2 ** 64, dropout_offset=2)[0], want)
