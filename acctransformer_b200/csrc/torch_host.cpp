@@ -212,12 +212,12 @@ struct FaBackward : public torch::autograd::Node {
     TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
     variable_list out(6);
     Tensor d_o = grads[0];
-    if (!d_o.defined()) return out;
     const Tensor q = q_.unpack(), k = k_.unpack(), v = v_.unpack(), o = o_.unpack(shared_from_this()), lse = lse_.unpack();
     const Tensor mask = mask_.unpack(), drop = drop_.unpack(), alibi = alibi_.unpack(), tiles = tiles_.unpack(),
                  plan = plan_.unpack();
     at::AutoDispatchBelowADInplaceOrView below;
     c10::cuda::OptionalCUDAGuard guard(q.device());
+    if (!d_o.defined()) d_o = at::zeros_like(o);       // (a function behind this one that hands back no gradient)
     int64_t ds[3] = {d_o.stride(0), d_o.stride(1), d_o.stride(2)};
     bool as_is = d_o.stride(3) == 1 && reinterpret_cast<uintptr_t>(d_o.const_data_ptr()) % 16 == 0 && ds[2] >= q.size(3);
     for (int i = 0; i < 3; ++i) as_is = as_is && ds[i] > 0 && ds[i] % 8 == 0;

@@ -168,3 +168,20 @@ def test_numbers_in_any_form_that_int_and_float_take():
     want = get_flash_attention(scale=0.125)(q, k, v, keep_prob=0.75, dropout_seed=7, dropout_offset=2)[0]
     assert torch.equal(fa(q, k, v, keep_prob="0.75", dropout_seed=7.0, dropout_offset=torch.tensor(2.0))[0], want)
     assert torch.equal(fa(q, k, v, keep_prob=0.75, dropout_seed=7 + 2 ** 64, dropout_offset=2)[0], want)
+
+
+class _NoGradient(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x):
+        return x.clone()
+
+    @staticmethod
+    def backward(ctx, g):
+        return None
+
+
+def test_output_gradient_that_is_not_there_counts_as_zero():
+    q, k, v, d_o = _inputs(1, 2, 130, 64)
+    xs = [t.requires_grad_() for t in (q, k, v)]
+    for g in torch.autograd.grad(_NoGradient.apply(_layer(64)(*xs)), xs, d_o):
+        assert g.shape == q.shape and not g.any()
