@@ -198,12 +198,26 @@ void check_fa_inputs(const Tensor& q, const Tensor& k, const Tensor& v, Tensor& 
   }
 }
 
+// A [B, N, S, D] operand that the kernels read in its own layout where they can (head_dim contiguous, address and the other
+// strides multiples of 16 bytes), else a packed copy; `strides` = those of B, N, S.  (The stride of a dimension of size 1
+// may be anything, also in a tensor that counts as contiguous: those of the packed form are computed.)
+Tensor readable(const Tensor& t, int64_t (&strides)[3]) {
+  bool as_is = t.stride(3) == 1 && reinterpret_cast<uintptr_t>(t.const_data_ptr()) % 16 == 0 && t.stride(2) >= t.size(3);
+  for (int i = 0; i < 3; ++i) {
+    strides[i] = t.stride(i);
+    as_is = as_is && strides[i] > 0 && strides[i] % 8 == 0;
+  }
+  if (as_is) return t;
+  for (int i = 2; i >= 0; --i) strides[i] = i == 2 ? t.size(3) : strides[i + 1] * t.size(i + 1);
+  return t.contiguous();
+}
+
 // The gradient of the training operator: dq, dk, dv in the inputs' type (what the reference's bprop hands back after
-// its cast, flash_attention_impl.py:117-124).  The output gradient is read in the layout it arrives in where the
-// kernels can (head_dim contiguous, strides and address multiples of 16 bytes): behind a transpose back to
-// [B, S, N*D] it is a strided view, and copying it would be one more pass over memory.
+// its cast, flash_attention_impl.py:117-124).  The output gradient is read in the layout it arrives in: behind a transpose
+// back to [B, S, N*D] it is a strided view, and copying it would be one more pass over memory.
 struct FaBackward : public torch::autograd::Node {
-  SavedVariable q_, k_, v_, o_, lse_, mask_, drop_, alibi_, tiles_, plan_;
+  SavedVariable q_, k_, v_, o_, lse_, mask_, drop_, alibi_;
+  Tensor tiles_, plan_;             // this library's own, for the mask that is saved: no user sees or changes them
   FaConfig cfg;
   bool released = false;
 
@@ -212,21 +226,24 @@ struct FaBackward : public torch::autograd::Node {
     TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
     variable_list out(6);
     Tensor d_o = grads[0];
-    const Tensor q = q_.unpack(), k = k_.unpack(), v = v_.unpack(), o = o_.unpack(shared_from_this()), lse = lse_.unpack();
-    const Tensor mask = mask_.unpack(), drop = drop_.unpack(), alibi = alibi_.unpack(), tiles = tiles_.unpack(),
-                 plan = plan_.unpack();
+    const Tensor q = q_.unpack(), k = k_.unpack(), v = v_.unpack();
+    Tensor o = o_.unpack(shared_from_this()), lse = lse_.unpack(), mask = mask_.unpack(), drop = drop_.unpack(), alibi = alibi_.unpack();
     at::AutoDispatchBelowADInplaceOrView below;
+    // saved-tensor hooks may have handed back tensors of another layout, or of another device: checked like the inputs
+    check_fa_inputs(q, k, v, mask, drop, alibi, tiles_, cfg);
+    require_on("o", o, q);
+    require_on("lse", lse, q);
+    HOST_CHECK(o.sizes() == q.sizes() && o.scalar_type() == q.scalar_type(), "o must have the shape and dtype of q");
+    HOST_CHECK(lse.sizes() == q.sizes().slice(0, 3) && lse.scalar_type() == at::kFloat, "lse must be float32 [B, N, S_q]");
+    lse = lse.contiguous();
     c10::cuda::OptionalCUDAGuard guard(q.device());
-    if (!d_o.defined()) d_o = at::zeros_like(o);       // (a function behind this one that hands back no gradient)
-    int64_t ds[3] = {d_o.stride(0), d_o.stride(1), d_o.stride(2)};
-    bool as_is = d_o.stride(3) == 1 && reinterpret_cast<uintptr_t>(d_o.const_data_ptr()) % 16 == 0 && ds[2] >= q.size(3);
-    for (int i = 0; i < 3; ++i) as_is = as_is && ds[i] > 0 && ds[i] % 8 == 0;
-    if (!as_is) {
-      d_o = d_o.contiguous();
-      ds[0] = ds[1] = ds[2] = 0;      // packed (the stride of a dimension of size 1 may be anything: not read)
-    }
+    if (!d_o.defined()) d_o = at::zeros_like(q);       // (a function behind this one that hands back no gradient)
+    int64_t o_strides[3], d_o_strides[3];
+    o = readable(o, o_strides);
+    d_o = readable(d_o, d_o_strides);
     acct_fa_args a;
-    fill_args(a, q, k, v, o, lse, mask, drop, alibi, tiles, cfg);
+    fill_args(a, q, k, v, o, lse, mask, drop, alibi, tiles_, cfg);
+    std::copy(o_strides, o_strides + 3, a.o_stride);
     if (cfg.deterministic) a.flags |= ACCT_FLAG_DETERMINISTIC;
     const auto dt = q.scalar_type();
     Tensor dq = empty_like_shape(q.sizes(), dt, q), dk = empty_like_shape(k.sizes(), dt, q), dv = empty_like_shape(v.sizes(), dt, q);
@@ -238,8 +255,8 @@ struct FaBackward : public torch::autograd::Node {
     g.d_o = d_o.const_data_ptr();
     g.dq = dq.data_ptr(); g.dk = dk.data_ptr(); g.dv = dv.data_ptr();
     g.workspace = ws.data_ptr(); g.workspace_bytes = nbytes;
-    check(g_lib.fa_bwd(&a, &g, ds, plan.defined() ? plan.const_data_ptr() : nullptr, static_cast<uint8_t*>(ws.data_ptr()) + own,
-                       stream_of(q)));
+    check(g_lib.fa_bwd(&a, &g, d_o_strides, plan_.defined() ? plan_.const_data_ptr() : nullptr,
+                       static_cast<uint8_t*>(ws.data_ptr()) + own, stream_of(q)));
     out[0] = std::move(dq); out[1] = std::move(dk); out[2] = std::move(dv);
     return out;
   }
@@ -247,7 +264,9 @@ struct FaBackward : public torch::autograd::Node {
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
     released = true;
-    for (SavedVariable* s : {&q_, &k_, &v_, &o_, &lse_, &mask_, &drop_, &alibi_, &tiles_, &plan_}) s->reset_data();
+    for (SavedVariable* s : {&q_, &k_, &v_, &o_, &lse_, &mask_, &drop_, &alibi_}) s->reset_data();
+    tiles_.reset();
+    plan_.reset();
   }
 
   std::string name() const override { return "FlashAttentionBackward"; }
@@ -378,8 +397,8 @@ PyObject* py_fa_apply(PyObject*, PyObject* const* args, Py_ssize_t n) {
       node->mask_ = SavedVariable(mask, false);
       node->drop_ = SavedVariable(drop, false);
       node->alibi_ = SavedVariable(alibi, false);
-      node->tiles_ = SavedVariable(tiles, false);
-      node->plan_ = SavedVariable(plan, false);
+      node->tiles_ = tiles;
+      node->plan_ = plan;
       torch::autograd::set_history(o, node);
       node->o_ = SavedVariable(o, true);
       node->lse_ = SavedVariable(lse, false);

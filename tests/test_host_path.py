@@ -185,3 +185,44 @@ def test_output_gradient_that_is_not_there_counts_as_zero():
     xs = [t.requires_grad_() for t in (q, k, v)]
     for g in torch.autograd.grad(_NoGradient.apply(_layer(64)(*xs)), xs, d_o):
         assert g.shape == q.shape and not g.any()
+
+
+# saved-tensor hooks that hand back the same values in another layout: rows of 128 elements of which 64 count, every second
+# element of a score-shaped tensor, an output that is aligned to nothing, and tensors that were on the host meanwhile
+@pytest.mark.parametrize("form", ["padded rows", "every second element", "misaligned output", "offloaded"])
+def test_saved_tensors_in_any_layout(form):
+    q, k, v, d_o = _inputs(2, 2, 200, 64)
+    mask = _documents(200)
+    want = _grads(_layer(64), (q, k, v), d_o, mask)
+    o_shape = q.shape
+
+    def unpack_misaligned(t):
+        if t.dim() != 4 or t.requires_grad or t.shape != o_shape:
+            return t
+        r = t.new_empty(t.shape[:3] + (t.shape[3] + 1,))[..., 1:]
+        return r.copy_(t)
+    pack, unpack = {
+        "padded rows": (lambda t: torch.cat([t, torch.zeros_like(t)], -1) if t.dim() == 4 else t,
+                        lambda t: t[..., :64] if t.dim() == 4 else t),
+        "every second element": (lambda t: torch.stack([t, torch.zeros_like(t)], -1) if t.dim() == 3 else t,
+                                 lambda t: t[..., 0] if t.shape[-1] == 2 else t),
+        "misaligned output": (lambda t: t, unpack_misaligned),
+        "offloaded": (lambda t: t.cpu(), lambda t: t.cuda()),
+    }[form]
+    xs = [t.detach().requires_grad_() for t in (q, k, v)]
+    with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+        out = _layer(64)(*xs, mask)
+    for a, b in zip(torch.autograd.grad(out, xs, d_o), want):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("which", ["q", "o", "lse", "mask"])
+def test_saved_tensors_left_on_the_host_are_refused(which):
+    q, k, v, d_o = _inputs(1, 2, 130, 64)
+    shape = {"q": (1, 2, 130, 64), "o": (1, 2, 130, 64), "lse": (1, 2, 130), "mask": (1, 130, 130)}[which]
+    xs = [t.detach().requires_grad_() for t in (q, k, v)]
+    mine = (lambda t: t.requires_grad and t.is_leaf) if which == "q" else (lambda t: not (t.requires_grad and t.is_leaf))
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: (t.shape == shape and mine(t), t), lambda p: p[1].cpu() if p[0] else p[1]):
+        out = _layer(64)(*xs, _documents(130))
+    with pytest.raises((ValueError, RuntimeError), match="CUDA tensor|device"):
+        torch.autograd.grad(out, xs, d_o)
