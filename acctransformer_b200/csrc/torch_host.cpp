@@ -368,7 +368,7 @@ PyObject* py_fa_apply(PyObject*, PyObject* const* args, Py_ssize_t n) {
   for (const Tensor* t : {&q, &k, &v, &std::as_const(mask), &std::as_const(drop), &std::as_const(alibi)})
     TORCH_CHECK_NOT_IMPLEMENTED(!t->defined() || !t->_fw_grad(/*level=*/0).defined(),
                                 "the flash attention operator does not support forward mode AD");
-  const variable_list inputs = {q, k, v, mask, drop, alibi};
+  const variable_list inputs = {q, k, v, mask, drop, alibi};      // (as given: below, the last three become packed)
   {
     pybind11::gil_scoped_release no_gil;
     {
@@ -394,9 +394,9 @@ PyObject* py_fa_apply(PyObject*, PyObject* const* args, Py_ssize_t n) {
       node->q_ = SavedVariable(q, false);
       node->k_ = SavedVariable(k, false);
       node->v_ = SavedVariable(v, false);
-      node->mask_ = SavedVariable(mask, false);
-      node->drop_ = SavedVariable(drop, false);
-      node->alibi_ = SavedVariable(alibi, false);
+      node->mask_ = SavedVariable(inputs[3], false);
+      node->drop_ = SavedVariable(inputs[4], false);
+      node->alibi_ = SavedVariable(inputs[5], false);
       node->tiles_ = tiles;
       node->plan_ = plan;
       torch::autograd::set_history(o, node);

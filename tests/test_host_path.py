@@ -226,3 +226,23 @@ def test_saved_tensors_left_on_the_host_are_refused(which):
         out = _layer(64)(*xs, _documents(130))
     with pytest.raises((ValueError, RuntimeError), match="CUDA tensor|device"):
         torch.autograd.grad(out, xs, d_o)
+
+
+# a mask that is a view is saved itself, not as the packed copy that the kernels read: it counts as memory of its owner,
+# and a change between forward and backward is noticed
+@pytest.mark.parametrize("packed", [True, False])
+def test_mask_changed_before_the_backward_is_refused(packed):
+    q, k, v, d_o = _inputs(1, 2, 200, 64)
+    owner = _documents(256)
+    mask = owner[:, :200, :200]
+    if packed:
+        mask = mask.contiguous()
+    xs = [t.detach().requires_grad_() for t in (q, k, v)]
+    saved = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: saved.append(t.data_ptr()) or t, lambda t: t):
+        _layer(64)(*xs, mask)
+    assert mask.data_ptr() in saved
+    out = _layer(64)(*xs, mask)
+    mask.zero_()
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        torch.autograd.grad(out, xs, d_o)
