@@ -1,6 +1,6 @@
 // The host path of the Python layers in native code: takes torch tensors, checks them, fills the C ABI's argument
 // blocks and launches, without a Python frame, a ctypes structure or a context manager per call, and carries the
-// autograd node of the training operator.
+// custom function of the training operator.
 //
 // Built as the CPython module `_torch_host` next to libacct_b200.so, whose entry points it looks up at load time
 // (`init`), so it adds no second copy of any kernel.  What bounds the small calls is this path: one forward + backward
@@ -9,8 +9,8 @@
 //
 // Error conditions and texts are those of the Python front end (ops.py); a non-zero status of the library becomes its
 // AcctError.  The reference registers its operators with the framework in Python
-// (train/acctransformer/flash_attention/ops/flash_attention/flash_attention_impl.py:96-154); the autograd node here
-// stands for the `bprop` there.
+// (train/acctransformer/flash_attention/ops/flash_attention/flash_attention_impl.py:96-154); its custom
+// function stands for the `bprop` there.
 #include <dlfcn.h>
 
 #include <ATen/ATen.h>
@@ -18,11 +18,8 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
-#include <torch/csrc/autograd/function.h>
-#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
-#include <torch/csrc/autograd/saved_variable.h>
-#include <torch/csrc/autograd/variable.h>
 #include <torch/csrc/utils/object_ptr.h>
 
 #include "../../include/acct_b200.h"
@@ -30,7 +27,7 @@
 namespace {
 
 using at::Tensor;
-using torch::autograd::SavedVariable;
+using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
 struct Library {
@@ -102,11 +99,24 @@ void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.devi
 
 // What a call carries besides tensors.
 struct FaConfig {
-  bool mask_tile128 = false, causal = false, deterministic = false, has_seed = false;
+  int64_t mask_tile128 = 0, causal = 0, deterministic = 0, has_seed = 0;      // (flags; no padding, see pack())
   double keep_prob = 1.0, scale = 1.0;
   int64_t prev = ACCT_BAND_UNBOUNDED, next = ACCT_BAND_UNBOUNDED, tri_block = 0;
   uint64_t seed = 0, offset = 0;
+
+  // in the form that a custom function may keep
+  std::vector<int64_t> pack() const {
+    std::vector<int64_t> out(sizeof(FaConfig) / 8);
+    memcpy(out.data(), this, sizeof(FaConfig));
+    return out;
+  }
+  static FaConfig unpack(const std::vector<int64_t>& from) {
+    FaConfig c;
+    memcpy(&c, from.data(), sizeof(FaConfig));
+    return c;
+  }
 };
+static_assert(std::is_trivially_copyable_v<FaConfig> && sizeof(FaConfig) == 11 * 8);
 
 // Fills `a` from the tensors (check_fa_inputs has seen to their shapes, and to contiguity where the ABI wants it).
 void fill_args(acct_fa_args& a, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse,
@@ -215,34 +225,68 @@ Tensor readable(const Tensor& t, int64_t (&strides)[3]) {
 // The gradient of the training operator: dq, dk, dv in the inputs' type (what the reference's bprop hands back after
 // its cast, flash_attention_impl.py:117-124).  The output gradient is read in the layout it arrives in: behind a transpose
 // back to [B, S, N*D] it is a strided view, and copying it would be one more pass over memory.
-struct FaBackward : public torch::autograd::Node {
-  SavedVariable q_, k_, v_, o_, lse_, mask_, drop_, alibi_;
-  Tensor tiles_, plan_;             // this library's own, for the mask that is saved: no user sees or changes them
+//
+// The forward and this are one custom function of torch's C++ interface, so that what autograd offers around a function --
+// saved-tensor hooks, compiled autograd, gradients that are not there -- works as around a Python one.
+struct FaCall {
   FaConfig cfg;
-  bool released = false;
+  Tensor tiles;          // of the mask: this library's own, like the plan; no user sees or changes them
+  Tensor* lse;           // (not an output of the function: it has no gradient, and its saved form is not an output's)
+};
 
-  variable_list apply(variable_list&& grads) override {
-    std::lock_guard<std::mutex> lock(mutex_);
-    TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
-    variable_list out(6);
-    Tensor d_o = grads[0];
-    const Tensor q = q_.unpack(), k = k_.unpack(), v = v_.unpack();
-    Tensor o = o_.unpack(shared_from_this()), lse = lse_.unpack(), mask = mask_.unpack(), drop = drop_.unpack(), alibi = alibi_.unpack();
+struct FaFunction : public torch::autograd::Function<FaFunction> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const std::optional<Tensor>& mask_in,
+                        const std::optional<Tensor>& drop_in, const std::optional<Tensor>& alibi_in, const FaCall& call) {
+    const FaConfig& c = call.cfg;
+    Tensor mask = mask_in.value_or(Tensor()), drop = drop_in.value_or(Tensor()), alibi = alibi_in.value_or(Tensor());
+    Tensor o, lse, plan;
+    at::AutoDispatchBelowADInplaceOrView below;
+    check_fa_inputs(q, k, v, mask, drop, alibi, call.tiles, c);     // (packs the last three)
+    c10::cuda::OptionalCUDAGuard guard(q.device());
+    o = empty_like_shape(q.sizes(), q.scalar_type(), q);
+    lse = empty_like_shape(q.sizes().slice(0, 3), at::kFloat, q);
+    acct_fa_args a;
+    fill_args(a, q, k, v, o, lse, mask, drop, alibi, call.tiles, c);
+    const size_t plan_bytes = g_lib.mask_plan_bytes(&a);
+    if (plan_bytes > 0) {
+      plan = empty_like_shape({static_cast<int64_t>(plan_bytes)}, at::kByte, q);
+      check(g_lib.mask_plan(&a, plan.data_ptr(), stream_of(q)));
+    }
+    check(g_lib.fa_fwd(&a, plan.defined() ? plan.const_data_ptr() : nullptr, stream_of(q)));
+    *call.lse = lse;
+    // (the optional inputs as given, not their packed copies)
+    ctx->save_for_backward({q, k, v, o, lse, mask_in.value_or(Tensor()), drop_in.value_or(Tensor()), alibi_in.value_or(Tensor())});
+    ctx->saved_data["config"] = c.pack();
+    if (call.tiles.defined()) ctx->saved_data["tiles"] = call.tiles;
+    if (plan.defined()) ctx->saved_data["plan"] = plan;
+    return o;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list saved = ctx->get_saved_variables();
+    const Tensor &q = saved[0], &k = saved[1], &v = saved[2];
+    Tensor o = saved[3], lse = saved[4], mask = saved[5], drop = saved[6], alibi = saved[7], d_o = grads[0];
+    const auto tensor_of = [ctx](const char* key) {
+      const auto it = ctx->saved_data.find(key);
+      return it == ctx->saved_data.end() ? Tensor() : it->second.toTensor();
+    };
+    const Tensor tiles = tensor_of("tiles"), plan = tensor_of("plan");
+    const FaConfig cfg = FaConfig::unpack(ctx->saved_data.at("config").toIntVector());
+
     at::AutoDispatchBelowADInplaceOrView below;
     // saved-tensor hooks may have handed back tensors of another layout, or of another device: checked like the inputs
-    check_fa_inputs(q, k, v, mask, drop, alibi, tiles_, cfg);
+    check_fa_inputs(q, k, v, mask, drop, alibi, tiles, cfg);
     require_on("o", o, q);
     require_on("lse", lse, q);
     HOST_CHECK(o.sizes() == q.sizes() && o.scalar_type() == q.scalar_type(), "o must have the shape and dtype of q");
     HOST_CHECK(lse.sizes() == q.sizes().slice(0, 3) && lse.scalar_type() == at::kFloat, "lse must be float32 [B, N, S_q]");
     lse = lse.contiguous();
     c10::cuda::OptionalCUDAGuard guard(q.device());
-    if (!d_o.defined()) d_o = at::zeros_like(q);       // (a function behind this one that hands back no gradient)
     int64_t o_strides[3], d_o_strides[3];
     o = readable(o, o_strides);
     d_o = readable(d_o, d_o_strides);
     acct_fa_args a;
-    fill_args(a, q, k, v, o, lse, mask, drop, alibi, tiles_, cfg);
+    fill_args(a, q, k, v, o, lse, mask, drop, alibi, tiles, cfg);
     std::copy(o_strides, o_strides + 3, a.o_stride);
     if (cfg.deterministic) a.flags |= ACCT_FLAG_DETERMINISTIC;
     const auto dt = q.scalar_type();
@@ -255,21 +299,10 @@ struct FaBackward : public torch::autograd::Node {
     g.d_o = d_o.const_data_ptr();
     g.dq = dq.data_ptr(); g.dk = dk.data_ptr(); g.dv = dv.data_ptr();
     g.workspace = ws.data_ptr(); g.workspace_bytes = nbytes;
-    check(g_lib.fa_bwd(&a, &g, d_o_strides, plan_.defined() ? plan_.const_data_ptr() : nullptr,
+    check(g_lib.fa_bwd(&a, &g, d_o_strides, plan.defined() ? plan.const_data_ptr() : nullptr,
                        static_cast<uint8_t*>(ws.data_ptr()) + own, stream_of(q)));
-    out[0] = std::move(dq); out[1] = std::move(dk); out[2] = std::move(dv);
-    return out;
+    return {dq, dk, dv, Tensor(), Tensor(), Tensor(), Tensor()};
   }
-
-  void release_variables() override {
-    std::lock_guard<std::mutex> lock(mutex_);
-    released = true;
-    for (SavedVariable* s : {&q_, &k_, &v_, &o_, &lse_, &mask_, &drop_, &alibi_}) s->reset_data();
-    tiles_.reset();
-    plan_.reset();
-  }
-
-  std::string name() const override { return "FlashAttentionBackward"; }
 };
 
 // ---------------------------------------------------------------------------------------------
@@ -347,7 +380,7 @@ PyObject* py_fa_apply(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   HOST_CHECK(n == 17, "fa_apply takes 17 arguments, got ", n);
   const Tensor q = tensor_arg(args[0], "q"), k = tensor_arg(args[1], "k"), v = tensor_arg(args[2], "v");
-  Tensor mask = tensor_or_undefined(args[3]), drop = tensor_or_undefined(args[4]), alibi = tensor_or_undefined(args[5]);
+  const Tensor mask = tensor_or_undefined(args[3]), drop = tensor_or_undefined(args[4]), alibi = tensor_or_undefined(args[5]);
   const Tensor tiles = tensor_or_undefined(args[6]);
   FaConfig c;
   c.mask_tile128 = bool_arg(args[7]);
@@ -359,50 +392,20 @@ PyObject* py_fa_apply(PyObject*, PyObject* const* args, Py_ssize_t n) {
   c.tri_block = static_cast<int32_t>(low_bits_arg(args[13]));
   c.deterministic = bool_arg(args[14]);
   if (args[15] != Py_None) {
-    c.has_seed = true;
+    c.has_seed = 1;
     c.seed = low_bits_arg(args[15]);
     c.offset = low_bits_arg(args[16]);
   }
-  Tensor o, lse, plan;
   // as a Python autograd Function without a `jvp` does; a tangent would be dropped silently otherwise
-  for (const Tensor* t : {&q, &k, &v, &std::as_const(mask), &std::as_const(drop), &std::as_const(alibi)})
+  for (const Tensor* t : {&q, &k, &v, &mask, &drop, &alibi})
     TORCH_CHECK_NOT_IMPLEMENTED(!t->defined() || !t->_fw_grad(/*level=*/0).defined(),
                                 "the flash attention operator does not support forward mode AD");
-  const variable_list inputs = {q, k, v, mask, drop, alibi};      // (as given: below, the last three become packed)
+  // (an optional input may require a gradient too: it gets none, but the output is part of the graph)
+  const auto given = [](const Tensor& t) { return t.defined() ? std::optional<Tensor>(t) : std::nullopt; };
+  Tensor o, lse;
   {
     pybind11::gil_scoped_release no_gil;
-    {
-      at::AutoDispatchBelowADInplaceOrView below;
-      check_fa_inputs(q, k, v, mask, drop, alibi, tiles, c);
-      c10::cuda::OptionalCUDAGuard guard(q.device());
-      o = empty_like_shape(q.sizes(), q.scalar_type(), q);
-      lse = empty_like_shape(q.sizes().slice(0, 3), at::kFloat, q);
-      acct_fa_args a;
-      fill_args(a, q, k, v, o, lse, mask, drop, alibi, tiles, c);
-      const size_t plan_bytes = g_lib.mask_plan_bytes(&a);
-      if (plan_bytes > 0) {
-        plan = empty_like_shape({static_cast<int64_t>(plan_bytes)}, at::kByte, q);
-        check(g_lib.mask_plan(&a, plan.data_ptr(), stream_of(q)));
-      }
-      check(g_lib.fa_fwd(&a, plan.defined() ? plan.const_data_ptr() : nullptr, stream_of(q)));
-    }
-    // (an optional input may require a gradient too: it gets none, but the output is part of the graph)
-    if (torch::autograd::compute_requires_grad(inputs)) {
-      auto node = std::shared_ptr<FaBackward>(new FaBackward(), torch::autograd::deleteNode);
-      node->set_next_edges(torch::autograd::collect_next_edges(inputs));
-      node->cfg = c;
-      node->q_ = SavedVariable(q, false);
-      node->k_ = SavedVariable(k, false);
-      node->v_ = SavedVariable(v, false);
-      node->mask_ = SavedVariable(inputs[3], false);
-      node->drop_ = SavedVariable(inputs[4], false);
-      node->alibi_ = SavedVariable(inputs[5], false);
-      node->tiles_ = tiles;
-      node->plan_ = plan;
-      torch::autograd::set_history(o, node);
-      node->o_ = SavedVariable(o, true);
-      node->lse_ = SavedVariable(lse, false);
-    }
+    o = FaFunction::apply(q, k, v, given(mask), given(drop), given(alibi), FaCall{c, tiles, &lse});
   }
   PyObject* r = PyTuple_New(2);
   PyTuple_SET_ITEM(r, 0, wrap(o));

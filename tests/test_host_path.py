@@ -246,3 +246,22 @@ def test_mask_changed_before_the_backward_is_refused(packed):
     mask.zero_()
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         torch.autograd.grad(out, xs, d_o)
+
+
+def test_backward_under_compiled_autograd():
+    from torch._dynamo import compiled_autograd
+    q, k, v, d_o = _inputs(1, 2, 200, 64)
+    mask = _documents(200)
+    xs = [t.requires_grad_() for t in (q, k, v)]
+    layer = _layer(64, dropout_rate=0.25)
+    for seed in (1, 2):      # the second backward is the same graph with another dropout key
+        def forward():
+            layer.generator = torch.Generator().manual_seed(seed)
+            return layer(*xs, mask)
+        want = torch.autograd.grad(forward(), xs, d_o)
+        out = forward()
+        with compiled_autograd._enable(lambda graph: graph):
+            out.backward(d_o)
+        for t, b in zip(xs, want):
+            assert torch.equal(t.grad, b)
+            t.grad = None
