@@ -22,6 +22,8 @@ sizes are fixed inside the CUDA kernels.
 """
 from __future__ import annotations
 
+import torch
+
 from .... import ops as _ops
 from ...._lib import host as _host
 
@@ -67,10 +69,42 @@ def get_flash_attention_grad(prev_block_num=65536, next_block_num=65536, tiling_
     return fa_grad
 
 
+class _Traced(torch.autograd.Function):
+    """The operator as torch.jit.trace can record it: a Python function that runs again on the new inputs.  (The tracer
+    does not see the native path and would put its result into the graph as a constant.)"""
+
+    @staticmethod
+    def forward(ctx, query, key, value, attn_mask, dropout_mask, alibi_mask, options):
+        output, rowsum = _native(query, key, value, attn_mask, dropout_mask, alibi_mask, **options)
+        ctx.options = options
+        ctx.save_for_backward(query, key, value, output, rowsum, attn_mask, dropout_mask, alibi_mask)
+        ctx.mark_non_differentiable(rowsum)
+        return output, rowsum
+
+    @staticmethod
+    def backward(ctx, d_output, _d_rowsum):
+        query, key, value, output, rowsum, attn_mask, dropout_mask, alibi_mask = ctx.saved_tensors
+        grads = _ops.fa_backward(query, key, value, output, rowsum, d_output.contiguous(), attn_mask,
+                                 mask_tile128=_is_tile_mask(attn_mask), dropout_mask=dropout_mask, alibi=alibi_mask,
+                                 mask_tiles=_mask_tiles(attn_mask), **ctx.options)
+        return (*grads, None, None, None, None)
+
+
 def _apply(query, key, value, attn_mask, dropout_mask, alibi_mask, causal, keep_prob, prev_block_num, next_block_num,
            scale, tri_block=0, deterministic=False, dropout_seed=None, dropout_offset=0):
-    """The differentiable operator: (output, rowsum), by the native host path (its autograd node calls the grad
+    """The differentiable operator: (output, rowsum), by the native host path (its custom function calls the grad
     kernels and hands back dq, dk, dv in the input type)."""
+    if torch.jit.is_tracing():
+        return _Traced.apply(query, key, value, attn_mask, dropout_mask, alibi_mask,
+                             dict(causal=causal, keep_prob=keep_prob, prev_block_num=prev_block_num,
+                                  next_block_num=next_block_num, scale=scale, tri_block=tri_block,
+                                  deterministic=deterministic, dropout_seed=dropout_seed, dropout_offset=dropout_offset))
+    return _native(query, key, value, attn_mask, dropout_mask, alibi_mask, causal, keep_prob, prev_block_num,
+                   next_block_num, scale, tri_block, deterministic, dropout_seed, dropout_offset)
+
+
+def _native(query, key, value, attn_mask, dropout_mask, alibi_mask, causal, keep_prob, prev_block_num, next_block_num,
+            scale, tri_block, deterministic, dropout_seed, dropout_offset):
     tiles, tile_form = None, False
     if attn_mask is not None:
         tile_form = _is_tile_mask(attn_mask)

@@ -265,3 +265,16 @@ def test_backward_under_compiled_autograd():
         for t, b in zip(xs, want):
             assert torch.equal(t.grad, b)
             t.grad = None
+
+
+@pytest.mark.parametrize("masked", [False, True])
+def test_traced_cell_runs_on_new_inputs(masked):
+    layer = _layer(64)
+    ins = _inputs(1, 2, 200, 64)[:3] + ([_documents(200)] if masked else [])
+    traced = torch.jit.trace(lambda *x: layer(*x), tuple(ins), check_trace=False)
+    q, k, v, d_o = _inputs(1, 2, 200, 64, seed=1)
+    rest = [_documents(200).roll(7, dims=2)] if masked else []
+    with torch.no_grad():
+        assert torch.equal(traced(q, k, v, *rest), layer(q, k, v, *rest))
+    for a, b in zip(_grads(traced, (q, k, v), d_o, *rest), _grads(layer, (q, k, v), d_o, *rest)):
+        assert torch.equal(a, b)
