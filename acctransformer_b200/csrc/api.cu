@@ -445,12 +445,15 @@ size_t acct_mask_plan_bytes(const acct_fa_args* a) {
   return plan_parts(nullptr, a->mask_batch, a->S_q, a->S_k, &parts);
 }
 
-int acct_mask_plan(const acct_fa_args* a, void* plan, void* stream) {
+int acct_mask_plan(const acct_fa_args* a, void* plan, void* stream) { return acct_mask_plan_norms(a, plan, nullptr, 0, stream); }
+
+int acct_mask_plan_norms(const acct_fa_args* a, void* plan, void* norms, int32_t known, void* stream) {
   Strides st;
   int rc = validate_fa(a, &st);
   if (rc) return rc;
   if (plan == nullptr) return fail(ACCT_ERR_NULL, "plan is NULL");
-  if (!aligned16(plan)) return fail(ACCT_ERR_ALIGN, "plan must be 16-byte aligned");
+  if (known && norms == nullptr) return fail(ACCT_ERR_NULL, "norms is NULL");
+  if (!aligned16(plan) || !aligned16(norms)) return fail(ACCT_ERR_ALIGN, "plan and norms must be 16-byte aligned");
   if (!plan_applies(a)) return fail(ACCT_ERR_SHAPE, "no mask plan for this call (acct_mask_plan_bytes returns 0)");
   PerDevice* dev = nullptr;
   if ((rc = init_device(&dev))) return rc;
@@ -461,7 +464,8 @@ int acct_mask_plan(const acct_fa_args* a, void* plan, void* stream) {
   PlanParts parts;
   plan_parts(plan, a->mask_batch, a->S_q, a->S_k, &parts);
   cudaError_t e = launch_mask_plan(a->attn_mask, a->mask_dtype, a->mask_batch, a->mask_tiles, a->S_q, a->S_k, qkv, a->B, a->D,
-                                   a->dtype == ACCT_BF16, parts, static_cast<cudaStream_t>(stream));
+                                   a->dtype == ACCT_BF16, parts, static_cast<MaskPlan*>(norms), known != 0,
+                                   static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail_cuda(e, "launching the mask plan kernels");
   return ACCT_OK;
 }

@@ -139,14 +139,16 @@ cudaError_t launch_mask_classify(const void* mask, int dtype, int batch, int S_q
                                  cudaStream_t stream);
 
 // Fills a plan for a mask with its tile classes `tiles` and for q [B,N,S_q,D], k and v [B,N_kv,S_k,D] with element strides
-// (B, N, S); at most kPlanTiles tiles per dimension.
+// (B, N, S); at most kPlanTiles tiles per dimension.  `norms` (may be null): a head outside the plan whose norms are written
+// as well, or, if `norms_known`, taken instead of a pass over q, k and v.
 struct PlanOperand {
   const void* ptr;
   int64_t stride[3];
   int heads, rows;
 };
 cudaError_t launch_mask_plan(const void* mask, int mask_dtype, int mask_batch, const uint8_t* tiles, int S_q, int S_k,
-                             const PlanOperand (&qkv)[3], int B, int D, bool bf16, const PlanParts& plan, cudaStream_t stream);
+                             const PlanOperand (&qkv)[3], int B, int D, bool bf16, const PlanParts& plan, MaskPlan* norms,
+                             bool norms_known, cudaStream_t stream);
 
 // Raises a kernel's dynamic shared memory limit, once per thread, kernel and device (the call costs the host about as
 // much as a launch argument block, and every operator call would repeat it).

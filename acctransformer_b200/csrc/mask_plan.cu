@@ -72,8 +72,15 @@ __global__ void __launch_bounds__(kPlanThreads) mask_bits_kernel(const void* mas
   }
 }
 
-// One block per (Q tile, mask of the batch), one thread per K/V tile.
-__global__ void __launch_bounds__(kPlanThreads) mask_plan_kernel(int S_q, int S_k, PlanParts plan) {
+// One block per (Q tile, mask of the batch), one thread per K/V tile.  `norms`: see launch_mask_plan.
+__global__ void __launch_bounds__(kPlanThreads) mask_plan_kernel(int S_q, int S_k, PlanParts plan, MaskPlan* norms, bool norms_known) {
+  if (norms != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
+    if (norms_known) {
+      plan.head->q2 = norms->q2; plan.head->k2 = norms->k2; plan.head->v2 = norms->v2;
+    } else {
+      norms->q2 = norms->k2 = norms->v2 = norms->any = 0u;      // (raised by the next kernel)
+    }
+  }
   const int i = blockIdx.x, mb = blockIdx.y, tiles_q = gridDim.x, tiles_k = (S_k + kTile - 1) / kTile;
   const int64_t row_of_tiles = static_cast<int64_t>(mb) * tiles_q + i;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -96,7 +103,7 @@ struct NormOperands {
 
 // Largest squared row norm of each operand.  16 bytes per lane, LPR lanes per row; compared as bits, so that a NaN wins.
 template <bool BF16, int LPR>
-__global__ void plan_norms_kernel(const __grid_constant__ NormOperands ops, int B, int D, MaskPlan* plan) {
+__global__ void plan_norms_kernel(const __grid_constant__ NormOperands ops, int B, int D, MaskPlan* plan, MaskPlan* copy) {
   if (plan->any == 0u) return;
   __shared__ unsigned int block_max;
   const PlanOperand& t = ops.t[blockIdx.y];
@@ -125,28 +132,31 @@ __global__ void plan_norms_kernel(const __grid_constant__ NormOperands ops, int 
   most = __reduce_max_sync(0xffffffffu, most);
   if (lane == 0) atomicMax(&block_max, most);
   __syncthreads();
-  if (threadIdx.x == 0) atomicMax(blockIdx.y == 0 ? &plan->q2 : blockIdx.y == 1 ? &plan->k2 : &plan->v2, block_max);
+  if (threadIdx.x != 0) return;
+  atomicMax(blockIdx.y == 0 ? &plan->q2 : blockIdx.y == 1 ? &plan->k2 : &plan->v2, block_max);
+  if (copy != nullptr) atomicMax(blockIdx.y == 0 ? &copy->q2 : blockIdx.y == 1 ? &copy->k2 : &copy->v2, block_max);
 }
 
 }  // namespace
 
 cudaError_t launch_mask_plan(const void* mask, int mask_dtype, int mask_batch, const uint8_t* tiles, int S_q, int S_k,
-                             const PlanOperand (&qkv)[3], int B, int D, bool bf16, const PlanParts& plan, cudaStream_t stream) {
+                             const PlanOperand (&qkv)[3], int B, int D, bool bf16, const PlanParts& plan, MaskPlan* norms,
+                             bool norms_known, cudaStream_t stream) {
   const int tiles_q = (S_q + kTile - 1) / kTile, tiles_k = (S_k + kTile - 1) / kTile;
   // head, need_t and seen are added into; they come first
   const size_t zeroed = reinterpret_cast<uint8_t*>(plan.need) - reinterpret_cast<uint8_t*>(plan.head);
   cudaError_t e = cudaMemsetAsync(plan.head, 0, zeroed, stream);
   if (e != cudaSuccess) return e;
   mask_bits_kernel<<<dim3(tiles_k, tiles_q, mask_batch), kPlanThreads, 0, stream>>>(mask, mask_dtype, S_q, S_k, tiles, plan);
-  mask_plan_kernel<<<dim3(tiles_q, mask_batch), kPlanThreads, 0, stream>>>(S_q, S_k, plan);
+  mask_plan_kernel<<<dim3(tiles_q, mask_batch), kPlanThreads, 0, stream>>>(S_q, S_k, plan, norms, norms_known);
   e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
+  if (e != cudaSuccess || norms_known) return e;
   NormOperands ops;
   for (int i = 0; i < 3; ++i) ops.t[i] = qkv[i];
   auto kern = D <= 64 ? (bf16 ? plan_norms_kernel<true, 8> : plan_norms_kernel<false, 8>)
               : D <= 128 ? (bf16 ? plan_norms_kernel<true, 16> : plan_norms_kernel<false, 16>)
                          : (bf16 ? plan_norms_kernel<true, 32> : plan_norms_kernel<false, 32>);
-  kern<<<dim3(148 * 4, 3), 256, 0, stream>>>(ops, B, D, plan.head);
+  kern<<<dim3(148 * 4, 3), 256, 0, stream>>>(ops, B, D, plan.head, norms);
   return cudaGetLastError();
 }
 

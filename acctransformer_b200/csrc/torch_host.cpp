@@ -34,7 +34,7 @@ struct Library {
   decltype(&acct_fa_fwd_planned) fa_fwd;
   decltype(&acct_fa_bwd_planned) fa_bwd;
   decltype(&acct_mask_plan_bytes) mask_plan_bytes;
-  decltype(&acct_mask_plan) mask_plan;
+  decltype(&acct_mask_plan_norms) mask_plan;
   decltype(&acct_fa_bwd_workspace_bytes) fa_bwd_workspace_bytes;
   decltype(&acct_infer_prefill) infer_prefill;
   decltype(&acct_infer_decode) infer_decode;
@@ -230,7 +230,7 @@ Tensor readable(const Tensor& t, int64_t (&strides)[3]) {
 // saved-tensor hooks, compiled autograd, gradients that are not there -- works as around a Python one.
 struct FaCall {
   FaConfig cfg;
-  Tensor tiles;          // of the mask: this library's own, like the plan; no user sees or changes them
+  Tensor tiles;          // of the mask: this library's own, no user sees or changes it
   Tensor* lse;           // (not an output of the function: it has no gradient, and its saved form is not an output's)
 };
 
@@ -239,7 +239,7 @@ struct FaFunction : public torch::autograd::Function<FaFunction> {
                         const std::optional<Tensor>& drop_in, const std::optional<Tensor>& alibi_in, const FaCall& call) {
     const FaConfig& c = call.cfg;
     Tensor mask = mask_in.value_or(Tensor()), drop = drop_in.value_or(Tensor()), alibi = alibi_in.value_or(Tensor());
-    Tensor o, lse, plan;
+    Tensor o, lse, plan, norms;
     at::AutoDispatchBelowADInplaceOrView below;
     check_fa_inputs(q, k, v, mask, drop, alibi, call.tiles, c);     // (packs the last three)
     c10::cuda::OptionalCUDAGuard guard(q.device());
@@ -248,17 +248,26 @@ struct FaFunction : public torch::autograd::Function<FaFunction> {
     acct_fa_args a;
     fill_args(a, q, k, v, o, lse, mask, drop, alibi, call.tiles, c);
     const size_t plan_bytes = g_lib.mask_plan_bytes(&a);
+    bool keep_plan = false;
     if (plan_bytes > 0) {
+      // The backward uses a plan up to head_dim 128 and where dQ is summed in any order.  The plan is kept for it where that
+      // adds at most a sixteenth to what is saved anyway; a larger one (up to 64 MB, in every layer) is drawn up again from
+      // the mask and its 16 bytes of norms, which takes about 25 us (3 000 tokens of four documents, 2 x 32 heads of 128:
+      // 4.7 MB next to 123 MB, forward and backward 471 us kept, 496 us drawn up again).
+      const bool wanted = q.size(3) <= 128 && !c.deterministic;
+      keep_plan = wanted && plan_bytes * 16 <= 2 * (q.nbytes() + k.nbytes());
       plan = empty_like_shape({static_cast<int64_t>(plan_bytes)}, at::kByte, q);
-      check(g_lib.mask_plan(&a, plan.data_ptr(), stream_of(q)));
+      if (wanted && !keep_plan) norms = empty_like_shape({16}, at::kByte, q);
+      check(g_lib.mask_plan(&a, plan.data_ptr(), norms.defined() ? norms.data_ptr() : nullptr, 0, stream_of(q)));
     }
     check(g_lib.fa_fwd(&a, plan.defined() ? plan.const_data_ptr() : nullptr, stream_of(q)));
     *call.lse = lse;
     // (the optional inputs as given, not their packed copies)
-    ctx->save_for_backward({q, k, v, o, lse, mask_in.value_or(Tensor()), drop_in.value_or(Tensor()), alibi_in.value_or(Tensor())});
+    ctx->save_for_backward({q, k, v, o, lse, mask_in.value_or(Tensor()), drop_in.value_or(Tensor()), alibi_in.value_or(Tensor()),
+                            keep_plan ? plan : Tensor()});
     ctx->saved_data["config"] = c.pack();
     if (call.tiles.defined()) ctx->saved_data["tiles"] = call.tiles;
-    if (plan.defined()) ctx->saved_data["plan"] = plan;
+    if (norms.defined()) ctx->saved_data["norms"] = norms;
     return o;
   }
 
@@ -270,7 +279,7 @@ struct FaFunction : public torch::autograd::Function<FaFunction> {
       const auto it = ctx->saved_data.find(key);
       return it == ctx->saved_data.end() ? Tensor() : it->second.toTensor();
     };
-    const Tensor tiles = tensor_of("tiles"), plan = tensor_of("plan");
+    const Tensor tiles = tensor_of("tiles"), norms = tensor_of("norms");
     const FaConfig cfg = FaConfig::unpack(ctx->saved_data.at("config").toIntVector());
 
     at::AutoDispatchBelowADInplaceOrView below;
@@ -299,6 +308,15 @@ struct FaFunction : public torch::autograd::Function<FaFunction> {
     g.d_o = d_o.const_data_ptr();
     g.dq = dq.data_ptr(); g.dk = dk.data_ptr(); g.dv = dv.data_ptr();
     g.workspace = ws.data_ptr(); g.workspace_bytes = nbytes;
+    Tensor plan = saved[8];
+    if (plan.defined()) {
+      require_on("plan", plan, q);
+      HOST_CHECK(plan.scalar_type() == at::kByte && static_cast<size_t>(plan.numel()) == g_lib.mask_plan_bytes(&a), "not the plan that was saved");
+      plan = plan.contiguous();
+    } else if (norms.defined()) {
+      plan = empty_like_shape({static_cast<int64_t>(g_lib.mask_plan_bytes(&a))}, at::kByte, q);
+      check(g_lib.mask_plan(&a, plan.data_ptr(), norms.data_ptr(), 1, stream_of(q)));
+    }
     check(g_lib.fa_bwd(&a, &g, d_o_strides, plan.defined() ? plan.const_data_ptr() : nullptr,
                        static_cast<uint8_t*>(ws.data_ptr()) + own, stream_of(q)));
     return {dq, dk, dv, Tensor(), Tensor(), Tensor(), Tensor()};
@@ -366,7 +384,7 @@ PyObject* py_init(PyObject*, PyObject* path) {
   g_lib.fa_fwd = reinterpret_cast<decltype(g_lib.fa_fwd)>(sym("acct_fa_fwd_planned"));
   g_lib.fa_bwd = reinterpret_cast<decltype(g_lib.fa_bwd)>(sym("acct_fa_bwd_planned"));
   g_lib.mask_plan_bytes = reinterpret_cast<decltype(g_lib.mask_plan_bytes)>(sym("acct_mask_plan_bytes"));
-  g_lib.mask_plan = reinterpret_cast<decltype(g_lib.mask_plan)>(sym("acct_mask_plan"));
+  g_lib.mask_plan = reinterpret_cast<decltype(g_lib.mask_plan)>(sym("acct_mask_plan_norms"));
   g_lib.fa_bwd_workspace_bytes = reinterpret_cast<decltype(g_lib.fa_bwd_workspace_bytes)>(sym("acct_fa_bwd_workspace_bytes"));
   g_lib.infer_prefill = reinterpret_cast<decltype(g_lib.infer_prefill)>(sym("acct_infer_prefill"));
   g_lib.infer_decode = reinterpret_cast<decltype(g_lib.infer_decode)>(sym("acct_infer_decode"));

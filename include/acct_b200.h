@@ -228,9 +228,13 @@ ACCT_API int acct_fa_bwd_strided(const acct_fa_args* a, const acct_fa_bwd_io* g,
  * computed.  acct_mask_plan_bytes: size of the plan, 0 where none applies (it takes an ACCT_MASK_FULL mask with mask_tiles
  * and no causal, alibi, band, seq_lens, tri_block or dropout_mask, at most 32 768 positions, and enough work to pay for the
  * plan's passes).  acct_mask_plan enqueues its passes over the mask's classes and q, k, v of `a` (device memory, 16-byte
- * aligned); the plan is good for calls with the same `a`.  plan_scratch: 8 bytes of device memory of the call's own. */
+ * aligned); the plan is good for calls with the same `a`.  plan_scratch: 8 bytes of device memory of the call's own.
+ * A plan holds bits for every tile and is large; what it takes from q, k and v is 16 bytes.  acct_mask_plan_norms writes
+ * those to `norms` (device memory, 16-byte aligned) as well, or, with `known`, takes them from there: a caller need not keep
+ * the plan from the forward to the backward. */
 ACCT_API size_t acct_mask_plan_bytes(const acct_fa_args* a);
 ACCT_API int acct_mask_plan(const acct_fa_args* a, void* plan, void* stream);
+ACCT_API int acct_mask_plan_norms(const acct_fa_args* a, void* plan, void* norms, int32_t known, void* stream);
 ACCT_API int acct_fa_fwd_planned(const acct_fa_args* a, const void* plan, void* stream);
 ACCT_API int acct_fa_bwd_planned(const acct_fa_args* a, const acct_fa_bwd_io* g, const int64_t* d_o_stride, const void* plan,
                                  void* plan_scratch, void* stream);

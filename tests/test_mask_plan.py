@@ -106,3 +106,35 @@ def test_operands_that_reach_past_the_mask(what):
         else:
             d_o[1, 5, 1499, 7] = float("-inf")
     _run(*_case("documents"), change)
+
+
+# what a call keeps for its backward besides the tensors that it has to: at most a sixteenth of those, nothing where the
+# backward uses no plan (deterministic, wide heads); (8 heads, 4 096 tokens): drawn up again, (64, 2 048): kept
+@pytest.mark.parametrize("N,S,D,deterministic", [(8, 4096, 64, False), (64, 2048, 64, False), (64, 2048, 64, True),
+                                                 (64, 2048, 160, False)])
+def test_memory_held_until_the_backward(N, S, D, deterministic):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from acctransformer_b200 import _lib, ops
+    from acctransformer_b200.flash_attention.ops.flash_attention.flash_attention_impl import get_flash_attention
+    g = torch.Generator(device="cuda").manual_seed(D)
+    q, k, v, d_o = (torch.randn(1, N, S, D, device="cuda", dtype=torch.float16, generator=g) for _ in range(4))
+    mask = _documents(S, [[500, 1100]]).half().cuda()
+    tiles = ops.mask_tile_classes(mask)
+    fa = get_flash_attention(scale=1.0 / math.sqrt(D), deterministic=deterministic)
+    xs = [t.requires_grad_() for t in (q, k, v)]
+    before = torch.cuda.memory_allocated()
+    o, lse = fa(*xs, mask)
+    held = torch.cuda.memory_allocated() - before - o.numel() * 2 - lse.numel() * 4
+    kept = N == 64 and D == 64 and not deterministic
+    assert held <= (4 * q.numel() * 2 // 16 if kept else 4096)
+    for retain in (True, False):     # the second backward finds what the first did
+        got = torch.autograd.grad(o, xs, d_o, retain_graph=retain)
+        with torch.no_grad():
+            want = ops.fa_backward(q, k, v, o, lse, d_o, mask, scale=1.0 / math.sqrt(D), mask_tiles=tiles, deterministic=deterministic)
+        for a, b in zip(got, want):      # one unit of a 16-bit P or dS, then the result's own rounding
+            assert (a.float() - b.float()).abs().max().item() <= 2 * 2.0 ** -11 * b.float().abs().max().item()
+    del got, want, a, b
+    assert torch.cuda.memory_allocated() - before - o.numel() * 2 - lse.numel() * 4 <= 4096      # given back, although the output still lives
+    torch.cuda.synchronize()
+    _lib.device_status()
