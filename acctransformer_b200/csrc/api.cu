@@ -685,7 +685,10 @@ int acct_infer_decode(const acct_decode_args* a, void* stream) {
   DeviceInfo info;
   if ((rc = device_info(&info))) return rc;
   const int64_t units = static_cast<int64_t>(a->B) * n_kv;
-  bool clustered = false;
+  DecodeParams p;
+  p.B = a->B; p.N = a->N; p.S_max = a->S_max; p.D = a->D;
+  p.kv_group = group;
+  p.clustered = 0;
   if (splits == 0) {
     // Automatic choice.  Sequence lengths differ between the sequences of a batch (1 024 .. 16 384 keys in the
     // benchmark configuration), and a (sequence, cache head) slice cut into few parts leaves the SMs unevenly
@@ -704,32 +707,42 @@ int acct_infer_decode(const acct_decode_args* a, void* stream) {
     if (want > fit) want = fit;
     splits = static_cast<int>(want < 1 ? 1 : want);
     // Short contexts of few slices: the parts of a slice form one cluster, which merges them without a second kernel
-    // (decode_common.cuh), and may be as short as 128 keys.  All clusters have to be resident at once (2 thread blocks
-    // of the grouped kernel or 4 of the other per SM): a cluster's blocks start together, so with more of them the SMs
-    // wait for whole clusters to fit (32 x 32 slices of 4 096 keys in 8 parts: 269 us against 227 for two kernels).
-    // Measured: 32 slices of 4 heads, 2 048 keys 15.3 -> 11.6 us; 128 slices of 512 keys 18.2 -> 9.3 us.
+    // (decode_common.cuh), and may be as short as 128 keys.  All clusters have to be resident at once: a cluster's blocks
+    // start together, so with more of them the SMs wait for whole clusters to fit (70 slices of 4 096 keys in 8 parts: 0.96 of
+    // the time of two kernels, 72 slices: 1.29).  And with fewer than 8 parts the longest sequence of a batch decides, so
+    // those may not be long: valid lengths uniform in [1/4, 1], 160 slices in 2 parts, 1 024 / 1 536 / 2 048 / 4 096 keys:
+    // 0.93 / 1.13 / 1.19 / 1.47; 88 slices in 4 parts, 2 048 / 3 072 keys: 0.96 / 1.12.  Grouped heads, of which one block
+    // carries a whole group, bear twice that: 64 slices of 4 heads in 4 parts, 4 096 keys: 0.89; 128 in 2 parts,
+    // 2 048 / 4 096 keys: 0.94 / 1.00.
+    // 32 slices of 4 heads, 2 048 keys 15.3 -> 11.6 us; 128 slices of 512 keys 18.2 -> 9.3 us.
     if (a->S_max <= 4096) {
-      const int64_t slots = static_cast<int64_t>(info.sm_count) * (group > 1 ? 2 : 4);
-      int parts = 8;
-      while (parts > 1 && (units * parts > slots || static_cast<int64_t>(parts) * 128 > a->S_max + 127)) parts /= 2;
-      clustered = units * parts <= slots && parts <= fit && (parts > 1 || a->S_max <= 128);
-      if (clustered) splits = parts;
+      const int longest = group > 1 ? 1024 : 512;
+      for (int parts : {8, 4, 2, 1}) {
+        if (parts * 128 > a->S_max + 127 || parts > fit) continue;
+        if (parts * longest < a->S_max || (parts == 1 && a->S_max > 128)) break;
+        p.clustered = 1;
+        p.splits = parts;
+        int resident = 0;
+        cudaError_t e = launch_decode(p, a->dtype == ACCT_BF16, nullptr, &resident);
+        if (e != cudaSuccess) return fail_cuda(e, "asking for the resident clusters");
+        if (units <= resident) {
+          splits = parts;
+          break;
+        }
+        p.clustered = 0;
+      }
     }
   }
   const size_t need = static_cast<size_t>(a->B) * a->N * splits * (static_cast<size_t>(a->D) + 2) * 4;
   if (a->workspace == nullptr || a->workspace_bytes < need)
     return fail(ACCT_ERR_WORKSPACE, "decode workspace: need %zu bytes, got %zu", need, a->workspace ? a->workspace_bytes : (size_t)0);
   if (!aligned16(a->workspace)) return fail(ACCT_ERR_ALIGN, "workspace must be 16-byte aligned");
-  DecodeParams p;
   p.q = a->q; p.k = a->k_cache; p.v = a->v_cache; p.y = a->y; p.seq_lens = a->seq_lens;
   p.part_acc = static_cast<float*>(a->workspace);
   p.part_ml = p.part_acc + static_cast<size_t>(a->B) * a->N * splits * a->D;
   p.kv_stride_b = kvs[0]; p.kv_stride_h = kvs[1]; p.kv_stride_s = kvs[2];
-  p.B = a->B; p.N = a->N; p.S_max = a->S_max; p.D = a->D;
-  p.kv_group = group;
   p.block_table = a->block_table; p.page_shift = page_shift; p.max_pages = a->max_pages;
   p.splits = splits;
-  p.clustered = clustered ? 1 : 0;
   p.scale_log2 = a->scale * kLog2e;
   cudaError_t e = launch_decode(p, a->dtype == ACCT_BF16, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail_cuda(e, "launching the decode kernels");

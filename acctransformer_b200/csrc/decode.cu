@@ -429,37 +429,37 @@ cudaError_t launch_merge(const DecodeParams& p, bool bf16, cudaStream_t stream) 
 }
 
 template <int LPR, int G>
-cudaError_t launch_decode_g(const DecodeParams& p, bool bf16, cudaStream_t stream) {
+cudaError_t launch_decode_g(const DecodeParams& p, bool bf16, cudaStream_t stream, int* resident) {
   auto kern = p.clustered ? (bf16 ? decode_split_kernel<LPR, true, G, true> : decode_split_kernel<LPR, false, G, true>)
                           : (bf16 ? decode_split_kernel<LPR, true, G, false> : decode_split_kernel<LPR, false, G, false>);
-  const cudaError_t e = launch_parts(kern, p, p.B * (p.N / G), kDecodeThreads, 0, stream);
+  const cudaError_t e = launch_parts(kern, p, p.B * (p.N / G), kDecodeThreads, 0, stream, resident);
   if (e != cudaSuccess || p.clustered) return e;
   return launch_merge(p, bf16, stream);
 }
 
 template <int LPR>
-cudaError_t launch_decode_lpr(const DecodeParams& p, bool bf16, cudaStream_t stream) {
+cudaError_t launch_decode_lpr(const DecodeParams& p, bool bf16, cudaStream_t stream, int* resident) {
   switch (p.kv_group) {
-    case 1: return launch_decode_g<LPR, 1>(p, bf16, stream);
-    case 2: return launch_decode_g<LPR, 2>(p, bf16, stream);
-    case 4: return launch_decode_g<LPR, 4>(p, bf16, stream);
-    case 8: return launch_decode_g<LPR, 8>(p, bf16, stream);
+    case 1: return launch_decode_g<LPR, 1>(p, bf16, stream, resident);
+    case 2: return launch_decode_g<LPR, 2>(p, bf16, stream, resident);
+    case 4: return launch_decode_g<LPR, 4>(p, bf16, stream, resident);
+    case 8: return launch_decode_g<LPR, 8>(p, bf16, stream, resident);
     default: return cudaErrorInvalidValue;   // the entry point admits 1, 2, 4, 8 only
   }
 }
 
 }  // namespace
 
-cudaError_t launch_decode(const DecodeParams& p, bool bf16, cudaStream_t stream) {
+cudaError_t launch_decode(const DecodeParams& p, bool bf16, cudaStream_t stream, int* resident) {
   // several query heads per cache head, head_dim <= 128: the group goes on the rows of a tensor-core MMA
   if (p.kv_group >= kDecodeGqaMinGroup && p.D <= 128) {
-    cudaError_t e = launch_decode_gqa_split(p, bf16, stream);
+    cudaError_t e = launch_decode_gqa_split(p, bf16, stream, resident);
     if (e != cudaSuccess || p.clustered) return e;
     return launch_merge(p, bf16, stream);
   }
-  if (p.D <= 64) return launch_decode_lpr<8>(p, bf16, stream);
-  if (p.D <= 128) return launch_decode_lpr<16>(p, bf16, stream);
-  return launch_decode_lpr<32>(p, bf16, stream);
+  if (p.D <= 64) return launch_decode_lpr<8>(p, bf16, stream, resident);
+  if (p.D <= 128) return launch_decode_lpr<16>(p, bf16, stream, resident);
+  return launch_decode_lpr<32>(p, bf16, stream, resident);
 }
 
 }  // namespace acct

@@ -71,9 +71,33 @@ __device__ __forceinline__ void cluster_merge(const DecodeParams& p, float* acc,
   cluster_sync();      // nobody's shared memory goes away while another block still reads it
 }
 
-// One thread block per part; the parts of a slice form a cluster where p.clustered says so.
+// How many clusters of p.splits blocks of this kernel the device holds at once.  Fewer than its SMs could hold blocks: a
+// cluster stays inside one GPC, and what is left over there is too small for another.  Asked once per thread, kernel,
+// cluster size and device.
+inline cudaError_t resident_clusters(void (*kern)(const DecodeParams), const cudaLaunchConfig_t& cfg, int splits, int* out) {
+  struct Seen {
+    const void* kernel;
+    int splits, dev, n;
+  };
+  static thread_local Seen seen[16];       // zero-initialised; newest entry overwrites the oldest
+  static thread_local unsigned next = 0;
+  int dev = -1;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  for (const Seen& s : seen)
+    if (s.kernel == reinterpret_cast<const void*>(kern) && s.splits == splits && s.dev == dev) {
+      *out = s.n;
+      return cudaSuccess;
+    }
+  e = cudaOccupancyMaxActiveClusters(out, kern, &cfg);
+  if (e == cudaSuccess) seen[next++ % 16] = {reinterpret_cast<const void*>(kern), splits, dev, *out};
+  return e;
+}
+
+// One thread block per part; the parts of a slice form a cluster where p.clustered says so.  With `resident` nothing is
+// launched: it receives the number of such clusters that fit at once.
 inline cudaError_t launch_parts(void (*kern)(const DecodeParams), const DecodeParams& p, int units, int threads, size_t smem,
-                                cudaStream_t stream) {
+                                cudaStream_t stream, int* resident) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(p.splits, units);
   cfg.blockDim = dim3(threads);
@@ -86,6 +110,7 @@ inline cudaError_t launch_parts(void (*kern)(const DecodeParams), const DecodePa
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = p.clustered ? 1 : 0;
+  if (resident != nullptr) return resident_clusters(kern, cfg, p.splits, resident);
   return cudaLaunchKernelEx(&cfg, kern, p);
 }
 

@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(kGqaThreads) decode_gqa_kernel(const DecodePar
 }
 
 template <int DPAD>
-cudaError_t launch_gqa(const DecodeParams& p, bool bf16, cudaStream_t stream) {
+cudaError_t launch_gqa(const DecodeParams& p, bool bf16, cudaStream_t stream, int* resident) {
   const size_t ring = static_cast<size_t>(kGqaWarps) * kRing * 2 * kTileRows * (DPAD * 2 + 16);
   const size_t merge = static_cast<size_t>(kGqaWarps + 1) * 16 * (DPAD + 2) * sizeof(float);
   const size_t smem = ring > merge ? ring : merge;
@@ -331,16 +331,16 @@ cudaError_t launch_gqa(const DecodeParams& p, bool bf16, cudaStream_t stream) {
 #undef ACCT_GQA
   cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), smem);
   if (e != cudaSuccess) return e;
-  return launch_parts(kern, p, p.B * (p.N / p.kv_group), kGqaThreads, smem, stream);
+  return launch_parts(kern, p, p.B * (p.N / p.kv_group), kGqaThreads, smem, stream, resident);
 }
 
 }  // namespace
 
 // The split kernel for a group of 2..16 query heads per cache head, head_dim <= 128 (the caller then runs the merge
 // kernel of decode.cu over the partial results).
-cudaError_t launch_decode_gqa_split(const DecodeParams& p, bool bf16, cudaStream_t stream) {
-  if (p.D <= 64) return launch_gqa<64>(p, bf16, stream);
-  return launch_gqa<128>(p, bf16, stream);
+cudaError_t launch_decode_gqa_split(const DecodeParams& p, bool bf16, cudaStream_t stream, int* resident) {
+  if (p.D <= 64) return launch_gqa<64>(p, bf16, stream, resident);
+  return launch_gqa<128>(p, bf16, stream, resident);
 }
 
 }  // namespace acct

@@ -172,9 +172,10 @@ cudaError_t launch_bwd_delta(const void* o, const void* d_o, float* delta, int64
                              float* zero_acc, unsigned int* counters, int64_t n_counters, unsigned int* plan_stats);
 cudaError_t launch_bwd_convert_dq(const float* dq_acc, void* dq, int64_t n_elems, bool bf16, bool f32_out,
                                   cudaStream_t stream);
-cudaError_t launch_decode(const DecodeParams& p, bool bf16, cudaStream_t stream);
+// (with `resident` nothing is launched: see launch_parts)
+cudaError_t launch_decode(const DecodeParams& p, bool bf16, cudaStream_t stream, int* resident = nullptr);
 // split kernel for 2..16 query heads per cache head at head_dim <= 128 (tensor-core path, decode_gqa.cu)
-cudaError_t launch_decode_gqa_split(const DecodeParams& p, bool bf16, cudaStream_t stream);
+cudaError_t launch_decode_gqa_split(const DecodeParams& p, bool bf16, cudaStream_t stream, int* resident);
 #ifndef ACCT_DECODE_GQA_MIN_GROUP
 #define ACCT_DECODE_GQA_MIN_GROUP 2
 #endif

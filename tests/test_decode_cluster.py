@@ -39,6 +39,31 @@ def test_clustered_parts_against_the_oracle(B, n_kv, group, S, D, dtype):
     assert float(np.max(np.abs(y.float().cpu().numpy() - want))) <= tol
 
 
+# around the lines of the rule: more slices than clusters of 8 (4, 2) parts fit at once, parts of 512 keys and one more (1 024
+# where a block carries a group), a workspace that holds fewer parts
+@pytest.mark.parametrize("B,n_kv,group,S,fit", [
+    (70, 1, 1, 600, 64), (71, 1, 1, 2048, 64), (72, 1, 1, 2049, 64), (142, 1, 1, 600, 64), (149, 1, 1, 1024, 64),
+    (149, 1, 1, 1025, 64), (297, 1, 1, 256, 64), (33, 1, 4, 1024, 64), (35, 1, 4, 4096, 64), (72, 1, 4, 2048, 64),
+    (74, 1, 4, 2049, 64), (149, 1, 4, 300, 64), (2, 2, 1, 1000, 3), (2, 2, 4, 1000, 1),
+])
+def test_around_the_lines_of_the_rule(B, n_kv, group, S, fit):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from acctransformer_b200 import _lib, ops
+    D = 64
+    g = torch.Generator(device="cuda").manual_seed(S + B)
+    q = torch.randn(B, n_kv * group, 1, D, device="cuda", generator=g).half()
+    k, v = (torch.randn(B, n_kv, S, D, device="cuda", generator=g).half() for _ in range(2))
+    lens = torch.randint(1, S + 1, (B,), generator=torch.Generator().manual_seed(S), dtype=torch.int32).cuda()
+    ws = ops.DecodeWorkspace(B, n_kv * group, D, "cuda", fit)
+    y = ops.infer_decode(q, k, v, lens, workspace=ws)
+    one = ops.infer_decode(q, k, v, lens, num_splits=1)          # the whole slice in one part
+    torch.cuda.synchronize()
+    _lib.device_status()
+    # one rounding of a result of up to 4, and with groups probabilities rounded against another running maximum
+    assert (y.float() - one.float()).abs().max().item() <= 4e-3
+
+
 # the second kernel, which merges the parts where they are no cluster: batches of 16 parts, two halves of 32; empty parts
 @pytest.mark.parametrize("splits", [1, 2, 15, 16, 17, 32, 33, 49, 64])
 @pytest.mark.parametrize("group,D,dtype", [(1, 40, "float16"), (4, 128, "bfloat16"), (1, 256, "float16")])
