@@ -101,11 +101,15 @@ def host():
     global _host
     if _host is None:
         load()
+        from . import build
+        rebuild = "build it with `python -m acctransformer_b200.build`; there is no fallback path"
+        built_for = build.host_built_for()      # (imports torch, whose libraries the module needs in the process)
         try:
             from . import _torch_host
         except ImportError as e:
-            raise ImportError("the _torch_host module is missing or does not match this torch: build it with "
-                              "`python -m acctransformer_b200.build`; there is no fallback path") from e
+            raise ImportError("the _torch_host module is missing or does not match this torch: " + rebuild) from e
+        if _torch_host.built_for != built_for:
+            raise ImportError(f"the _torch_host module was built for {_torch_host.built_for}, but this is {built_for}: " + rebuild)
         _torch_host.init(LIB_PATH)
         _host = _torch_host
     return _host

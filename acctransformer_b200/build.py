@@ -27,6 +27,22 @@ NVCC_FLAGS = [
 ]
 HOST_SOURCE = "torch_host.cpp"
 HOST_PATH = os.path.join(HERE, "_torch_host.so")
+HOST_STAMP = os.path.join(OBJ_DIR, "_torch_host.built_for")
+
+
+def host_built_for():
+    """What the host module is compiled against and only good for: torch's C++ classes and the interpreter."""
+    import torch
+    python = ".".join(map(str, sys.version_info[:2]))
+    return f"torch {torch.__version__}, C++ ABI {int(torch._C._GLIBCXX_USE_CXX11_ABI)}, Python {python}"
+
+
+def host_is_stale():
+    sources = [os.path.join(CSRC, HOST_SOURCE), os.path.join(os.path.dirname(HERE), "include", "acct_b200.h")]
+    if _stale(HOST_PATH, sources) or not os.path.exists(HOST_STAMP):
+        return True
+    with open(HOST_STAMP) as f:
+        return f.read() != host_built_for()
 
 
 def _host_command(src, out):
@@ -38,7 +54,7 @@ def _host_command(src, out):
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
     lib = os.path.join(os.path.dirname(torch.__file__), "lib")
     return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wno-attributes",
-            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DACCT_BUILT_FOR="{host_built_for()}"',
             "-I" + inc, "-I" + os.path.join(inc, "torch", "csrc", "api", "include"), "-I" + sysconfig.get_paths()["include"],
             "-I" + os.path.join(cuda, "include"), src, "-o", out,
             "-L" + lib, "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10", "-ldl"]
@@ -81,13 +97,16 @@ def build(force=False, verbose=False):
         if r.returncode != 0:
             raise RuntimeError("compiling failed: " + " ".join(cmd))
 
-    host_src = os.path.join(CSRC, HOST_SOURCE)
-    if force or _stale(HOST_PATH, [host_src, os.path.join(os.path.dirname(HERE), "include", "acct_b200.h")]):
-        jobs.append(_host_command(host_src, HOST_PATH))
+    host = force or host_is_stale()
+    if host:
+        jobs.append(_host_command(os.path.join(CSRC, HOST_SOURCE), HOST_PATH))
     device_jobs = any(cmd[0] == nvcc for cmd in jobs)
 
     with ThreadPoolExecutor(max_workers=4) as ex:
         list(ex.map(run, jobs))
+    if host:
+        with open(HOST_STAMP, "w") as f:
+            f.write(host_built_for())
     if force or device_jobs or _stale(LIB_PATH, objs):
         run([nvcc, "-shared", "-o", LIB_PATH] + objs + ["-lcudart"])
     return LIB_PATH

@@ -551,4 +551,12 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_torch_host", "native host path o
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__torch_host(void) { return PyModule_Create(&kModule); }
+// (the loader compares `built_for` with the running torch and interpreter before it calls anything: build.py)
+PyMODINIT_FUNC PyInit__torch_host(void) {
+  PyObject* m = PyModule_Create(&kModule);
+  if (m != nullptr && PyModule_AddStringConstant(m, "built_for", ACCT_BUILT_FOR) != 0) {
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}
