@@ -1,7 +1,7 @@
 """Builds ``libacct_b200.so`` (the C-ABI library) from ``csrc/*.cu`` with nvcc for sm_100a.
 
 Beside it, ``_torch_host.so`` (the native host path of the Python layers) is compiled from ``csrc/torch_host.cpp`` with
-the host compiler against the installed torch.
+the host compiler against the installed torch; without torch, only the library is built.
 
 The library is built in-tree, next to this file, so that it travels with the source tree.
 ``python -m acctransformer_b200.build`` rebuilds it; ``build()`` is also what
@@ -97,7 +97,12 @@ def build(force=False, verbose=False):
         if r.returncode != 0:
             raise RuntimeError("compiling failed: " + " ".join(cmd))
 
-    host = force or host_is_stale()
+    try:
+        host_built_for()
+        host = force or host_is_stale()
+    except ImportError:      # the C ABI (MindSpore and other callers) needs no torch
+        sys.stderr.write("no torch here: _torch_host is not built (the Python layers need it, the library does not)\n")
+        host = False
     if host:
         jobs.append(_host_command(os.path.join(CSRC, HOST_SOURCE), HOST_PATH))
     device_jobs = any(cmd[0] == nvcc for cmd in jobs)

@@ -19,3 +19,11 @@ def test_host_module_of_another_torch_is_refused(monkeypatch):
     monkeypatch.setattr(build, "host_built_for", lambda: "torch 0.0.0")
     with pytest.raises(ImportError, match="was built for torch .* but this is torch 0.0.0"):
         _lib.host()
+
+
+def test_library_is_built_without_torch(monkeypatch, capfd):
+    import os
+    import sys
+    monkeypatch.setitem(sys.modules, "torch", None)      # `import torch` fails
+    assert os.path.exists(build.build())
+    assert "_torch_host is not built" in capfd.readouterr().err
