@@ -1,13 +1,16 @@
 """Backward at head_dim in (128, 160]: one thread block holds dK and dV of a K/V tile whole, in steps of 64 queries.
 
-Checked against the split-width kernel, which the deterministic flag selects: two kernels that share nothing but the
-formulas (that one is checked against the oracle elsewhere).  Both round P and dS to 16 bits and sum in fp32, so a
-gradient differs by the rounding of its 16 bits and by fp32 sums in another order.
+Checked against the split-width kernel, which the deterministic flag selects: two kernels that share the formulas and the
+keep bits of in-kernel dropout (those are checked against the oracle below, that kernel elsewhere).  Both round P and dS to
+16 bits and sum in fp32, so a gradient differs by the rounding of its 16 bits and by fp32 sums in another order.
 """
 import math
 
+import numpy as np
 import pytest
 import torch
+
+from oracle import attention_ref as ref
 
 pytestmark = pytest.mark.gpu
 
@@ -67,3 +70,23 @@ def test_against_the_split_width_kernel(case, dtype, f32):
         assert torch.isfinite(a).all()
         err = (a.float() - b.float()).abs().max().item()
         assert err <= 2 * unit * max(b.float().abs().max().item(), 1e-3)
+
+
+@pytest.mark.parametrize("causal", [False, True])
+def test_in_kernel_dropout_against_the_oracle(causal):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from acctransformer_b200 import _lib, ops
+    S, D = 200, 160
+    g = torch.Generator().manual_seed(D)
+    q, k, v, d_o = (torch.randn(1, 2, S, D, generator=g).half() for _ in range(4))
+    scale, kw = 1.0 / math.sqrt(D), dict(causal=causal, keep_prob=0.75, dropout_seed=11, dropout_offset=3)
+    o, lse = ops.fa_forward(q.cuda(), k.cuda(), v.cuda(), scale=scale, **kw)
+    got = ops.fa_backward(q.cuda(), k.cuda(), v.cuda(), o, lse, d_o.cuda(), scale=scale, grads_fp32=True, **kw)
+    torch.cuda.synchronize()
+    _lib.device_status()
+    drop = ops.dropout_mask(1, 2, S, S, 0.75, 11, 3).cpu().numpy()
+    want = ref.sa_grad(*(t.float().numpy() for t in (q, k, v, d_o)), drop_mask=drop, keep_prob=ref.dropout_threshold(0.75) / 256.0,
+                       causal=causal, scale=scale)
+    for a, b in zip(got, want):      # P, dS and the forward's O to 2^-11, sums of 200 terms of both signs: 1e-2 of the largest
+        assert float(np.max(np.abs(a.cpu().numpy() - b))) <= 1e-2 * float(np.max(np.abs(b)))

@@ -278,3 +278,42 @@ def test_traced_cell_runs_on_new_inputs(masked):
         assert torch.equal(traced(q, k, v, *rest), layer(q, k, v, *rest))
     for a, b in zip(_grads(traced, (q, k, v), d_o, *rest), _grads(layer, (q, k, v), d_o, *rest)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("reentrant", [False, True])
+def test_checkpointed_cell(reentrant):
+    from torch.utils.checkpoint import checkpoint
+    q, k, v, d_o = _inputs(1, 2, 200, 64)
+    mask, layer = _documents(200), _layer(64, dropout_rate=0.25)
+    torch.manual_seed(3)
+    want = _grads(layer, (q, k, v), d_o, mask)
+    xs = [t.detach().requires_grad_() for t in (q, k, v)]
+    torch.manual_seed(3)
+    checkpoint(layer, *xs, mask, use_reentrant=reentrant).backward(d_o)
+    for t, b in zip(xs, want):
+        assert torch.equal(t.grad, b)
+
+
+def test_threads_and_streams():
+    """Four threads, each with a stream and inputs of its own, run the cell forward and backward at the same time."""
+    import threading
+    layer, mask = _layer(64), _documents(200)
+    ins = [_inputs(1, 2, 200, 64, seed=s) for s in range(4)]
+    want = [_grads(layer, x[:3], x[3], mask) for x in ins]
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(i):
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            for _ in range(20):
+                got = _grads(layer, ins[i][:3], ins[i][3], mask)
+                stream.synchronize()
+                if not all(torch.equal(a, b) for a, b in zip(got, want[i])):
+                    wrong.append(i)
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong

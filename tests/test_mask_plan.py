@@ -138,3 +138,51 @@ def test_memory_held_until_the_backward(N, S, D, deterministic):
     assert torch.cuda.memory_allocated() - before - o.numel() * 2 - lse.numel() * 4 <= 4096      # given back, although the output still lives
     torch.cuda.synchronize()
     _lib.device_status()
+
+
+# what else goes with a plan: in-kernel dropout, masks of other types, of two dimensions, that are views, that are not square
+@pytest.mark.parametrize("form", ["dropout", "uint8", "bool, two dimensions", "view", "fewer queries than keys"])
+def test_with_a_plan_as_without(form):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from acctransformer_b200 import _lib, ops
+    from acctransformer_b200.flash_attention.ops.flash_attention.flash_attention_impl import get_flash_attention
+    N, S_q, S_k, D = 64, 1500, 1500, 64
+    if form == "fewer queries than keys":
+        S_q, S_k = 1100, 1800
+    g = torch.Generator(device="cuda").manual_seed(S_k)
+    q, d_o = (torch.randn(1, N, S_q, D, device="cuda", dtype=torch.float16, generator=g) for _ in range(2))
+    k, v = (torch.randn(1, N, S_k, D, device="cuda", dtype=torch.float16, generator=g) for _ in range(2))
+    mask = _documents(S_k, [[400, 900, 1400]])[:, :S_q].half().cuda()
+    given = mask
+    if form == "uint8":
+        given = mask.to(torch.uint8)
+    elif form.startswith("bool"):
+        given = mask[0].bool()
+    elif form == "view":
+        given = torch.nn.functional.pad(mask, (3, 5, 2, 1))[:, 2:-1, 3:-5]
+        assert not given.is_contiguous()
+    kw = dict(keep_prob=0.75, dropout_seed=11, dropout_offset=5) if form == "dropout" else {}
+    scale = 1.0 / math.sqrt(D)
+    xs = [t.clone().requires_grad_() for t in (q, k, v)]
+    o1, lse1 = get_flash_attention(scale=scale)(*xs, given, **kw)
+    g1 = torch.autograd.grad(o1, xs, d_o)
+    o0, lse0 = ops.fa_forward(q, k, v, mask, scale=scale, **kw)
+    g0 = ops.fa_backward(q, k, v, o0, lse0, d_o, mask, scale=scale, **kw)
+    torch.cuda.synchronize()
+    _lib.device_status()
+    for a, b in ((o1, o0), *zip(g1, g0)):      # the bound of _run
+        assert (a.float() - b.float()).abs().max().item() <= 2 * 2.0 ** -11 * b.float().abs().max().item()
+    # and one slice against the oracle
+    h = 5
+    drop, keep = None, 1.0
+    if kw:
+        drop = ops.dropout_mask(1, N, S_q, S_k, 0.75, 11, 5)[:, h:h + 1].cpu().numpy()
+        keep = ref.dropout_threshold(0.75) / 256.0
+    ins = [t[:, h:h + 1].float().cpu().numpy() for t in (q, k, v, d_o)]
+    m = mask.float().cpu().numpy()
+    o_ref, _ = ref.sa_fwd(*ins[:3], attn_mask=m, drop_mask=drop, keep_prob=keep, scale=scale)
+    assert float(np.max(np.abs(o1[:, h:h + 1].detach().float().cpu().numpy() - o_ref))) <= 4e-3     # P and O to 2^-11 of up to 4 / keep
+    for a, b in zip(g1, ref.sa_grad(*ins, attn_mask=m, drop_mask=drop, keep_prob=keep, scale=scale)):
+        # dS and P to 2^-11 per term, sums of up to 1 500 terms of both signs, the result to 2^-11: 1e-2 of the largest
+        assert float(np.max(np.abs(a[:, h:h + 1].float().cpu().numpy() - b))) <= 1e-2 * float(np.max(np.abs(b)))
