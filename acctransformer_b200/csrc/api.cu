@@ -292,6 +292,19 @@ bool plan_applies(const acct_fa_args* a) {
          static_cast<int64_t>(a->B) * a->N * tq * tk >= kPlanMinTilePairs;
 }
 
+// Whether the backward runs on pairs of thread blocks (fa_bwd_pair.cu): long walks without per-element work.  Forward and
+// backward, one block -> pairs: 2 x 32 heads of 128, 8 192 tokens causal 4 452 -> 4 008 us, 8 x 32 heads, 4 096 tokens in row
+// groups of 512 4 845 -> 4 519; 4 x 16 heads, 2 048 tokens with alibi (16 tiles, the line) 391 -> 390, where two tiles to an item
+// leave fewer and less even items.  Documents of 3 000 tokens lost (499 -> 517: short walks, and a Q tile that either tile of
+// a pair needs is walked by both), and so did a band with in-kernel dropout (backward 1 306 -> 1 824).
+constexpr int64_t kPairMinTiles = 16;
+bool bwd_on_pairs(const acct_fa_args* a) {
+  const int64_t tiles_q = (static_cast<int64_t>(a->S_q) + kTile - 1) / kTile, tiles_k = (static_cast<int64_t>(a->S_k) + kTile - 1) / kTile;
+  return a->D > 64 && a->D <= 128 && !(a->flags & (ACCT_FLAG_DETERMINISTIC | ACCT_FLAG_DROPOUT_PHILOX)) && a->dropout_mask == nullptr &&
+         a->mask_kind == ACCT_MASK_NONE && a->prev_block_num >= ACCT_BAND_UNBOUNDED && a->next_block_num >= ACCT_BAND_UNBOUNDED &&
+         a->tri_block % kTile == 0 && tiles_q >= kPairMinTiles && tiles_k >= kPairMinTiles && tiles_k < 65536 && tiles_q < 65536;
+}
+
 ScoreMods make_mods(const acct_fa_args* a, const void* plan = nullptr) {
   ScoreMods m;
   memset(&m.plan, 0, sizeof(m.plan));
@@ -549,6 +562,7 @@ int acct_fa_bwd_planned(const acct_fa_args* a, const acct_fa_bwd_io* g, const in
   float* delta = static_cast<float*>(g->workspace);
   // up to 160 columns one CTA holds dK and dV whole; with an ordered dQ reduction the split-width kernel does it
   const bool mid = a->D > 128 && a->D <= kMidHeadDim && !(a->flags & ACCT_FLAG_DETERMINISTIC);
+  const bool pair = bwd_on_pairs(a);
   const bool wide = a->D > 128;      // the split-width kernel: 64-row Q / dO boxes, 64-row dQ box, 2 counters per tile
   const size_t q_tiles = static_cast<size_t>(a->B) * a->N * ((a->S_q + kTile - 1) / kTile) * (wide ? 2 : 1) + 1;   // + work counter
   const size_t order_bytes = ((q_tiles * 4 + 255) / 256) * 256;
@@ -560,17 +574,17 @@ int acct_fa_bwd_planned(const acct_fa_args* a, const acct_fa_bwd_io* g, const in
 
   BwdParams p;
   memset(&p, 0, sizeof(p));
-  if ((rc = make_qkv_maps(a, st, &p.map_q, &p.map_k, &p.map_v, wide ? 64 : kTile))) return rc;
+  if ((rc = make_qkv_maps(a, st, &p.map_q, &p.map_k, &p.map_v, wide || pair ? 64 : kTile))) return rc;
   TensorDesc4 t;
   t.dtype = a->dtype; t.ptr = g->d_o;
   t.dims[0] = a->D; t.dims[1] = a->S_q; t.dims[2] = a->N; t.dims[3] = a->B;
   t.strides[0] = st_do[2]; t.strides[1] = st_do[1]; t.strides[2] = st_do[0];
-  if ((rc = make_tmap_4d(&p.map_do, t, wide ? 64 : kTile))) return rc;
+  if ((rc = make_tmap_4d(&p.map_do, t, wide || pair ? 64 : kTile))) return rc;
   // the fp32 dQ accumulator, packed [B,N,S_q,D]: target of the kernel's TMA reduce-add
   t.dtype = ACCT_F32; t.ptr = dq_acc;
   t.strides[0] = a->D; t.strides[1] = static_cast<int64_t>(a->S_q) * a->D;
   t.strides[2] = static_cast<int64_t>(a->N) * a->S_q * a->D;
-  if ((rc = make_tmap_4d(&p.map_dq, t, mid ? 32 : wide ? 64 : kTile))) return rc;
+  if ((rc = make_tmap_4d(&p.map_dq, t, mid ? 32 : wide || pair ? 64 : kTile))) return rc;
   if ((!wide || mid) && !(a->flags & ACCT_FLAG_GRAD_F32)) {
     // 16-bit dk, dv, packed [B,N_kv,S_k,D]: the kernel writes a tile through shared memory and one TMA store
     const int n_kv = kv_heads(a);
@@ -608,7 +622,10 @@ int acct_fa_bwd_planned(const acct_fa_args* a, const acct_fa_bwd_io* g, const in
     e = cudaEventRecord(static_cast<cudaEvent_t>(g->ev_kernel_start), s);
     if (e != cudaSuccess) return fail_cuda(e, "recording the kernel-start event");
   }
-  e = mid ? launch_fa_bwd_mid(p, bf16, s) : wide ? launch_fa_bwd_wide(p, bf16, s) : launch_fa_bwd(p, bf16, dev->info.sm_count, s);
+  e = mid    ? launch_fa_bwd_mid(p, bf16, s)
+      : wide ? launch_fa_bwd_wide(p, bf16, s)
+      : pair ? launch_fa_bwd_pair(p, bf16, dev->info.sm_count, s)
+             : launch_fa_bwd(p, bf16, dev->info.sm_count, s);
   if (e != cudaSuccess) return fail_cuda(e, "launching the backward kernel");
   if (g->ev_kernel_stop != nullptr) {
     e = cudaEventRecord(static_cast<cudaEvent_t>(g->ev_kernel_stop), s);

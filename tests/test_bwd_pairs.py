@@ -1,0 +1,58 @@
+"""Backward at head_dim in (64, 128] on pairs of thread blocks: two K/V tiles per work item, products over both.
+
+Checked against the one-block kernel, which the deterministic flag selects: the two share the formulas, round P and dS to 16
+bits and sum in fp32, so a gradient differs by the rounding of its 16 bits and by fp32 sums in another order.
+"""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# (B, N, N_kv, S_q, S_k, D, options): the fewest tiles that take this path (16), pairs with an absent second tile (17), a last
+# Q tile of one row, of one block's rows (64) and of one more, fewer and more items than pairs of SMs, query heads in a group
+CASES = [
+    (1, 1, 1, 1921, 1921, 72, {}),
+    (1, 2, 2, 1984, 2100, 128, {"causal": True}),
+    (2, 2, 1, 2049, 2048, 96, {"causal": True}),
+    (1, 12, 12, 1985, 2177, 128, {}),
+    (2, 20, 5, 2048, 2048, 120, {"causal": True}),
+    (2, 8, 8, 2000, 2300, 128, {"lens": [1, 1333]}),
+    (1, 4, 2, 2048, 2048, 128, {"causal": True, "alibi": True}),
+    (1, 2, 2, 2304, 2304, 128, {"tri_block": 384}),
+]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "-".join(map(str, c[:6])) + "-" + "+".join(c[6]))
+@pytest.mark.parametrize("f32", [False, True])
+def test_against_the_one_block_kernel(case, dtype, f32):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from acctransformer_b200 import _lib, ops
+    B, N, N_kv, S_q, S_k, D, opt = case
+    g = torch.Generator().manual_seed(S_q + S_k + D)
+
+    def rnd(*shape):
+        return torch.randn(*shape, generator=g).to(dtype).cuda()
+    q, d_o, k, v = rnd(B, N, S_q, D), rnd(B, N, S_q, D), rnd(B, N_kv, S_k, D), rnd(B, N_kv, S_k, D)
+    kw = {x: opt[x] for x in ("causal", "tri_block") if x in opt}
+    if "lens" in opt:
+        kw["seq_lens"] = torch.tensor(opt["lens"], dtype=torch.int32).cuda()
+    if "alibi" in opt:
+        kw["alibi"] = (-0.1 * torch.arange(S_k).float()).expand(B, N, 1, S_k).to(dtype).cuda()
+    scale = 1.0 / math.sqrt(D)
+    o, lse = ops.fa_forward(q, k, v, scale=scale, **kw)
+    want = ops.fa_backward(q, k, v, o, lse, d_o, scale=scale, grads_fp32=f32, deterministic=True, **kw)
+    # a P or dS that rounds to its other 16-bit neighbour moves a gradient by 2^-11 (fp16) / 2^-8 (bf16) of one term;
+    # the terms are of the size of the largest gradient at most
+    unit = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for _ in range(3):                # (the blocks of a pair meet in another order each time)
+        got = ops.fa_backward(q, k, v, o, lse, d_o, scale=scale, grads_fp32=f32, **kw)
+        torch.cuda.synchronize()
+        _lib.device_status()
+        for a, b in zip(got, want):
+            assert torch.isfinite(a).all()
+            err = (a.float() - b.float()).abs().max().item()
+            assert err <= 2 * unit * max(b.float().abs().max().item(), 1e-3)
