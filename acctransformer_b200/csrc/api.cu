@@ -294,14 +294,14 @@ bool plan_applies(const acct_fa_args* a) {
 
 // Whether the backward runs on pairs of thread blocks (fa_bwd_pair.cu): long walks without per-element work.  Forward and
 // backward, one block -> pairs: 2 x 32 heads of 128, 8 192 tokens causal 4 452 -> 4 008 us, 8 x 32 heads, 4 096 tokens in row
-// groups of 512 4 845 -> 4 519; 4 x 16 heads, 2 048 tokens with alibi (16 tiles, the line) 391 -> 390, where two tiles to an item
-// leave fewer and less even items.  Documents of 3 000 tokens lost (499 -> 517: short walks, and a Q tile that either tile of
+// groups of 512 4 845 -> 4 519; 4 x 16 heads, 2 048 tokens (16 tiles, the line) backward 278 -> 265, but with
+// alibi 377 -> 383 in all.  Documents of 3 000 tokens lost (499 -> 517: short walks, and a Q tile that either tile of
 // a pair needs is walked by both), and so did a band with in-kernel dropout (backward 1 306 -> 1 824).
 constexpr int64_t kPairMinTiles = 16;
 bool bwd_on_pairs(const acct_fa_args* a) {
   const int64_t tiles_q = (static_cast<int64_t>(a->S_q) + kTile - 1) / kTile, tiles_k = (static_cast<int64_t>(a->S_k) + kTile - 1) / kTile;
   return a->D > 64 && a->D <= 128 && !(a->flags & (ACCT_FLAG_DETERMINISTIC | ACCT_FLAG_DROPOUT_PHILOX)) && a->dropout_mask == nullptr &&
-         a->mask_kind == ACCT_MASK_NONE && a->prev_block_num >= ACCT_BAND_UNBOUNDED && a->next_block_num >= ACCT_BAND_UNBOUNDED &&
+         a->mask_kind == ACCT_MASK_NONE && a->alibi == nullptr && a->alibi_slopes == nullptr && a->prev_block_num >= ACCT_BAND_UNBOUNDED && a->next_block_num >= ACCT_BAND_UNBOUNDED &&
          a->tri_block % kTile == 0 && tiles_q >= kPairMinTiles && tiles_k >= kPairMinTiles && tiles_k < 65536 && tiles_q < 65536;
 }
 
