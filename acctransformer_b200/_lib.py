@@ -16,6 +16,7 @@ MASK_NONE, MASK_FULL, MASK_TILE128 = 0, 1, 2
 BAND_UNBOUNDED = 65536
 ABI_VERSION = 3       # ACCT_ABI_VERSION of include/acct_b200.h these mirrors were written for
 FLAG_GRAD_F32, FLAG_DETERMINISTIC, FLAG_DROPOUT_PHILOX = 1, 2, 4
+BWD_ONE_BLOCK, BWD_PAIR, BWD_MID, BWD_WIDE = 0, 1, 2, 3
 DECODE_STATIC_SCRATCH_BYTES = 8 * 1024 * 1024
 
 ERR_NAMES = {
@@ -25,7 +26,7 @@ ERR_NAMES = {
 }
 
 EXPORTS = [
-    "acct_fa_fwd", "acct_fa_bwd_workspace_bytes", "acct_fa_bwd", "acct_fa_bwd_strided", "acct_mask_plan_bytes",
+    "acct_fa_fwd", "acct_fa_bwd_workspace_bytes", "acct_fa_bwd_kernel", "acct_fa_bwd", "acct_fa_bwd_strided", "acct_mask_plan_bytes",
     "acct_mask_plan", "acct_mask_plan_norms", "acct_fa_fwd_planned", "acct_fa_bwd_planned", "acct_infer_prefill",
     "acct_infer_decode_workspace_bytes", "acct_infer_decode", "acct_infer_decode_static", "acct_device_status",
     "acct_last_error", "acct_abi_version",
@@ -129,6 +130,8 @@ def load():
     lib.acct_fa_fwd.restype = C.c_int
     lib.acct_fa_bwd_workspace_bytes.argtypes = [C.POINTER(FaArgs)]
     lib.acct_fa_bwd_workspace_bytes.restype = C.c_size_t
+    lib.acct_fa_bwd_kernel.argtypes = [C.POINTER(FaArgs)]
+    lib.acct_fa_bwd_kernel.restype = C.c_int
     lib.acct_fa_bwd.argtypes = [C.POINTER(FaArgs), C.POINTER(FaBwdIO), C.c_void_p]
     lib.acct_fa_bwd.restype = C.c_int
     lib.acct_infer_prefill.argtypes = [C.POINTER(InferArgs), C.c_void_p]

@@ -296,13 +296,23 @@ bool plan_applies(const acct_fa_args* a) {
 // backward, one block -> pairs: 2 x 32 heads of 128, 8 192 tokens causal 4 452 -> 4 008 us, 8 x 32 heads, 4 096 tokens in row
 // groups of 512 4 845 -> 4 519; 4 x 16 heads, 2 048 tokens (16 tiles, the line) backward 278 -> 265, but with
 // alibi 377 -> 383 in all.  Documents of 3 000 tokens lost (499 -> 517: short walks, and a Q tile that either tile of
-// a pair needs is walked by both), and so did a band with in-kernel dropout (backward 1 306 -> 1 824).
+// a pair needs is walked by both), and so did a band with in-kernel dropout (backward 1 306 -> 1 824).  Valid lengths keep
+// one block: they are known on the GPU only, half of a pair idles where one ends in its first tile (2 x 64 heads, 2 048 keys
+// of which 128 valid: backward call 220 -> 256 us, 384: 290 -> 312, 1 024: 410 -> 373), and a product over both tiles must
+// not see keys that do not exist.
 constexpr int64_t kPairMinTiles = 16;
 bool bwd_on_pairs(const acct_fa_args* a) {
   const int64_t tiles_q = (static_cast<int64_t>(a->S_q) + kTile - 1) / kTile, tiles_k = (static_cast<int64_t>(a->S_k) + kTile - 1) / kTile;
   return a->D > 64 && a->D <= 128 && !(a->flags & (ACCT_FLAG_DETERMINISTIC | ACCT_FLAG_DROPOUT_PHILOX)) && a->dropout_mask == nullptr &&
-         a->mask_kind == ACCT_MASK_NONE && a->alibi == nullptr && a->alibi_slopes == nullptr && a->prev_block_num >= ACCT_BAND_UNBOUNDED && a->next_block_num >= ACCT_BAND_UNBOUNDED &&
+         a->mask_kind == ACCT_MASK_NONE && a->alibi == nullptr && a->alibi_slopes == nullptr && a->seq_lens == nullptr &&
+         a->prev_block_num >= ACCT_BAND_UNBOUNDED && a->next_block_num >= ACCT_BAND_UNBOUNDED &&
          a->tri_block % kTile == 0 && tiles_q >= kPairMinTiles && tiles_k >= kPairMinTiles && tiles_k < 65536 && tiles_q < 65536;
+}
+
+// up to 160 columns one CTA holds dK and dV whole; with an ordered dQ reduction the split-width kernel does it
+int bwd_kernel(const acct_fa_args* a) {
+  if (a->D > 128) return a->D <= kMidHeadDim && !(a->flags & ACCT_FLAG_DETERMINISTIC) ? ACCT_BWD_MID : ACCT_BWD_WIDE;
+  return bwd_on_pairs(a) ? ACCT_BWD_PAIR : ACCT_BWD_ONE_BLOCK;
 }
 
 ScoreMods make_mods(const acct_fa_args* a, const void* plan = nullptr) {
@@ -527,6 +537,8 @@ size_t acct_fa_bwd_workspace_bytes(const acct_fa_args* a) {
   return ((rows * 4 + 255) / 256) * 256 + ((q_tiles * 4 + 255) / 256) * 256 + acc;
 }
 
+int acct_fa_bwd_kernel(const acct_fa_args* a) { return a != nullptr ? bwd_kernel(a) : -1; }
+
 int acct_fa_bwd(const acct_fa_args* a, const acct_fa_bwd_io* g, void* stream) {
   return acct_fa_bwd_planned(a, g, nullptr, nullptr, nullptr, stream);
 }
@@ -560,9 +572,8 @@ int acct_fa_bwd_planned(const acct_fa_args* a, const acct_fa_bwd_io* g, const in
   const bool bf16 = a->dtype == ACCT_BF16;
   const size_t rows = static_cast<size_t>(a->B) * a->N * a->S_q;
   float* delta = static_cast<float*>(g->workspace);
-  // up to 160 columns one CTA holds dK and dV whole; with an ordered dQ reduction the split-width kernel does it
-  const bool mid = a->D > 128 && a->D <= kMidHeadDim && !(a->flags & ACCT_FLAG_DETERMINISTIC);
-  const bool pair = bwd_on_pairs(a);
+  const int kernel = bwd_kernel(a);
+  const bool mid = kernel == ACCT_BWD_MID, pair = kernel == ACCT_BWD_PAIR;
   const bool wide = a->D > 128;      // the split-width kernel: 64-row Q / dO boxes, 64-row dQ box, 2 counters per tile
   const size_t q_tiles = static_cast<size_t>(a->B) * a->N * ((a->S_q + kTile - 1) / kTile) * (wide ? 2 : 1) + 1;   // + work counter
   const size_t order_bytes = ((q_tiles * 4 + 255) / 256) * 256;

@@ -89,7 +89,7 @@ struct PairShared {
 constexpr size_t kPSmem = 3 * kPTile + 4 * kPHalf + kPTile + 2 * kPHalf + sizeof(PairShared);
 static_assert(kPSmem <= 232448, "shared memory of a thread block");
 
-// Q tiles i that need K/V tile j (decode_item of the one-block kernel, without a band)
+// Q tiles i that need K/V tile j (decode_item of the one-block kernel, without a band or valid lengths)
 __device__ __forceinline__ void q_range(const BwdParams& p, int j, int& lo, int& hi) {
   const ScoreMods& mods = p.mods;
   lo = 0;
@@ -98,24 +98,17 @@ __device__ __forceinline__ void q_range(const BwdParams& p, int j, int& lo, int&
   if (mods.tri_block > 0) lo = max(lo, (((j * kTile) / mods.tri_block) * mods.tri_block) / kTile);
 }
 
-__device__ __forceinline__ int kv_length(const BwdParams& p, int b) {
-  return p.mods.seq_lens != nullptr ? min(p.S_k, max(0, p.mods.seq_lens[b])) : p.S_k;
-}
-
 // Item number -> item: inside a group of kPUnitGroup slices the heaviest pairs of all slices first (decode_item of the
 // one-block kernel).
 __device__ __forceinline__ PairItem decode_pair(const BwdParams& p, int w) {
   PairItem it;
   it.w = w;
-  const int n_kv = p.N / p.kv_group;
   const int n_j = (p.S_k + kTile - 1) / kTile, n_jp = (n_j + 1) / 2;
-  const int n_units = p.B * n_kv;
+  const int n_units = p.B * (p.N / p.kv_group);
   const int per_group = n_jp * kPUnitGroup;
   const int grp = w / per_group, within = w % per_group;
   const int g_units = min(kPUnitGroup, n_units - grp * kPUnitGroup);
   const int jp = within / g_units, bh_kv = grp * kPUnitGroup + within % g_units;
-  const int b = bh_kv / n_kv;
-  const int kv_len = kv_length(p, b);
   int lo, hi;
   q_range(p, 2 * jp, lo, hi);
   if (2 * jp + 1 < n_j) {
@@ -127,7 +120,6 @@ __device__ __forceinline__ PairItem decode_pair(const BwdParams& p, int w) {
       hi = max(hi, hi1);
     }
   }
-  if (2 * jp * kTile >= kv_len) hi = lo - 1;
   const int n_per = max(0, hi - lo + 1);
   it.bh_kv = static_cast<uint16_t>(bh_kv);
   it.jp = static_cast<uint16_t>(jp);
@@ -556,10 +548,8 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
     // what an item needs from global memory before its first step is requested before the write-out of the item before it
     float pre_lse = 0.f, pre_dlt = 0.f;
     uint32_t pre_bias = 0u;
-    int pre_len = 0;
     auto request_first = [&](const PairItem& t) {
       const int b = t.bh_kv / n_kv, h0 = (t.bh_kv % n_kv) * p.kv_group;
-      pre_len = kv_length(p, b);
       if (t.n_iter <= 0) return;
       if (hf == 0) {
         const int64_t idx = (static_cast<int64_t>(b) * p.N + h0) * p.S_q + min(t.i_lo * kTile + r, p.S_q - 1);
@@ -589,11 +579,10 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
       const int n_per = it.n_per, n_iter = it.n_iter;
       const int b = it.bh_kv / n_kv, h_kv = it.bh_kv % n_kv;
       const int j = 2 * it.jp + rank;
-      const int kv_len = pre_len;
       // Q tile and query head of the step, and of the next one (counted on: divisions here took some 600 clk a step)
       int i = n_iter > 0 ? it.i_lo : 0, h = h_kv * p.kv_group, m1 = 0;
       const int kv_idx = j * kTile + r;
-      const bool kv_ok = kv_idx < kv_len;
+      const bool kv_ok = kv_idx < p.S_k;
       int own_lo, own_hi;           // Q tiles that need this block's tile; at the others of the item it has no part
       q_range(p, j, own_lo, own_hi);
       // alibi term of this key row in log2 units for query head h; -inf removes a key row that does not exist

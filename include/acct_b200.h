@@ -214,6 +214,14 @@ ACCT_API int acct_fa_fwd(const acct_fa_args* a, void* stream);
  * (flash_attention_bwd.py:55-57); here the library zero-fills its own accumulator on `stream`. */
 ACCT_API size_t acct_fa_bwd_workspace_bytes(const acct_fa_args* a);
 
+/* Which kernel a backward call with `a` runs: a function of the sizes, the flags and of which operands are given, which it
+ * does not read.  -1 for NULL. */
+#define ACCT_BWD_ONE_BLOCK 0 /* head_dim <= 128: a thread block per K/V tile */
+#define ACCT_BWD_PAIR 1      /* the same on pairs of thread blocks and K/V tiles, where that is faster */
+#define ACCT_BWD_MID 2       /* head_dim in (128, 160] */
+#define ACCT_BWD_WIDE 3      /* head_dim above that, and in (128, 160] with an ordered dQ */
+ACCT_API int acct_fa_bwd_kernel(const acct_fa_args* a);
+
 /* Backward: reads q,k,v,o,lse,d_o (+ the same mask/dropout/alibi/band arguments as the forward). */
 ACCT_API int acct_fa_bwd(const acct_fa_args* a, const acct_fa_bwd_io* g, void* stream);
 

@@ -233,3 +233,15 @@ int main(int argc, char** argv) {
     assert "null tensors -> 1" in out
     ws_line = [ln for ln in out.splitlines() if ln.startswith("workspace bytes")][0]
     assert int(ws_line.split()[-1]) >= 1 * 2 * 256 * 64 * 4     # at least the fp32 dQ accumulator
+
+
+def test_backward_kernel_of_a_call(lib):
+    """acct_fa_bwd_kernel: pairs of thread blocks only for calls whose sizes say that they are faster there."""
+    def kernel(**kw):
+        a = _args(**{"B": 2, "N": 8, "S_q": 4096, "S_k": 4096, "D": 128, "causal": 1, **kw})
+        return lib.acct_fa_bwd_kernel(C.byref(a))
+    assert kernel() == _lib.BWD_PAIR
+    assert kernel(seq_lens=64) == _lib.BWD_ONE_BLOCK      # (device memory, not read: the lengths are not known here)
+    assert kernel(flags=_lib.FLAG_DETERMINISTIC) == _lib.BWD_ONE_BLOCK
+    assert kernel(D=160) == _lib.BWD_MID and kernel(D=256) == _lib.BWD_WIDE
+    assert lib.acct_fa_bwd_kernel(None) == -1

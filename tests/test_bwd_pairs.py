@@ -56,3 +56,29 @@ def test_against_the_one_block_kernel(case, dtype, f32):
             assert torch.isfinite(a).all()
             err = (a.float() - b.float()).abs().max().item()
             assert err <= 2 * unit * max(b.float().abs().max().item(), 1e-3)
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("f32", [False, True])
+@pytest.mark.parametrize("fill", [float("nan"), float("inf")])
+def test_keys_past_the_valid_length_do_not_exist(causal, f32, fill):
+    """What a padded buffer holds behind the valid keys reaches no gradient, wherever in a pair of tiles the length ends."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from acctransformer_b200 import ops
+    lens = [0, 128, 384, 2176]
+    g = torch.Generator().manual_seed(5)
+    q, k, v, d_o = (torch.randn(4, 2, 2304, 128, generator=g).half().cuda() for _ in range(4))
+    kw = {"scale": 128 ** -0.5, "causal": causal, "seq_lens": torch.tensor(lens, dtype=torch.int32).cuda()}
+    o, lse = ops.fa_forward(q, k, v, **kw)
+    want = ops.fa_backward(q, k, v, o, lse, d_o, grads_fp32=f32, deterministic=True, **kw)
+    for b, n in enumerate(lens):
+        k[b, :, n:] = v[b, :, n:] = fill
+    got = ops.fa_backward(q, k, v, o, lse, d_o, grads_fp32=f32, **kw)
+    for a, b in zip(got[1:], want[1:]):      # (the sums behind dK and dV have a fixed order)
+        assert torch.equal(a, b)
+        for i, n in enumerate(lens):
+            assert not a[i, :, n:].any()
+    # dQ: fp32 sums of up to 17 tiles in another order, rounded to 16 bits unless f32
+    bound = (2.0 ** -18 if f32 else 2.0 ** -10) * want[0].float().abs().amax()
+    assert (got[0].float() - want[0].float()).abs().amax() <= bound
