@@ -15,6 +15,11 @@
 // 384 KB and 32 KB of dQ per block.  A block of rank r keeps, of Q and dO: rows [64r, 64r+64) of the tile (for S^T, dP^T) and
 // columns [64r, 64r+64) (for dK, dV), each with one buffer that is refilled as soon as its product has finished.
 //
+// The first Q tiles of a head may need the first K/V tile alone (under a causal mask one, at the end of a row group several;
+// all of them where there is no second tile).  In those steps the second tile has no part in any product's result: dQ
+// contracts over the first 128 keys, and dV and dK write the first block's rows.  That its P and dS are 0 there would not do:
+// 0 times a NaN or infinity of a key or query that do not see one another is NaN.
+//
 // Tensor memory (512 columns): X = S^T | Y = dP^T | dK | dV, 128 each.  P^T goes over columns 0-31 and 96-127 of X (each half
 // of the compute warps over its own), dS^T likewise in Y; dQ (64 columns of a block: its 64 rows, columns 0-63 in lanes 0-63,
 // columns 64-127 in lanes 64-127) takes columns 32-95 of X, which are free from when S^T is in registers until the
@@ -60,6 +65,7 @@ struct PairItem {
   int w;                         // its number; >= the number of items: none is left
   int n_iter;                    // steps: Q tiles x query heads of the group
   uint16_t bh_kv, jp, i_lo, n_per;   // slice, pair of K/V tiles, first Q tile, Q tiles per query head
+  uint16_t n_first;              // how many of those, from the first on, need the first K/V tile alone
 };
 
 struct PairShared {
@@ -111,16 +117,11 @@ __device__ __forceinline__ PairItem decode_pair(const BwdParams& p, int w) {
   const int jp = within / g_units, bh_kv = grp * kPUnitGroup + within % g_units;
   int lo, hi;
   q_range(p, 2 * jp, lo, hi);
-  if (2 * jp + 1 < n_j) {
-    int lo1, hi1;
-    q_range(p, 2 * jp + 1, lo1, hi1);
-    if (lo1 <= hi1) {
-      if (lo > hi) { lo = lo1; hi = hi1; }
-      lo = min(lo, lo1);
-      hi = max(hi, hi1);
-    }
-  }
   const int n_per = max(0, hi - lo + 1);
+  // (the second tile needs no Q tile that the first does not, and the same last one)
+  int lo1 = hi + 1, hi1;
+  if (2 * jp + 1 < n_j) q_range(p, 2 * jp + 1, lo1, hi1);
+  it.n_first = static_cast<uint16_t>(min(n_per, max(0, lo1 - lo)));
   it.bh_kv = static_cast<uint16_t>(bh_kv);
   it.jp = static_cast<uint16_t>(jp);
   it.i_lo = static_cast<uint16_t>(n_per > 0 ? lo : 0);
@@ -270,7 +271,7 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
           }
           PairItem it;
           if (w < total_items) it = decode_pair(p, w);
-          else { it.w = total_items; it.n_iter = 0; it.bh_kv = it.jp = it.i_lo = it.n_per = 0; }
+          else { it.w = total_items; it.n_iter = 0; it.bh_kv = it.jp = it.i_lo = it.n_per = it.n_first = 0; }
           sh.item[slot] = it;
           mbar_arrive(&sh.item_full[slot]);
           return it;
@@ -358,6 +359,16 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
       };
       // queries 16 kk .. + 15 of P^T / dS^T: over columns 0-31 for the first 64 queries, 96-127 for the others
       auto packed_col = [](int kk) { return static_cast<uint32_t>(kk < 4 ? kk * 8 : 64 + kk * 8); };
+      // queries 16 kk .. + 15 of dV or dK += (P^T or dS^T) (dO or Q), of the blocks that take part in the step.  acc0, acc1: the
+      // block's accumulator holds the sum of earlier steps
+      auto gradient = [&](uint32_t col, uint32_t col_a, uint32_t bb, int kk, bool both, bool acc0, bool acc1) {
+        const uint32_t d = tmem + col, a = tmem + col_a + packed_col(kk), b_lo = bb + kk * 128u;
+        if (both && (acc0 == acc1 || kk > 0)) umma_pair_ts(d, a, b_lo, mn_hi, idesc_kv, acc0 || kk > 0);
+        else {
+          umma_pair_ts_one(0, d, a, b_lo, mn_hi, idesc_kv, acc0 || kk > 0);
+          if (both) umma_pair_ts_one(1, d, a, b_lo, mn_hi, idesc_kv, acc1 || kk > 0);
+        }
+      };
 
       int g0 = 0, live = 0;
       for (int k = 0;; ++k) {
@@ -369,9 +380,12 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
         scores(kColX, kK, kQ, &sh.st_full);
         mbar_wait(&sh.dok_full, g0 & 1, abort_flag, p.status, DEV_TIMEOUT_TMA);
         scores(kColY, kV, kDO, &sh.dp_full);
-        for (int n = 0; n < it.n_iter; ++n) {
+        bool acc1 = false;
+        for (int n = 0, m = 0; n < it.n_iter; ++n) {
           const int g = g0 + n;
           const bool more = n + 1 < it.n_iter;
+          const bool both = m >= it.n_first;
+          if (++m == it.n_per) m = 0;
           // dV += P^T dO, in two parts as P^T arrives
           mbar_wait(&sh.dom_full, g & 1, abort_flag, p.status, DEV_TIMEOUT_TMA);
           if (n == 0 && live > 0) mbar_wait(&sh.acc_free, (live - 1) & 1, abort_flag, p.status, DEV_TIMEOUT_SYNC);
@@ -383,7 +397,7 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
 #pragma unroll
               for (int u = 0; u < 4; ++u) {
                 const int kk = (u >> 1) * 4 + part * 2 + (u & 1);
-                umma_pair_ts(tmem + kColDV, tmem + kColX + packed_col(kk), mDO + kk * 128u, mn_hi, idesc_kv, n > 0 || kk > 0);
+                gradient(kColDV, kColX, mDO, kk, both, n > 0, acc1);
               }
             }
           }
@@ -399,9 +413,9 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
           tc_fence_after_sync();
           if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk)
-              umma_pair_ts(tmem + kColDK, tmem + kColY + packed_col(kk), mQ + kk * 128u, mn_hi, idesc_kv, n > 0 || kk > 0);
+            for (int kk = 0; kk < 8; ++kk) gradient(kColDK, kColY, mQ, kk, both, n > 0, acc1);
           }
+          acc1 = acc1 || both;
           // dP^T of the next tile behind it
           if (more) {
             mbar_wait(&sh.dok_full, (g + 1) & 1, abort_flag, p.status, DEV_TIMEOUT_TMA);
@@ -418,7 +432,7 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
           if (elect_one()) {
 #pragma unroll
             for (int kk = 0; kk < 16; ++kk)
-              umma_pair_ss(tmem + kColX + kColDQ, mDS + kk * 128u, mn_hi, mKm + kk * 128u, mn_hi, idesc_dq, kk > 0);
+              if (kk < 8 || both) umma_pair_ss(tmem + kColX + kColDQ, mDS + kk * 128u, mn_hi, mKm + kk * 128u, mn_hi, idesc_dq, kk > 0);
             umma_commit_pair(&sh.dq_full);
           }
         }
@@ -489,6 +503,7 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
       // dV of the item (16-bit gradients) through the staging area, 64 columns at a time, while the compute warps write dK.
       // Thread t owns key row t here.
       const int j = 2 * it.jp + rank;
+      const bool summed = it.n_iter > 0 && (rank == 0 || it.n_first < it.n_per);
       if (!p.grads_f32) {
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
@@ -497,7 +512,7 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
             named_barrier(3, kTile);
           }
           uint32_t dv[32];
-          if (it.n_iter > 0) { tmem_ld32(tmem + lane_base + kColDV + c * 32, dv); tmem_wait_ld(); }
+          if (summed) { tmem_ld32(tmem + lane_base + kColDV + c * 32, dv); tmem_wait_ld(); }
           else {
 #pragma unroll
             for (int e = 0; e < 32; ++e) dv[e] = 0u;
@@ -583,8 +598,6 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
       int i = n_iter > 0 ? it.i_lo : 0, h = h_kv * p.kv_group, m1 = 0;
       const int kv_idx = j * kTile + r;
       const bool kv_ok = kv_idx < p.S_k;
-      int own_lo, own_hi;           // Q tiles that need this block's tile; at the others of the item it has no part
-      q_range(p, j, own_lo, own_hi);
       // alibi term of this key row in log2 units for query head h; -inf removes a key row that does not exist
       auto bias_of = [&](int h) {
         float v = kNegInf;
@@ -623,9 +636,7 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
         }
         const float* nlse2 = sh.nlse2[g & 1];
         const float* ndlt = sh.ndelta[g & 1];
-        const bool absent = i < own_lo || i > own_hi;
-        const float tile_bias = absent ? kNegInf : bias;
-        const uint64_t bias2 = f2_pack(tile_bias, tile_bias);
+        const uint64_t bias2 = f2_pack(bias, bias);
         const bool diag = mods.causal && (q_base < j * kTile + kTile - 1);
 
         // ---- P part
@@ -725,6 +736,7 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
       }
 
       // write-out of dK (scaled) and, with fp32 gradients, dV; each half writes its half of head_dim
+      const bool summed = n_iter > 0 && (rank == 0 || it.n_first < n_per);      // (else nothing has been written there)
       if (n_iter > 0) mbar_wait(&sh.dq_full, (g0 + n_iter - 1) & 1, abort_flag, p.status, DEV_TIMEOUT_MMA);
       tc_fence_after_sync();
       if (!next_known) {      // (an item without steps)
@@ -741,7 +753,7 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
         for (int cq = 0; cq < 2; ++cq) {
           const int c = hf * 2 + cq;
           uint32_t v[32];
-          if (n_iter > 0) { tmem_ld32(tmem + lane_base + kColDK + c * 32, v); tmem_wait_ld(); }
+          if (summed) { tmem_ld32(tmem + lane_base + kColDK + c * 32, v); tmem_wait_ld(); }
           else {
 #pragma unroll
             for (int e = 0; e < 32; ++e) v[e] = 0u;
@@ -778,7 +790,7 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
           for (int cq = 0; cq < 2; ++cq) {
             const int c = hf * 2 + cq;
             uint32_t v[32];
-            if (n_iter > 0) { tmem_ld32(t_src + c * 32, v); tmem_wait_ld(); }
+            if (summed) { tmem_ld32(t_src + c * 32, v); tmem_wait_ld(); }
             else {
 #pragma unroll
               for (int e = 0; e < 32; ++e) v[e] = 0u;

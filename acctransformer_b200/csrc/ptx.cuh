@@ -458,6 +458,18 @@ __device__ __forceinline__ void umma_pair_ts(uint32_t d_tmem, uint32_t a_tmem, u
       ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(acc)
       : "memory");
 }
+// umma_pair_ts that writes one block's rows of D only: the other block's lanes are disabled
+__device__ __forceinline__ void umma_pair_ts_one(uint32_t block, uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi,
+                                                 uint32_t idesc, bool accumulate) {
+  uint32_t acc = accumulate ? 1u : 0u;
+  const uint32_t off0 = block == 0u ? 0u : 0xffffffffu, off1 = ~off0;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\tsetp.ne.b32 p, %5, 0;\n\t"
+      "mov.b64 db, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], db, %4, {%6, %6, %6, %6, %7, %7, %7, %7}, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(acc), "r"(off0), "r"(off1)
+      : "memory");
+}
 // completes `bar` in both blocks of the pair
 __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
   asm volatile(

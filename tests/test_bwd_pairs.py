@@ -82,3 +82,36 @@ def test_keys_past_the_valid_length_do_not_exist(causal, f32, fill):
     # dQ: fp32 sums of up to 17 tiles in another order, rounded to 16 bits unless f32
     bound = (2.0 ** -18 if f32 else 2.0 ** -10) * want[0].float().abs().amax()
     assert (got[0].float() - want[0].float()).abs().amax() <= bound
+
+
+@pytest.mark.parametrize("S_q, S_k, opt", [
+    (2304, 2304, {"causal": True}),                         # the first Q tile of a pair needs its first K/V tile alone
+    (2176, 2304, {"causal": True}),                         # and no Q tile needs the last K/V tile
+    (2176, 2176, {}),                                       # a pair without a second tile
+    (2304, 2304, {"tri_block": 384}),                       # a pair across the end of a row group
+    (2304, 2304, {"tri_block": 384, "causal": True}),
+    (2100, 2300, {"tri_block": 128, "causal": True}),
+])
+@pytest.mark.parametrize("where", ["q", "k", "v", "d_o"])
+@pytest.mark.parametrize("f32", [False, True])
+def test_what_is_not_finite_stays_with_the_tiles_that_see_it(S_q, S_k, opt, where, f32):
+    """NaN and infinity reach the gradients that they reach on the one-block kernel, and no others."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from acctransformer_b200 import ops
+    g = torch.Generator().manual_seed(S_q + S_k)
+    t = {n: torch.randn(1, h, s, 128, generator=g).half().cuda() for n, h, s in
+         (("q", 2, S_q), ("k", 1, S_k), ("v", 1, S_k), ("d_o", 2, S_q))}
+    kw = {"scale": 128 ** -0.5, **opt}
+    for row, value in ((5, float("nan")), (200, float("inf")), (450, float("nan")), (S_q - 3, float("inf"))):
+        x = {n: u.clone() for n, u in t.items()}
+        x[where][0, 0, row] = value
+        o, lse = ops.fa_forward(x["q"], x["k"], x["v"], **kw)
+        want = ops.fa_backward(x["q"], x["k"], x["v"], o, lse, x["d_o"], grads_fp32=f32, deterministic=True, **kw)
+        got = ops.fa_backward(x["q"], x["k"], x["v"], o, lse, x["d_o"], grads_fp32=f32, **kw)
+        for a, b in zip(got, want):
+            ok = torch.isfinite(b)
+            assert torch.equal(torch.isfinite(a), ok)
+            # sums of the same fp32 terms in another order, rounded to 16 bits unless f32
+            a, b = a.float()[ok], b.float()[ok]
+            assert a.numel() == 0 or (a - b).abs().amax() <= (2.0 ** -17 if f32 else 2.0 ** -9) * b.abs().amax()
