@@ -57,7 +57,9 @@ constexpr int kPThreads = 512;
 constexpr int kPComputeThreads = 256;
 constexpr int kPDrainWarp0 = 8, kPProducerWarp = 12, kPMmaWarp = 13;     // (warp 13 of rank 1: the relay)
 constexpr int kPUnitGroup = 8;          // (batch, head) slices whose items are interleaved, heaviest tiles first
-constexpr int kPRegsCompute = 176, kPRegsDrain = 104, kPRegsControl = 56;   // 256 x 176 + 128 x 104 + 128 x 56 = 512 x 128
+// 256 x 168 + 128 x 96 + 128 x 80 = 512 x 128.  Backward call, 2 x 32 heads, 8 192 tokens causal: 2 590 us; 176 / 88 / 72 2 639;
+// 176 / 104 / 56, where the MMA warp spills, 2 741.
+constexpr int kPRegsCompute = 168, kPRegsDrain = 96, kPRegsControl = 80;
 constexpr uint32_t kPTile = 32768;      // 128 rows x 128 columns of 16-bit values
 constexpr uint32_t kPHalf = 16384;      // 64 rows x 128 columns, or 128 rows x 64 columns
 
@@ -359,15 +361,17 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
       };
       // queries 16 kk .. + 15 of P^T / dS^T: over columns 0-31 for the first 64 queries, 96-127 for the others
       auto packed_col = [](int kk) { return static_cast<uint32_t>(kk < 4 ? kk * 8 : 64 + kk * 8); };
-      // queries 16 kk .. + 15 of dV or dK += (P^T or dS^T) (dO or Q), of the blocks that take part in the step.  acc0, acc1: the
-      // block's accumulator holds the sum of earlier steps
-      auto gradient = [&](uint32_t col, uint32_t col_a, uint32_t bb, int kk, bool both, bool acc0, bool acc1) {
-        const uint32_t d = tmem + col, a = tmem + col_a + packed_col(kk), b_lo = bb + kk * 128u;
-        if (both && (acc0 == acc1 || kk > 0)) umma_pair_ts(d, a, b_lo, mn_hi, idesc_kv, acc0 || kk > 0);
-        else {
-          umma_pair_ts_one(0, d, a, b_lo, mn_hi, idesc_kv, acc0 || kk > 0);
-          if (both) umma_pair_ts_one(1, d, a, b_lo, mn_hi, idesc_kv, acc1 || kk > 0);
-        }
+      // dV or dK += (P^T or dS^T) (dO or Q) over the queries 16 (4 x + y) .. + 15, x < 2, from <= y < to.  A step in which the
+      // second block has no part, or whose sum starts in one block only, goes through `one_by_one`, out of the way of the others.
+      auto one_by_one = [&](uint32_t d, uint32_t a, uint32_t bb, int from, int to, bool both, bool acc0, bool acc1) {
+#pragma unroll 1
+        for (int x = 0; x < 2; ++x)
+#pragma unroll 1
+          for (int y = from; y < to; ++y) {
+            const int kk = 4 * x + y;
+            umma_pair_ts_one(0, d, a + packed_col(kk), bb + kk * 128u, mn_hi, idesc_kv, acc0 || kk > 0);
+            if (both) umma_pair_ts_one(1, d, a + packed_col(kk), bb + kk * 128u, mn_hi, idesc_kv, acc1 || kk > 0);
+          }
       };
 
       int g0 = 0, live = 0;
@@ -384,7 +388,7 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
         for (int n = 0, m = 0; n < it.n_iter; ++n) {
           const int g = g0 + n;
           const bool more = n + 1 < it.n_iter;
-          const bool both = m >= it.n_first;
+          const bool both = m >= it.n_first, regular = both && acc1 == (n > 0);
           if (++m == it.n_per) m = 0;
           // dV += P^T dO, in two parts as P^T arrives
           mbar_wait(&sh.dom_full, g & 1, abort_flag, p.status, DEV_TIMEOUT_TMA);
@@ -394,10 +398,14 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
             mbar_wait(part == 0 ? &sh.p_half : &sh.p_ready, g & 1, abort_flag, p.status, DEV_TIMEOUT_SYNC);
             tc_fence_after_sync();
             if (elect_one()) {
+              if (regular) {
 #pragma unroll
-              for (int u = 0; u < 4; ++u) {
-                const int kk = (u >> 1) * 4 + part * 2 + (u & 1);
-                gradient(kColDV, kColX, mDO, kk, both, n > 0, acc1);
+                for (int u = 0; u < 4; ++u) {
+                  const int kk = (u >> 1) * 4 + part * 2 + (u & 1);
+                  umma_pair_ts(tmem + kColDV, tmem + kColX + packed_col(kk), mDO + kk * 128u, mn_hi, idesc_kv, n > 0 || kk > 0);
+                }
+              } else {
+                one_by_one(tmem + kColDV, tmem + kColX, mDO, part * 2, part * 2 + 2, both, n > 0, acc1);
               }
             }
           }
@@ -412,8 +420,13 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
           mbar_wait(&sh.ds_tmem, g & 1, abort_flag, p.status, DEV_TIMEOUT_SYNC);
           tc_fence_after_sync();
           if (elect_one()) {
+            if (regular) {
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk) gradient(kColDK, kColY, mQ, kk, both, n > 0, acc1);
+              for (int kk = 0; kk < 8; ++kk)
+                umma_pair_ts(tmem + kColDK, tmem + kColY + packed_col(kk), mQ + kk * 128u, mn_hi, idesc_kv, n > 0 || kk > 0);
+            } else {
+              one_by_one(tmem + kColDK, tmem + kColY, mQ, 0, 4, both, n > 0, acc1);
+            }
           }
           acc1 = acc1 || both;
           // dP^T of the next tile behind it
@@ -431,8 +444,13 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
           tc_fence_after_sync();
           if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < 16; ++kk)
-              if (kk < 8 || both) umma_pair_ss(tmem + kColX + kColDQ, mDS + kk * 128u, mn_hi, mKm + kk * 128u, mn_hi, idesc_dq, kk > 0);
+            for (int kk = 0; kk < 8; ++kk)
+              umma_pair_ss(tmem + kColX + kColDQ, mDS + kk * 128u, mn_hi, mKm + kk * 128u, mn_hi, idesc_dq, kk > 0);
+            if (both) {
+#pragma unroll
+              for (int kk = 8; kk < 16; ++kk)
+                umma_pair_ss(tmem + kColX + kColDQ, mDS + kk * 128u, mn_hi, mKm + kk * 128u, mn_hi, idesc_dq, true);
+            }
             umma_commit_pair(&sh.dq_full);
           }
         }
