@@ -580,7 +580,6 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
     bool ds_stage_busy = false;     // a dK store may still be reading the dS^T areas
     // what an item needs from global memory before its first step is requested before the write-out of the item before it
     float pre_lse = 0.f, pre_dlt = 0.f;
-    uint32_t pre_bias = 0u;
     auto request_first = [&](const PairItem& t) {
       const int b = t.bh_kv / n_kv, h0 = (t.bh_kv % n_kv) * p.kv_group;
       if (t.n_iter <= 0) return;
@@ -588,13 +587,6 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
         const int64_t idx = (static_cast<int64_t>(b) * p.N + h0) * p.S_q + min(t.i_lo * kTile + r, p.S_q - 1);
         pre_lse = p.lse[idx];
         pre_dlt = p.delta[idx];
-      }
-      const int kv = (2 * t.jp + rank) * kTile + r;
-      if (kv < p.S_k) {
-        if (mods.alibi != nullptr)
-          pre_bias = reinterpret_cast<const uint16_t*>(mods.alibi)[(static_cast<int64_t>(b) * p.N + h0) * p.S_k + kv];
-        else if (mods.alibi_slopes != nullptr)
-          pre_bias = __float_as_uint(mods.alibi_slopes[h0]);
       }
     };
     auto park = [&](int g, int q_row, float lse, float dlt) {       // statistics of step g (threads of half 0)
@@ -615,25 +607,8 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
       // Q tile and query head of the step, and of the next one (counted on: divisions here took some 600 clk a step)
       int i = n_iter > 0 ? it.i_lo : 0, h = h_kv * p.kv_group, m1 = 0;
       const int kv_idx = j * kTile + r;
-      const bool kv_ok = kv_idx < p.S_k;
-      // alibi term of this key row in log2 units for query head h; -inf removes a key row that does not exist
-      auto bias_of = [&](int h) {
-        float v = kNegInf;
-        if (kv_ok) {
-          v = 0.f;
-          if (mods.alibi != nullptr) v = load16<BF16>(mods.alibi, (static_cast<int64_t>(b) * p.N + h) * p.S_k + kv_idx) * kLog2e;
-          else if (mods.alibi_slopes != nullptr) v = mods.alibi_slopes[h] * static_cast<float>(kv_idx) * kLog2e;
-        }
-        return v;
-      };
-      float bias = kNegInf;
-      if (kv_ok) {
-        bias = 0.f;
-        if (mods.alibi != nullptr)
-          bias = (BF16 ? __uint_as_float(pre_bias << 16) : __half2float(__ushort_as_half(static_cast<unsigned short>(pre_bias)))) * kLog2e;
-        else if (mods.alibi_slopes != nullptr)
-          bias = __uint_as_float(pre_bias) * static_cast<float>(kv_idx) * kLog2e;
-      }
+      const float bias = kv_idx < p.S_k ? 0.f : kNegInf;       // -inf removes a key row that does not exist
+      const uint64_t bias2 = f2_pack(bias, bias);
       // Statistics go through shared memory, double-buffered by step: parked at the end of the step before (buffer g & 1 was
       // last read for step g - 2, whose dS part every thread finished before dP^T of step g - 1 could be issued).
       if (hf == 0 && n_iter > 0) park(g0, i * kTile + r, pre_lse, pre_dlt);
@@ -654,7 +629,6 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
         }
         const float* nlse2 = sh.nlse2[g & 1];
         const float* ndlt = sh.ndelta[g & 1];
-        const uint64_t bias2 = f2_pack(bias, bias);
         const bool diag = mods.causal && (q_base < j * kTile + kTile - 1);
 
         // ---- P part
@@ -749,7 +723,6 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
           next_known = true;
           if (it_next.w < total_items) request_first(it_next);
         }
-        if (h1 != h && more) bias = bias_of(h1);       // another query head
         i = i1; h = h1;
       }
 
