@@ -300,13 +300,18 @@ bool plan_applies(const acct_fa_args* a) {
 // one block: they are known on the GPU only, half of a pair idles where one ends in its first tile (2 x 64 heads, 2 048 keys
 // of which 128 valid: backward call 220 -> 256 us, 384: 290 -> 312, 1 024: 410 -> 373), and a product over both tiles must
 // not see keys that do not exist.
-constexpr int64_t kPairMinTiles = 16;
+// At head_dim up to 96 the one-block kernel has less of dQ to add, the pair's products are as wide as ever, and the line lies
+// higher.  Backward call, head_dim 80, causal, 16 tiles, 48 heads 159 -> 170 us, 32 x 24 267 -> 273, 56 x 16 482 -> 501,
+// 64 x 32 1 225 -> 1 205, 96 x 8 711 -> 679; dense, 16 x 8 65 -> 66 (head_dim 96: 66 -> 68), 24 x 32 389 -> 373,
+// 48 x 20 886 -> 835.  At 104, causal, 16 x 48 209 -> 196, 64 x 16 934 -> 703.
+constexpr int64_t kPairMinTiles = 16, kPairMinTilesNarrow = 24, kPairMinTilesNarrowPartial = 64;
 bool bwd_on_pairs(const acct_fa_args* a) {
   const int64_t tiles_q = (static_cast<int64_t>(a->S_q) + kTile - 1) / kTile, tiles_k = (static_cast<int64_t>(a->S_k) + kTile - 1) / kTile;
+  const int64_t min_q = a->D > 96 ? kPairMinTiles : a->causal || a->tri_block > 0 ? kPairMinTilesNarrowPartial : kPairMinTilesNarrow;
   return a->D > 64 && a->D <= 128 && !(a->flags & (ACCT_FLAG_DETERMINISTIC | ACCT_FLAG_DROPOUT_PHILOX)) && a->dropout_mask == nullptr &&
          a->mask_kind == ACCT_MASK_NONE && a->alibi == nullptr && a->alibi_slopes == nullptr && a->seq_lens == nullptr &&
          a->prev_block_num >= ACCT_BAND_UNBOUNDED && a->next_block_num >= ACCT_BAND_UNBOUNDED &&
-         a->tri_block % kTile == 0 && tiles_q >= kPairMinTiles && tiles_k >= kPairMinTiles && tiles_k < 65536 && tiles_q < 65536;
+         a->tri_block % kTile == 0 && tiles_q >= min_q && tiles_k >= kPairMinTiles && tiles_k < 65536 && tiles_q < 65536;
 }
 
 // up to 160 columns one CTA holds dK and dV whole; with an ordered dQ reduction the split-width kernel does it

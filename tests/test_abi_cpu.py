@@ -241,6 +241,11 @@ def test_backward_kernel_of_a_call(lib):
         a = _args(**{"B": 2, "N": 8, "S_q": 4096, "S_k": 4096, "D": 128, "causal": 1, **kw})
         return lib.acct_fa_bwd_kernel(C.byref(a))
     assert kernel() == _lib.BWD_PAIR
+    # narrow heads: longer walks
+    for D, causal, tiles in ((104, 1, 16), (96, 0, 24), (96, 1, 64), (72, 1, 64)):
+        for S_q, want in ((tiles * 128 - 127, _lib.BWD_PAIR), ((tiles - 1) * 128, _lib.BWD_ONE_BLOCK)):
+            assert kernel(D=D, causal=causal, S_q=S_q, S_k=2048) == want
+    assert kernel(D=80, causal=0, tri_block=512) == _lib.BWD_ONE_BLOCK
     assert kernel(seq_lens=64) == _lib.BWD_ONE_BLOCK      # (device memory, not read: the lengths are not known here)
     assert kernel(flags=_lib.FLAG_DETERMINISTIC) == _lib.BWD_ONE_BLOCK
     assert kernel(D=160) == _lib.BWD_MID and kernel(D=256) == _lib.BWD_WIDE

@@ -10,12 +10,12 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-# (B, N, N_kv, S_q, S_k, D, options): the fewest tiles that take this path (16), pairs with an absent second tile (17), a last
+# (B, N, N_kv, S_q, S_k, D, options): the fewest tiles that take this path (16, and 24 at head_dim up to 96), pairs with an absent second tile (17), a last
 # Q tile of one row, of one block's rows (64) and of one more, fewer and more items than pairs of SMs, query heads in a group
 CASES = [
-    (1, 1, 1, 1921, 1921, 72, {}),
+    (1, 1, 1, 2945, 1921, 72, {}),
     (1, 2, 2, 1984, 2100, 128, {"causal": True}),
-    (2, 2, 1, 2049, 2048, 96, {"causal": True}),
+    (2, 2, 1, 2049, 2048, 104, {"causal": True}),
     (1, 12, 12, 1985, 2177, 128, {}),
     (2, 20, 5, 2048, 2048, 120, {"causal": True}),
     (2, 8, 8, 2000, 2300, 128, {"lens": [1, 1333]}),
