@@ -304,14 +304,36 @@ bool plan_applies(const acct_fa_args* a) {
 // higher.  Backward call, head_dim 80, causal, 16 tiles, 48 heads 159 -> 170 us, 32 x 24 267 -> 273, 56 x 16 482 -> 501,
 // 64 x 32 1 225 -> 1 205, 96 x 8 711 -> 679; dense, 16 x 8 65 -> 66 (head_dim 96: 66 -> 68), 24 x 32 389 -> 373,
 // 48 x 20 886 -> 835.  At 104, causal, 16 x 48 209 -> 196, 64 x 16 934 -> 703.
+// A pair's item is twice a block's, and of an odd number of K/V tiles the last one is half empty: with few items the longest
+// chain of them grows by more than the quarter that a step on pairs is shorter.  Dense, 1 x 4 heads, 37 tiles (148 items, 76 pairs)
+// 131 -> 185 us, 7 heads, 21 tiles 87 -> 121, 8 heads, 37 tiles (2 rounds -> 3) 242 -> 275, 14 heads, 31 tiles (3 -> 4) 303 -> 312;
+// 32 heads, 23 tiles (5 -> 6) 387 -> 371.
 constexpr int64_t kPairMinTiles = 16, kPairMinTilesNarrow = 24, kPairMinTilesNarrowPartial = 64;
+constexpr int64_t kSms = 148, kPairMaxRounds = 8;      // (of more rounds than that one more is less than a quarter)
+
+// Steps of the longest chain of items, a lower bound: items of `width` K/V tiles come in descending order, so the one that starts
+// round k follows k others that are no shorter.
+int64_t longest_chain(const acct_fa_args* a, int64_t tiles_q, int64_t tiles_k, int64_t width) {
+  const int64_t units = static_cast<int64_t>(a->B) * kv_heads(a), workers = kSms / width, items = (tiles_k + width - 1) / width * units;
+  int64_t longest = 0;
+  for (int64_t k = 0; k * workers < items; ++k) {
+    const int64_t j = k * workers / units * width;                       // its first tile
+    int64_t lo = a->causal ? j : 0;
+    if (a->tri_block > 0 && j * kTile / a->tri_block * a->tri_block / kTile > lo) lo = j * kTile / a->tri_block * a->tri_block / kTile;
+    if ((k + 1) * (tiles_q - lo) > longest) longest = (k + 1) * (tiles_q - lo);
+  }
+  return longest;
+}
+
 bool bwd_on_pairs(const acct_fa_args* a) {
   const int64_t tiles_q = (static_cast<int64_t>(a->S_q) + kTile - 1) / kTile, tiles_k = (static_cast<int64_t>(a->S_k) + kTile - 1) / kTile;
   const int64_t min_q = a->D > 96 ? kPairMinTiles : a->causal || a->tri_block > 0 ? kPairMinTilesNarrowPartial : kPairMinTilesNarrow;
-  return a->D > 64 && a->D <= 128 && !(a->flags & (ACCT_FLAG_DETERMINISTIC | ACCT_FLAG_DROPOUT_PHILOX)) && a->dropout_mask == nullptr &&
+  const bool suits = a->D > 64 && a->D <= 128 && !(a->flags & (ACCT_FLAG_DETERMINISTIC | ACCT_FLAG_DROPOUT_PHILOX)) && a->dropout_mask == nullptr &&
          a->mask_kind == ACCT_MASK_NONE && a->alibi == nullptr && a->alibi_slopes == nullptr && a->seq_lens == nullptr &&
          a->prev_block_num >= ACCT_BAND_UNBOUNDED && a->next_block_num >= ACCT_BAND_UNBOUNDED &&
          a->tri_block % kTile == 0 && tiles_q >= min_q && tiles_k >= kPairMinTiles && tiles_k < 65536 && tiles_q < 65536;
+  return suits && (tiles_k * a->B * kv_heads(a) > kPairMaxRounds * kSms ||
+                   4 * longest_chain(a, tiles_q, tiles_k, 2) <= 5 * longest_chain(a, tiles_q, tiles_k, 1));
 }
 
 // up to 160 columns one CTA holds dK and dV whole; with an ordered dQ reduction the split-width kernel does it

@@ -246,6 +246,13 @@ def test_backward_kernel_of_a_call(lib):
         for S_q, want in ((tiles * 128 - 127, _lib.BWD_PAIR), ((tiles - 1) * 128, _lib.BWD_ONE_BLOCK)):
             assert kernel(D=D, causal=causal, S_q=S_q, S_k=2048) == want
     assert kernel(D=80, causal=0, tri_block=512) == _lib.BWD_ONE_BLOCK
+    # few items: not where pairs take a round more.  (units, tiles, causal)
+    for units, tiles, causal, want in ((4, 37, 0, _lib.BWD_ONE_BLOCK), (4, 37, 1, _lib.BWD_PAIR), (4, 36, 0, _lib.BWD_PAIR),
+                                       (14, 31, 0, _lib.BWD_ONE_BLOCK), (32, 23, 0, _lib.BWD_PAIR), (17, 17, 1, _lib.BWD_PAIR)):
+        assert kernel(B=1, N=units, S_q=tiles * 128, S_k=tiles * 128, causal=causal) == want
+        assert kernel(B=1, N=4 * units, N_kv=units, S_q=tiles * 128, S_k=tiles * 128, causal=causal) == want
+    assert kernel(B=1, N=17, S_q=8192, S_k=2176) == _lib.BWD_ONE_BLOCK
+    assert kernel(B=1, N=4, S_q=37 * 128, S_k=37 * 128, causal=0, tri_block=37 * 128) == _lib.BWD_ONE_BLOCK
     assert kernel(seq_lens=64) == _lib.BWD_ONE_BLOCK      # (device memory, not read: the lengths are not known here)
     assert kernel(flags=_lib.FLAG_DETERMINISTIC) == _lib.BWD_ONE_BLOCK
     assert kernel(D=160) == _lib.BWD_MID and kernel(D=256) == _lib.BWD_WIDE
