@@ -17,8 +17,9 @@
 //
 // The first Q tiles of a head may need the first K/V tile alone (under a causal mask one, at the end of a row group several;
 // all of them where there is no second tile).  In those steps the second tile has no part in any product's result: dQ
-// contracts over the first 128 keys, and dV and dK write the first block's rows.  That its P and dS are 0 there would not do:
-// 0 times a NaN or infinity of a key or query that do not see one another is NaN.
+// contracts over the first 128 keys, and dV and dK write the first block's rows only, or into the second's accumulators what
+// its first step with a part overwrites.  That its P and dS are 0 there would not do: 0 times a NaN or infinity of a key or
+// query that do not see one another is NaN.
 //
 // Tensor memory (512 columns): X = S^T | Y = dP^T | dK | dV, 128 each.  P^T goes over columns 0-31 and 96-127 of X (each half
 // of the compute warps over its own), dS^T likewise in Y; dQ (64 columns of a block: its 64 rows, columns 0-63 in lanes 0-63,
@@ -361,16 +362,21 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
       };
       // queries 16 kk .. + 15 of P^T / dS^T: over columns 0-31 for the first 64 queries, 96-127 for the others
       auto packed_col = [](int kk) { return static_cast<uint32_t>(kk < 4 ? kk * 8 : 64 + kk * 8); };
-      // dV or dK += (P^T or dS^T) (dO or Q) over the queries 16 (4 x + y) .. + 15, x < 2, from <= y < to.  A step in which the
-      // second block has no part, or whose sum starts in one block only, goes through `one_by_one`, out of the way of the others.
-      auto one_by_one = [&](uint32_t d, uint32_t a, uint32_t bb, int from, int to, bool both, bool acc0, bool acc1) {
+      // dV or dK += (P^T or dS^T) (dO or Q) over the queries 16 (4 x + y) .. + 15, x < 2, from <= y < to, in the steps that are not
+      // alike for both blocks, out of the way of the others: without a part of the second block (both = false), or the first one
+      // with a part of it, which starts its sum.
+      auto one_by_one = [&](uint32_t d, uint32_t a, uint32_t bb, int from, int to, bool both) {
 #pragma unroll 1
         for (int x = 0; x < 2; ++x)
 #pragma unroll 1
           for (int y = from; y < to; ++y) {
             const int kk = 4 * x + y;
-            umma_pair_ts_one(0, d, a + packed_col(kk), bb + kk * 128u, mn_hi, idesc_kv, acc0 || kk > 0);
-            if (both) umma_pair_ts_one(1, d, a + packed_col(kk), bb + kk * 128u, mn_hi, idesc_kv, acc1 || kk > 0);
+            if (both && kk > 0) {
+              umma_pair_ts(d, a + packed_col(kk), bb + kk * 128u, mn_hi, idesc_kv, true);
+            } else {
+              umma_pair_ts_one(0, d, a + packed_col(kk), bb + kk * 128u, mn_hi, idesc_kv, true);
+              if (both) umma_pair_ts_one(1, d, a + packed_col(kk), bb + kk * 128u, mn_hi, idesc_kv, false);
+            }
           }
       };
 
@@ -388,7 +394,9 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
         for (int n = 0, m = 0; n < it.n_iter; ++n) {
           const int g = g0 + n;
           const bool more = n + 1 < it.n_iter;
-          const bool both = m >= it.n_first, regular = both && acc1 == (n > 0);
+          const bool both = m >= it.n_first;
+          // (before its first step with a part, what the second block sums up is of no account: that step starts over)
+          const bool regular = both ? acc1 == (n > 0) : !acc1;
           if (++m == it.n_per) m = 0;
           // dV += P^T dO, in two parts as P^T arrives
           mbar_wait(&sh.dom_full, g & 1, abort_flag, p.status, DEV_TIMEOUT_TMA);
@@ -405,7 +413,7 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
                   umma_pair_ts(tmem + kColDV, tmem + kColX + packed_col(kk), mDO + kk * 128u, mn_hi, idesc_kv, n > 0 || kk > 0);
                 }
               } else {
-                one_by_one(tmem + kColDV, tmem + kColX, mDO, part * 2, part * 2 + 2, both, n > 0, acc1);
+                one_by_one(tmem + kColDV, tmem + kColX, mDO, part * 2, part * 2 + 2, both);
               }
             }
           }
@@ -425,7 +433,7 @@ __global__ void __launch_bounds__(kPThreads, 1) __cluster_dims__(2, 1, 1) fa_bwd
               for (int kk = 0; kk < 8; ++kk)
                 umma_pair_ts(tmem + kColDK, tmem + kColY + packed_col(kk), mQ + kk * 128u, mn_hi, idesc_kv, n > 0 || kk > 0);
             } else {
-              one_by_one(tmem + kColDK, tmem + kColY, mQ, 0, 4, both, n > 0, acc1);
+              one_by_one(tmem + kColDK, tmem + kColY, mQ, 0, 4, both);
             }
           }
           acc1 = acc1 || both;
