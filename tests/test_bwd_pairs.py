@@ -1,8 +1,10 @@
 """Backward at head_dim in (64, 128] on pairs of thread blocks: two K/V tiles per work item, products over both.
 
-Checked against the one-block kernel, which the deterministic flag selects: the two share the formulas, round P and dS to 16
-bits and sum in fp32, so a gradient differs by the rounding of its 16 bits and by fp32 sums in another order.
+Checked against the one-block kernel, which the deterministic flag selects, and against float64.  The two kernels share the
+formulas, the roundings of P and dS to 16 bits and the products behind them, so their gradients differ by fp32 sums in another
+order and the last rounding.
 """
+import ctypes as C
 import math
 
 import pytest
@@ -10,18 +12,46 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-# (B, N, N_kv, S_q, S_k, D, options): the fewest tiles that take this path (16, and 24 at head_dim up to 96), pairs with an absent second tile (17), a last
-# Q tile of one row, of one block's rows (64) and of one more, fewer and more items than pairs of SMs, query heads in a group
+# (B, N, N_kv, S_q, S_k, D, options): the fewest tiles that take this path (16, and 24 at head_dim up to 96), pairs with an
+# absent second tile, a last Q tile of one row, of one block's rows (64) and of one more, fewer and more items than pairs of SMs,
+# query heads in a group, pairs of which no Q tile needs the second K/V tile or either of them
 CASES = [
     (1, 1, 1, 2945, 1921, 72, {}),
     (1, 2, 2, 1984, 2100, 128, {"causal": True}),
     (2, 2, 1, 2049, 2048, 104, {"causal": True}),
     (1, 12, 12, 1985, 2177, 128, {}),
     (2, 20, 5, 2048, 2048, 120, {"causal": True}),
-    (2, 8, 8, 2000, 2300, 128, {"lens": [1, 1333]}),
-    (1, 4, 2, 2048, 2048, 128, {"causal": True, "alibi": True}),
     (1, 2, 2, 2304, 2304, 128, {"tri_block": 384}),
+    (1, 4, 1, 2176, 4200, 128, {"causal": True}),
+    (1, 2, 1, 8191, 2100, 96, {"causal": True}),
 ]
+
+
+def kernel_of(q, k, causal=False, tri_block=0):
+    from acctransformer_b200 import _lib
+    a = _lib.FaArgs()
+    a.B, a.N, a.S_q, a.D = q.shape
+    a.N_kv, a.S_k = k.shape[1:3]
+    a.causal, a.tri_block = int(causal), tri_block
+    a.prev_block_num = a.next_block_num = _lib.BAND_UNBOUNDED
+    return _lib.load().acct_fa_bwd_kernel(C.byref(a))
+
+
+def assert_same_sums(got, want, steps):
+    """Gradients of the two kernels, tile by tile: a late tile under a causal mask is small beside the early ones."""
+    for a, b in zip(got, want):
+        # 16 bits: values next to one another at most, beside what the sums differ by
+        ulp = {torch.float32: 0.0, torch.float16: 2.0 ** -10, torch.bfloat16: 2.0 ** -7}[b.dtype]
+        tiny = {torch.float32: 0.0, torch.float16: 2.0 ** -24, torch.bfloat16: 2.0 ** -133}[b.dtype]
+        a, b = a.float(), b.float()
+        assert torch.isfinite(a).all()
+        for i in range(0, b.shape[2], 128):
+            x, y = a[:, :, i:i + 128], b[:, :, i:i + 128]
+            # 8 additions per 128 positions, each off by 2^-23 (a truncated sum) of a partial sum, which is no larger than the
+            # largest results of its tile; on both sides
+            size = y.abs().amax(dim=(2, 3), keepdim=True)
+            assert ((x - y).abs() <= 2 * 8 * steps * 2.0 ** -23 * size + ulp * y.abs() + tiny).all()
+            assert not x[(y == 0).all(-1)].any()      # no query sees the key, or the other way round
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
@@ -37,25 +67,50 @@ def test_against_the_one_block_kernel(case, dtype, f32):
     def rnd(*shape):
         return torch.randn(*shape, generator=g).to(dtype).cuda()
     q, d_o, k, v = rnd(B, N, S_q, D), rnd(B, N, S_q, D), rnd(B, N_kv, S_k, D), rnd(B, N_kv, S_k, D)
-    kw = {x: opt[x] for x in ("causal", "tri_block") if x in opt}
-    if "lens" in opt:
-        kw["seq_lens"] = torch.tensor(opt["lens"], dtype=torch.int32).cuda()
-    if "alibi" in opt:
-        kw["alibi"] = (-0.1 * torch.arange(S_k).float()).expand(B, N, 1, S_k).to(dtype).cuda()
+    assert kernel_of(q, k, **opt) == _lib.BWD_PAIR
     scale = 1.0 / math.sqrt(D)
-    o, lse = ops.fa_forward(q, k, v, scale=scale, **kw)
-    want = ops.fa_backward(q, k, v, o, lse, d_o, scale=scale, grads_fp32=f32, deterministic=True, **kw)
-    # a P or dS that rounds to its other 16-bit neighbour moves a gradient by 2^-11 (fp16) / 2^-8 (bf16) of one term;
-    # the terms are of the size of the largest gradient at most
-    unit = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    o, lse = ops.fa_forward(q, k, v, scale=scale, **opt)
+    want = ops.fa_backward(q, k, v, o, lse, d_o, scale=scale, grads_fp32=f32, deterministic=True, **opt)
     for _ in range(3):                # (the blocks of a pair meet in another order each time)
-        got = ops.fa_backward(q, k, v, o, lse, d_o, scale=scale, grads_fp32=f32, **kw)
+        got = ops.fa_backward(q, k, v, o, lse, d_o, scale=scale, grads_fp32=f32, **opt)
         torch.cuda.synchronize()
         _lib.device_status()
-        for a, b in zip(got, want):
-            assert torch.isfinite(a).all()
-            err = (a.float() - b.float()).abs().max().item()
-            assert err <= 2 * unit * max(b.float().abs().max().item(), 1e-3)
+        assert_same_sums(got, want, -(-max(S_q * N // N_kv, S_k) // 128))
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("S, N, N_kv, opt", [(2048, 2, 2, {}), (2100, 4, 1, {"causal": True}), (2200, 2, 1, {"tri_block": 640}),
+                                             (2304, 2, 2, {"tri_block": 384, "causal": True})])
+def test_views_of_a_projection_against_float64(S, N, N_kv, opt, dtype):
+    """q, k, v as views of one fused projection, o and its gradient in the layout of the output projection."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from acctransformer_b200 import _lib, ops
+    B, D = 2, 128
+    g = torch.Generator().manual_seed(S)
+    x = torch.randn(B, S, (N + 2 * N_kv) * D, generator=g).to(dtype).cuda()
+    q, k, v = (t.view(B, S, -1, D).transpose(1, 2) for t in x.split([N * D, N_kv * D, N_kv * D], dim=2))
+    d_o = torch.randn(B, S, N, D, generator=g).to(dtype).cuda().transpose(1, 2)
+    assert kernel_of(q, k, **opt) == _lib.BWD_PAIR
+    out = torch.empty(B, S, N, D, dtype=dtype, device="cuda").transpose(1, 2)
+    o, lse = ops.fa_forward(q, k, v, scale=D ** -0.5, **opt)
+    out.copy_(o)
+    got = (out,) + tuple(ops.fa_backward(q, k, v, out, lse, d_o, scale=D ** -0.5, **opt))
+    _lib.device_status()
+    qd, kd, vd = (t.double().detach().requires_grad_() for t in (q, k, v))
+    s = qd @ kd.repeat_interleave(N // N_kv, 1).transpose(-1, -2) * D ** -0.5
+    row, col = torch.arange(S, device="cuda")[:, None], torch.arange(S, device="cuda")[None]
+    if opt.get("causal"):
+        s = s.masked_fill(col > row, -math.inf)
+    if "tri_block" in opt:
+        s = s.masked_fill(col >= (row // opt["tri_block"] + 1) * opt["tri_block"], -math.inf)
+    ref = torch.softmax(s, -1) @ vd.repeat_interleave(N // N_kv, 1)
+    want = (ref,) + torch.autograd.grad(ref, (qd, kd, vd), d_o.double())
+    for a, b in zip(got, want):
+        # a handful of roundings to 16 bits (2^-9, 2^-12 of the values' size each), tile by tile
+        for i in range(0, S, 128):
+            y = b[:, :, i:i + 128]
+            assert (a[:, :, i:i + 128].double() - y).norm() <= (1e-2 if dtype == torch.bfloat16 else 2e-3) * y.norm()
 
 
 @pytest.mark.parametrize("causal", [False, True])
@@ -98,11 +153,12 @@ def test_what_is_not_finite_stays_with_the_tiles_that_see_it(S_q, S_k, opt, wher
     """NaN and infinity reach the gradients that they reach on the one-block kernel, and no others."""
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
-    from acctransformer_b200 import ops
+    from acctransformer_b200 import _lib, ops
     g = torch.Generator().manual_seed(S_q + S_k)
     t = {n: torch.randn(1, h, s, 128, generator=g).half().cuda() for n, h, s in
          (("q", 2, S_q), ("k", 1, S_k), ("v", 1, S_k), ("d_o", 2, S_q))}
     kw = {"scale": 128 ** -0.5, **opt}
+    assert kernel_of(t["q"], t["k"], **opt) == _lib.BWD_PAIR
     for row, value in ((5, float("nan")), (200, float("inf")), (450, float("nan")), (S_q - 3, float("inf"))):
         x = {n: u.clone() for n, u in t.items()}
         x[where][0, 0, row] = value
