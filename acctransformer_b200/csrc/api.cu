@@ -292,16 +292,18 @@ bool plan_applies(const acct_fa_args* a) {
          static_cast<int64_t>(a->B) * a->N * tq * tk >= kPlanMinTilePairs;
 }
 
-// Whether the backward runs on pairs of thread blocks (fa_bwd_pair.cu): long walks without per-element work.  Forward and
-// backward, one block -> pairs: 2 x 32 heads of 128, 8 192 tokens causal 4 452 -> 4 008 us, 8 x 32 heads, 4 096 tokens in row
-// groups of 512 4 845 -> 4 519; 4 x 16 heads, 2 048 tokens (16 tiles, the line) backward 278 -> 265, but with
-// alibi 377 -> 383 in all.  Documents of 3 000 tokens lost (499 -> 517: short walks, and a Q tile that either tile of
-// a pair needs is walked by both), and so did a band with in-kernel dropout (backward 1 306 -> 1 824).  Valid lengths keep
-// one block: they are known on the GPU only, half of a pair idles where one ends in its first tile (2 x 64 heads, 2 048 keys
-// of which 128 valid: backward call 220 -> 256 us, 384: 290 -> 312, 1 024: 410 -> 373), and a product over both tiles must
-// not see keys that do not exist.
+// Whether the backward runs on pairs of thread blocks (fa_bwd_pair.cu): long walks without per-element work.  All times are of
+// a backward call, one block -> pairs; 1 x heads of 128 in fp16 unless it says otherwise.
+// Causal: 64 tiles, 2 x 32 heads 3 416 -> 2 583 us, 16 heads 853 -> 671; 32 tiles, 24 heads 336 -> 291; 16 tiles, 48 heads
+// 212 -> 200.  Dense: 64 tiles, 16 heads 1 683 -> 1 247; 16 tiles, 48 heads 404 -> 330.  Row groups of 512: 8 x 32 heads, 4 096 tokens
+// 3 693 -> 2 985.  32 query heads on 8 of K/V, 2 x 3 000 tokens, bf16, causal: 547 -> 423.  Shorter walks were not timed.
+// What kept one block when it was timed: alibi (4 x 16 heads, 2 048 tokens, forward and backward 377 -> 383; longer ones were not
+// timed), documents of 3 000 tokens (499 -> 517: short walks, and a Q tile that either tile of a pair needs is walked by both),
+// a band with in-kernel dropout (1 306 -> 1 824; neither was timed without the other).  Valid lengths keep one block: they are
+// known on the GPU only, half of a pair idles where one ends in its first tile (2 x 64 heads, 2 048 keys of which 128 valid:
+// 220 -> 256, 384: 290 -> 312, 1 024: 410 -> 373), and a product over both tiles must not see keys that do not exist.
 // At head_dim up to 96 the one-block kernel has less of dQ to add, the pair's products are as wide as ever, and the line lies
-// higher.  Backward call, head_dim 80, causal, 16 tiles, 48 heads 159 -> 170 us, 32 x 24 267 -> 273, 56 x 16 482 -> 501,
+// higher.  Head_dim 80, causal, 16 tiles, 48 heads 159 -> 170 us, 32 x 24 267 -> 273, 56 x 16 482 -> 501,
 // 64 x 32 1 225 -> 1 205, 96 x 8 711 -> 679; dense, 16 x 8 65 -> 66 (head_dim 96: 66 -> 68), 24 x 32 389 -> 373,
 // 48 x 20 886 -> 835.  At 104, causal, 16 x 48 209 -> 196, 64 x 16 934 -> 703.
 // A pair's item is twice a block's, and of an odd number of K/V tiles the last one is half empty: with few items the longest

@@ -36,8 +36,9 @@
 // other block's shared memory goes there by an asynchronous copy (plain and st.async stores of the same 16 KB took 1 400 and
 // 3 000 clk).
 //
-// 2 x 32 heads of 128, 8 192 tokens, causal: backward call 2 865-3 160 -> 2 495 us, forward and backward 4 452 -> 4 008; a step
-// 4 800 -> 4 100 clk.  What bounds it now: the compute warps (S^T -> P^T -> dS^T, 3 500 clk of a step), whose two halves wait for
+// 2 x 32 heads of 128, 8 192 tokens, causal, against the one-block kernel: backward call 3 416 -> 2 583 us, forward and backward
+// 4 421 -> 3 933; a step 4 800 -> 4 100 clk (cycle counters; with the register split of before).  The tensor pipe is busy 59 % of
+// the time (43 %).  What bounds it now: the compute warps (S^T -> P^T -> dS^T, 3 500 clk of a step), whose two halves wait for
 // one another through the tensor pipe.
 //
 // Follows the reference's backward (train/acctransformer/flash_attention/ops/flash_attention/flash_attention_bwd.py:259-415)

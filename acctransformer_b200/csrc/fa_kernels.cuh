@@ -157,8 +157,8 @@ cudaError_t allow_smem(const void* kernel, size_t bytes);
 // Launchers: return cudaGetLastError() of the launch.
 cudaError_t launch_fa_fwd(const FwdParams& p, bool bf16, int sm_count, cudaStream_t stream);
 cudaError_t launch_fa_bwd(const BwdParams& p, bool bf16, int sm_count, cudaStream_t stream);
-// head_dim in (64, 128], dQ in any order, no mask tensor, band, valid lengths or dropout, row groups of whole tiles: like
-// launch_fa_bwd with 64-row boxes of the Q, dO and dQ maps
+// head_dim in (64, 128], dQ in any order, no mask tensor, alibi, band, valid lengths or dropout, row groups of whole tiles:
+// like launch_fa_bwd with 64-row boxes of the Q, dO and dQ maps
 cudaError_t launch_fa_bwd_pair(const BwdParams& p, bool bf16, int sm_count, cudaStream_t stream);
 // head_dim in (128, 256]: Q / dO maps with 64-row boxes, the dQ map with a 32 x 64 box, two turn counters per Q tile
 cudaError_t launch_fa_bwd_wide(const BwdParams& p, bool bf16, cudaStream_t stream);

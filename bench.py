@@ -190,6 +190,17 @@ def measured_peaks():
     return {"tflops": 1400.0, "tflops_burst": 1590.0, "hbm_gbs": 6650.0, "which": "fallback"}
 
 
+def backward_kernel(_lib, cfg):
+    """Name of the kernel that the timed backward runs, and DRAM bytes of one launch of it on workload P under ncu."""
+    import ctypes
+    a = _lib.FaArgs()
+    a.B, a.N, a.S_q, a.S_k, a.D, a.causal = cfg["B"], cfg["N"], cfg["S"], cfg["S"], cfg["D"], 1
+    a.prev_block_num = a.next_block_num = _lib.BAND_UNBOUNDED
+    if _lib.load().acct_fa_bwd_kernel(ctypes.byref(a)) == _lib.BWD_PAIR:
+        return "fa_bwd_pair_kernel", 202.5e6 + 87.7e6
+    return "fa_bwd_kernel", 203.8e6 + 89.3e6
+
+
 def run_ours(args):
     import torch
     import torch.distributed as dist
@@ -397,15 +408,16 @@ def run_ours(args):
     # The kernel is timed alone by an event pair, so the burst figure is the denominator; the sustained one (a
     # seconds-long GEMM loop under the power cap) is given beside it.  kcycles = ms x median SM MHz sampled during
     # the timed legs: runs that the power cap held at different clocks compare on that.
-    roofline = {"kernel": "fa_bwd_kernel (CUDA events recorded by the library directly around its launch)",
+    bwd_name, bwd_bytes = backward_kernel(_lib, cfg)
+    roofline = {"kernel": bwd_name + " (CUDA events recorded by the library directly around its launch)",
                 "bound": "tensor", "achieved": bwd_tflops, "peak": peaks["tflops_burst"], "unit": "TFLOP/s",
                 "frac": bwd_tflops / peaks["tflops_burst"], "peak_source": f"{peaks['which']} bf16_tflops (burst)",
                 "frac_of_sustained": bwd_tflops / peaks["tflops"], "peak_sustained": peaks["tflops"],
                 "kcycles": ms_bwd_kernel * mhz if mhz else None,
                 "ms_whole_backward_call": ms_bwd,   # + row-sum kernel, zero-fill, dQ conversion
-                # DRAM read + write bytes of one backward-kernel launch: ncu capture on workload P (203.8 + 89.3 MB,
-                # profiles/fa_bwd_kernel_P_ncu_full.md) scaled by the units x sequence ratio of the workload
-                "traffic": 293.1e6 * (cfg["B"] * cfg["N"] * cfg["S"]) / (2 * 16 * 4096), "ms": ms_bwd_kernel,
+                # DRAM read + write bytes of one backward-kernel launch: ncu capture on workload P scaled by the units x
+                # sequence ratio of the workload
+                "traffic": bwd_bytes * (cfg["B"] * cfg["N"] * cfg["S"]) / (2 * 16 * 4096), "ms": ms_bwd_kernel,
                 "fwd": {"kernel": "fa_fwd_kernel", "achieved": fwd_tflops, "frac": fwd_tflops / peaks["tflops_burst"],
                         "frac_of_sustained": fwd_tflops / peaks["tflops"], "ms": ms_fwd,
                         "kcycles": ms_fwd * mhz if mhz else None},
